@@ -45,7 +45,8 @@ class OrcConfig(C.Structure):
 def build(ref: bool = True) -> None:
     """Compile the restatement, and the reference when its sources are present."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
-    if ref and os.path.isdir(REF_SRC_DIR):
+    # an empty directory of that name holds no sources: the reference is then not built
+    if ref and os.path.isfile(os.path.join(REF_SRC_DIR, "range_kutta.cpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF_DIR={REF_SRC_DIR}"], check=True)
         if os.path.exists(os.path.join(os.path.dirname(HERE), "ns3d_wcns_b200", "libns3d_b200.so")):
             subprocess.run(["make", "-s", "-C", HERE, "dropin", f"REF_DIR={REF_SRC_DIR}"], check=True)
