@@ -183,9 +183,10 @@ __device__ __forceinline__ double cfl_bound(const double U[5], double gamma, dou
 // The wave speed |u| + a of cfl_bound (cfl_bound = dx / cfl_speed, same bits).
 __device__ __forceinline__ double cfl_speed(const double U[5], double gamma) {
     double rho = U[0];
-    double u = U[1] / rho;
+    const double ir = rcp_fp64(rho);
+    double u = div_fp64(U[1], rho, ir);
     double p = __dmul_rn(gamma - 1., __dsub_rn(U[4], __dmul_rn(__dmul_rn(__dmul_rn(0.5, rho), u), u)));
-    double a = sqrt(__dmul_rn(gamma, p) / rho);
+    double a = sqrt(div_fp64(__dmul_rn(gamma, p), rho, ir));
     return __dadd_rn(fabs(u), a);
 }
 

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) stage_kernel64(StageArgs64 a) {
     const long o = L.at(i, j, k);
 #pragma unroll
     for (int q = 0; q < 5; ++q) a.Wout[q][o] = W[q];
-    a.Tout[o] = W[4] / __dmul_rn(W[0], a.Rgas);
+    a.Tout[o] = temperature_exact(W, a.Rgas);
     if (a.cfl_part) {
         const int co[3] = {i, j, k};
         if (is_interior(L, co)) {
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256) stage_ghost_kernel64(StageArgs64 a) {
     const long o = L.at(i, j, k);
 #pragma unroll
     for (int q = 0; q < 5; ++q) a.Wout[q][o] = W[q];
-    a.Tout[o] = W[4] / __dmul_rn(W[0], a.Rgas);
+    a.Tout[o] = temperature_exact(W, a.Rgas);
 }
 
 // Ghost cells after the mixed path's fused z-sweep (increment form, see

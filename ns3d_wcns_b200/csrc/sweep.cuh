@@ -183,7 +183,7 @@ __device__ __forceinline__ void fused_stage_cell(const FusedStage &f, double dt,
     c2p_exact(U, f.gamma, W);
 #pragma unroll
     for (int q = 0; q < 5; ++q) f.Wout[q][c] = W[q];
-    f.Tout[c] = W[4] / __dmul_rn(W[0], f.Rgas);
+    f.Tout[c] = temperature_exact(W, f.Rgas);
     if (f.stage == 3) {
         double Un[5];
         p2c_exact(W[0], W[1], W[2], W[3], W[4], f.gamma, Un);
@@ -767,6 +767,7 @@ inline cudaError_t launch_sweep(const SweepArgs<R> &a, cudaStream_t st) {
 cudaError_t sweep_x(const SweepArgs<double> &, cudaStream_t);
 cudaError_t sweep_y(const SweepArgs<double> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<double> &, cudaStream_t);
+long sweep_z_blocks(const SweepArgs<double> &);
 cudaError_t sweep_x(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_y(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<float> &, cudaStream_t);

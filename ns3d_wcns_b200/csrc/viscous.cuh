@@ -71,6 +71,7 @@ __device__ __forceinline__ R dstencil(F f, int order, R h) {
 // Sutherland's law mu0 T^1.5 (1+S)/(T+S), with T^1.5 evaluated as T sqrt(T).
 template <typename R>
 __device__ __forceinline__ R sutherland(R mu0, R S, R T) {
+    if constexpr (sizeof(R) == 8) return mu0 * (T * sqrt_fp64(T)) * (R(1) + S) * rcp_fp64(T + S);
     return mu0 * (T * sqrt(T)) * (R(1) + S) / (T + S);
 }
 
