@@ -9,6 +9,7 @@
 // result is mathematically identical and differs only in rounding.
 #pragma once
 
+#include <cmath>
 #include <cstring>
 
 #include "common.cuh"
@@ -30,6 +31,31 @@ struct SchemeParams {
     R hd[4];            // MDCD-WENO linear weights d0..d3 (interpolation.cpp:179-182)
     int interp, riemann, char_recon;  // runtime selection for the generic kernel
 };
+
+// Reciprocal and square root of the schemes: on the device FP64 takes the
+// branch-free forms of common.cuh; FP32 and the host take the operations.
+template <typename R>
+NS3D_HD R rcp_(R x) {
+#ifdef __CUDA_ARCH__
+    if constexpr (sizeof(R) == 8) return rcp_fp64(x);
+#endif
+    return R(1) / x;
+}
+template <typename R>
+NS3D_HD R sqrt_(R x) {
+#ifdef __CUDA_ARCH__
+    if constexpr (sizeof(R) == 8) return sqrt_fp64(x);
+#endif
+    return sqrt(x);
+}
+// a / b; FP64 on the device as a times the reciprocal
+template <typename R>
+NS3D_HD R quot_(R a, R b) {
+#ifdef __CUDA_ARCH__
+    if constexpr (sizeof(R) == 8) return a * rcp_fp64(b);
+#endif
+    return a / b;
+}
 
 // ------------------------------------------------------------ interpolation
 
@@ -55,7 +81,7 @@ NS3D_HD R weno5(R f0, R f1, R f2, R f3, R f4) {
     R p0 = R(3) * f0 - R(10) * f1 + R(15) * f2;
     R p1 = -f1 + R(6) * f2 + R(3) * f3;
     R p2 = R(3) * f2 + R(6) * f3 - f4;
-    return (a0 * p0 + a1 * p1 + a2 * p2) / (R(8) * (a0 + a1 + a2));
+    return quot_(a0 * p0 + a1 * p1 + a2 * p2, R(8) * (a0 + a1 + a2));
 }
 
 // mdcd_linear_interpolate, interpolation.cpp:118-133.
@@ -156,7 +182,12 @@ NS3D_HD bool mdcd_smooth_fast(R fm2, R fm1, R f0, R fp1, R fp2, bool &near) {
     R a = fabs(f0 - fm1) + fabs(f0 - R(2) * fm1 + fm2);
     R b = fabs(f0 - fp1) + fabs(f0 - R(2) * fp1 + fp2);
     const R lhs = R(2) * a * b + eps, rhs = R(0.4) * (a * a + b * b + eps);
-    if constexpr (sizeof(R) == 8) near |= (unsigned)(f64_hi_word(lhs) - f64_hi_word(rhs) + 1) <= 2u;
+    if constexpr (sizeof(R) == 8) {
+        // where near stays clear the high words decide (both sides are positive)
+        const int d = f64_hi_word(lhs) - f64_hi_word(rhs);
+        near |= (unsigned)(d + 1) <= 2u;
+        return d > 0;
+    }
     return lhs > rhs;
 }
 
@@ -186,13 +217,13 @@ NS3D_HD R mdcd_weno_branch(const R *hd, R f0, R f1, R f2, R f3, R f4, R f5) {
     using Wt = double;
     Wt tau6 = fabs((Wt)be3 - ((Wt)be0 + Wt(4) * (Wt)be1 + (Wt)be2) / Wt(6));
     const Wt es = sizeof(R) == 8 ? (Wt)eps_small : Wt(1e-40);
-    Wt g0 = Wt(20) + tau6 / ((Wt)be0 + es);
-    Wt g1 = Wt(20) + tau6 / ((Wt)be1 + es);
-    Wt g2 = Wt(20) + tau6 / ((Wt)be2 + es);
-    Wt g3 = Wt(20) + tau6 / ((Wt)be3 + es);
+    Wt g0 = Wt(20) + quot_(tau6, (Wt)be0 + es);
+    Wt g1 = Wt(20) + quot_(tau6, (Wt)be1 + es);
+    Wt g2 = Wt(20) + quot_(tau6, (Wt)be2 + es);
+    Wt g3 = Wt(20) + quot_(tau6, (Wt)be3 + es);
     Wt al0 = (Wt)hd[0] * (g0 * g0), al1 = (Wt)hd[1] * (g1 * g1), al2 = (Wt)hd[2] * (g2 * g2),
        al3 = (Wt)hd[3] * (g3 * g3);
-    return (R)((al0 * (Wt)q0 + al1 * (Wt)q1 + al2 * (Wt)q2 + al3 * (Wt)q3) / (Wt(8) * (al0 + al1 + al2 + al3)));
+    return (R)quot_(al0 * (Wt)q0 + al1 * (Wt)q1 + al2 * (Wt)q2 + al3 * (Wt)q3, Wt(8) * (al0 + al1 + al2 + al3));
 }
 
 template <typename R>
@@ -242,7 +273,7 @@ template <int DIR, typename R>
 struct Side {
     R r, ir, u, v, w, E, p, un;
     NS3D_HD void load(const R *U, R g) {
-        r = U[0]; ir = R(1) / r;
+        r = U[0]; ir = rcp_(r);
         u = U[1] * ir; v = U[2] * ir; w = U[3] * ir; E = U[4];
         p = (E - R(0.5) * r * (u * u + v * v + w * w)) * (g - R(1));
         un = DIR == 0 ? u : (DIR == 1 ? v : w);
@@ -270,18 +301,16 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     R FL[5], FR[5];
     L.flux(FL); Rt.flux(FR);
     const R gm1 = g - R(1);
-    const R kfac = g / gm1;
-    R HL = R(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w) + kfac * L.p * L.ir;
-    R HR = R(0.5) * (Rt.u * Rt.u + Rt.v * Rt.v + Rt.w * Rt.w) + kfac * Rt.p * Rt.ir;
-    R sL = sqrt(L.r), sR = sqrt(Rt.r);
-    R den = R(1) / (sL + sR);
+    R HL = (L.E + L.p) * L.ir, HR = (Rt.E + Rt.p) * Rt.ir;
+    R sL = sqrt_(L.r), sR = sqrt_(Rt.r);
+    R den = rcp_(sL + sR);
     R ub = (sL * L.u + sR * Rt.u) * den;
     R vb = (sL * L.v + sR * Rt.v) * den;
     R wb = (sL * L.w + sR * Rt.w) * den;
     R Hb = (sL * HL + sR * HR) * den;
     R q2 = ub * ub + vb * vb + wb * wb;
     R c2 = gm1 * (Hb - R(0.5) * q2);
-    R c = sqrt(c2);
+    R c = sqrt_(c2);
     R V = DIR == 0 ? ub : (DIR == 1 ? vb : wb);
     R phi = R(0.5) * gm1 * q2;
     R dU[5];
@@ -290,14 +319,14 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     const R dUn = dU[1 + DIR];
     R t = phi * dU[0] + gm1 * (dU[4] - ub * dU[1] - vb * dU[2] - wb * dU[3]);
     R s = c * (V * dU[0] - dUn);
-    R i2c2 = R(1) / (R(2) * c2);
+    R i2c2 = rcp_(R(2) * c2);
     R A0 = (t + s) * i2c2;   // acoustic wave V - c: alpha0 * a3
     R A4 = (t - s) * i2c2;   // acoustic wave V + c
     R l0 = fabs(V - c), lv = fabs(V), l4 = fabs(V + c);
     R delta = R(0.1) * (lv + c);
     // (l^2 + delta^2) / (2 delta) below delta, through one reciprocal and
     // selects (no divergent division per eigenvalue)
-    const R i2d = R(1) / (R(2) * delta), d2 = delta * delta;
+    const R i2d = rcp_(R(2) * delta), d2 = delta * delta;
     l0 = l0 < delta ? (l0 * l0 + d2) * i2d : l0;
     lv = lv < delta ? (lv * lv + d2) * i2d : lv;
     l4 = l4 < delta ? (l4 * l4 + d2) * i2d : l4;
@@ -323,7 +352,7 @@ NS3D_HD void rusanov_flux(const R *UL, const R *UR, R g, R *F) {
     L.load(UL, g); Rt.load(UR, g);
     R FL[5], FR[5];
     L.flux(FL); Rt.flux(FR);
-    R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rt.p * Rt.ir);
+    R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rt.p * Rt.ir);
     R smax = fmax(fabs(L.un) + aL, fabs(Rt.un) + aR);
 #pragma unroll
     for (int n = 0; n < 5; ++n) F[n] = R(0.5) * (FL[n] + FR[n]) - R(0.5) * smax * (UR[n] - UL[n]);
@@ -336,7 +365,7 @@ NS3D_HD void hll_flux(const R *UL, const R *UR, R g, R *F) {
     L.load(UL, g); Rt.load(UR, g);
     R FL[5], FR[5];
     L.flux(FL); Rt.flux(FR);
-    R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rt.p * Rt.ir);
+    R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rt.p * Rt.ir);
     R SL = fmin(L.un - aL, Rt.un - aR);
     R SR = fmax(L.un + aL, Rt.un + aR);
     if (SL >= R(0)) {
@@ -346,7 +375,7 @@ NS3D_HD void hll_flux(const R *UL, const R *UR, R g, R *F) {
 #pragma unroll
         for (int n = 0; n < 5; ++n) F[n] = FR[n];
     } else {
-        R id = R(1) / (SR - SL);
+        R id = rcp_(SR - SL);
 #pragma unroll
         for (int n = 0; n < 5; ++n) F[n] = (SR * FL[n] - SL * FR[n] + SL * SR * (UR[n] - UL[n])) * id;
     }
@@ -357,9 +386,9 @@ template <int DIR, typename R>
 NS3D_HD void hllc_star(const Side<DIR, R> &S, const R *U, const R *Fs, R Sk, R SM,
                                           R *F) {
     R dk = Sk - S.un;
-    R rs = S.r * dk / (Sk - SM);
+    R rs = quot_(S.r * dk, Sk - SM);
     R us = DIR == 0 ? SM : S.u, vs = DIR == 1 ? SM : S.v, ws = DIR == 2 ? SM : S.w;
-    R Es = S.E * S.ir + (SM - S.un) * (SM + S.p / (S.r * dk));
+    R Es = S.E * S.ir + (SM - S.un) * (SM + quot_(S.p, S.r * dk));
     F[0] = Fs[0] + Sk * (rs - U[0]);
     F[1] = Fs[1] + Sk * (rs * us - U[1]);
     F[2] = Fs[2] + Sk * (rs * vs - U[2]);
@@ -369,37 +398,48 @@ NS3D_HD void hllc_star(const Side<DIR, R> &S, const R *U, const R *Fs, R Sk, R S
 
 // HLLC_Riemann_solver, InviscousFlux.cpp:449-592: Davis S_L/S_R, Batten S_M
 // (Roe-averaged normal velocity when the S_M denominator is below 1e-12).
+//
+// The star flux F_k + S_k (U* - U_k) of the upwind side, through the jump
+// conditions that define U*:
+//   rho* = m / (S_k - S_M), p* = p + m (S_M - u_n), m = rho (S_k - u_n),
+//   E* = ((S_k - u_n) E - p u_n + p* S_M) / (S_k - S_M),
+//   F = (rho* S_M, rho* S_M V + p* n, (E* + p*) S_M)
+// -- the same flux with half of the operations and one quotient less.
 template <int DIR, typename R>
 NS3D_HD void hllc_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
     L.load(UL, g); Rt.load(UR, g);
-    R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rt.p * Rt.ir);
+    R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rt.p * Rt.ir);
     R SL = fmin(L.un - aL, Rt.un - aR);
     R SR = fmax(L.un + aL, Rt.un + aR);
     if (SL >= R(0)) { L.flux(F); return; }
     if (SR <= R(0)) { Rt.flux(F); return; }
-    R num = Rt.r * Rt.un * (SR - Rt.un) - L.r * L.un * (SL - L.un) + L.p - Rt.p;
-    R den = Rt.r * (SR - Rt.un) - L.r * (SL - L.un);
+    const R dL = SL - L.un, dR = SR - Rt.un;
+    const R mL = L.r * dL, mR = Rt.r * dR;
+    const R num = mR * Rt.un - mL * L.un + L.p - Rt.p;
+    const R den = mR - mL;
     R SM;
     if (fabs(den) > R(1e-12)) {
-        SM = num / den;
+        SM = quot_(num, den);
     } else {
-        R sL = sqrt(L.r), sR = sqrt(Rt.r);
-        SM = (sL * L.un + sR * Rt.un) / (sL + sR);
+        R sL = sqrt_(L.r), sR = sqrt_(Rt.r);
+        SM = quot_(sL * L.un + sR * Rt.un, sL + sR);
     }
     // the star state of the upwind side: selected, not branched, so faces of
     // one warp with different signs of S_M do not diverge
     const bool left = SM >= R(0);
-    Side<DIR, R> S;
-    S.r = left ? L.r : Rt.r; S.ir = left ? L.ir : Rt.ir;
-    S.u = left ? L.u : Rt.u; S.v = left ? L.v : Rt.v; S.w = left ? L.w : Rt.w;
-    S.E = left ? L.E : Rt.E; S.p = left ? L.p : Rt.p; S.un = left ? L.un : Rt.un;
-    R Us[5];
-#pragma unroll
-    for (int n = 0; n < 5; ++n) Us[n] = left ? UL[n] : UR[n];
-    R Fs[5];
-    S.flux(Fs);
-    hllc_star<DIR, R>(S, Us, Fs, left ? SL : SR, SM, F);
+    const R Sk = left ? SL : SR, m = left ? mL : mR, dk = left ? dL : dR;
+    const R u = left ? L.u : Rt.u, v = left ? L.v : Rt.v, w = left ? L.w : Rt.w;
+    const R E = left ? L.E : Rt.E, p = left ? L.p : Rt.p, un = DIR == 0 ? u : (DIR == 1 ? v : w);
+    const R is = rcp_(Sk - SM);
+    const R ps = p + m * (SM - un);
+    const R Es = (dk * E - p * un + ps * SM) * is;
+    const R ms = m * is * SM;  // rho* S_M
+    F[0] = ms;
+    F[1] = DIR == 0 ? ms * SM + ps : ms * u;
+    F[2] = DIR == 1 ? ms * SM + ps : ms * v;
+    F[3] = DIR == 2 ? ms * SM + ps : ms * w;
+    F[4] = (Es + ps) * SM;
 }
 
 // HLLC_p_Riemann_solver, InviscousFlux.cpp:594-717: PVRS p*, Toro speeds.
@@ -407,16 +447,16 @@ template <int DIR, typename R>
 NS3D_HD void hllc_p_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
     L.load(UL, g); Rt.load(UR, g);
-    R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rt.p * Rt.ir);
+    R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rt.p * Rt.ir);
     R ps = R(0.5) * (L.p + Rt.p) - R(0.125) * (Rt.un - L.un) * (L.r + Rt.r) * (aL + aR);
     ps = fmax(R(0), ps);
     const R c1 = (g + R(1)) / (R(2) * g), c2 = (g - R(1)) / (R(2) * g);
-    R SL = ps <= L.p ? L.un - aL : L.un - aL * sqrt(c1 * ps / L.p + c2);
-    R SR = ps <= Rt.p ? Rt.un + aR : Rt.un + aR * sqrt(c1 * ps / Rt.p + c2);
+    R SL = ps <= L.p ? L.un - aL : L.un - aL * sqrt_(c1 * ps / L.p + c2);
+    R SR = ps <= Rt.p ? Rt.un + aR : Rt.un + aR * sqrt_(c1 * ps / Rt.p + c2);
     if (SL >= R(0)) { L.flux(F); return; }
     if (SR <= R(0)) { Rt.flux(F); return; }
-    R SM = (Rt.p - L.p + L.r * L.un * (SL - L.un) - Rt.r * Rt.un * (SR - Rt.un)) /
-           (L.r * (SL - L.un) - Rt.r * (SR - Rt.un));
+    R SM = quot_(Rt.p - L.p + L.r * L.un * (SL - L.un) - Rt.r * Rt.un * (SR - Rt.un),
+                 L.r * (SL - L.un) - Rt.r * (SR - Rt.un));
     R Fs[5];
     if (SM >= R(0)) { L.flux(Fs); hllc_star<DIR, R>(L, UL, Fs, SL, SM, F); }
     else { Rt.flux(Fs); hllc_star<DIR, R>(Rt, UR, Fs, SR, SM, F); }
@@ -431,10 +471,10 @@ NS3D_HD void ausm_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
     L.load(UL, g); Rt.load(UR, g);
     R pL = fmax(L.p, R(1e-12)), pR = fmax(Rt.p, R(1e-12));
-    R aL = sqrt(g * pL * L.ir), aR = sqrt(g * pR * Rt.ir);
+    R aL = sqrt_(g * pL * L.ir), aR = sqrt_(g * pR * Rt.ir);
     R HL = (L.E + pL) * L.ir, HR = (Rt.E + pR) * Rt.ir;
     R ab = R(0.5) * (aL + aR), rb = R(0.5) * (L.r + Rt.r);
-    R iab = R(1) / ab;
+    R iab = rcp_(ab);
     R ML = L.un * iab, MR = Rt.un * iab;
     R Mb2 = (L.un * L.un + Rt.un * Rt.un) * (R(0.5) * iab * iab);
     R Mo2 = fmin(R(1), fmax(Mb2, R(0.5)));
@@ -473,7 +513,7 @@ template <int DIR, typename R>
 NS3D_HD void sw_split(const R *U, R g, R sgn, R *F) {
     Side<DIR, R> S;
     S.load(U, g);
-    const R c2 = g * S.p * S.ir, c = sqrt(c2);
+    const R c2 = g * S.p * S.ir, c = sqrt_(c2);
     auto part = [&](R l) { return R(0.5) * (l + sgn * fabs(l)); };
     const R l1 = part(S.un), l2 = part(S.un + c), l3 = part(S.un - c);
     const R k = S.r / (R(2) * g);
@@ -522,23 +562,25 @@ NS3D_HD void cell_eigen(const R *w, R g, R Lm[5][5], R Rm[5][5]) {
     const R nx = DIR == 0 ? R(1) : R(0), ny = DIR == 1 ? R(1) : R(0), nz = DIR == 2 ? R(1) : R(0);
     const R gm1 = g - R(1);
     R r = w[0], u = w[1], v = w[2], ww = w[3], p = w[4];
-    R E = r * (R(0.5) * (u * u + v * v + ww * ww) + p / (gm1 * r));
-    R sq = sqrt(r);
+    R E = r * (R(0.5) * (u * u + v * v + ww * ww) + quot_(p, gm1 * r));
+    R sq = sqrt_(r);
     R rb = sq * sq;
-    R den = R(1) / (sq + sq);
+    R den = rcp_(sq + sq);
     R ub = (sq * u + sq * u) * den, vb = (sq * v + sq * v) * den, wb = (sq * ww + sq * ww) * den;
-    R H = (E + p) / r;
+    R H = quot_(E + p, r);
     R Hb = (sq * H + sq * H) * den;
-    R c = sqrt(gm1 * (Hb - R(0.5) * (ub * ub + vb * vb + wb * wb)));
+    R c = sqrt_(gm1 * (Hb - R(0.5) * (ub * ub + vb * vb + wb * wb)));
     R V = nx * ub + ny * vb + nz * wb;
     R phi = R(0.5) * gm1 * (ub * ub + vb * vb + wb * wb);
     R a1 = gm1;
-    R a2 = R(1) / (sqrt(R(2)) * rb * c);
-    R a3 = rb / (sqrt(R(2)) * c);
-    R a4 = (phi + c * c) / gm1;
-    R ic2 = R(1) / (c * c), irb = R(1) / rb;
+    const R ic = rcp_(c), irb = rcp_(rb);
+    R a2 = R(M_SQRT1_2) * irb * ic;
+    R a3 = R(M_SQRT1_2) * rb * ic;
+    const R igm1 = rcp_(gm1);
+    R a4 = (phi + c * c) * igm1;
+    R ic2 = ic * ic;
     R a5 = R(1) - phi * ic2;
-    R a6 = phi / gm1;
+    R a6 = phi * igm1;
     Lm[0][0] = a2 * (phi + c * V); Lm[0][1] = -a2 * (a1 * ub + nx * c); Lm[0][2] = -a2 * (a1 * vb + ny * c);
     Lm[0][3] = -a2 * (a1 * wb + nz * c); Lm[0][4] = a1 * a2;
     Lm[1][0] = nx * a5 - (nz * vb - ny * wb) * irb; Lm[1][1] = nx * a1 * ub * ic2;
