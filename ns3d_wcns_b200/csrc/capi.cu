@@ -687,8 +687,7 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
     h->launches += 1;
     CK(h, cudaGetLastError(), "ghost kernel");
     if (stage == 3) {
-        const int gx = (h->L64.nx + SweepGeom<2, double>::NLINE - 1) / SweepGeom<2, double>::NLINE;
-        h->cfl_count = (long)gx * h->L64.ny;  // z-sweep blocks
+        h->cfl_count = sweep_z_blocks(sweep_args<double>(h, 2));
         h->cfl_valid = true;
     }
     return NS3D_OK;
