@@ -84,6 +84,58 @@ NS3D_HD R weno5(R f0, R f1, R f2, R f3, R f4) {
     return quot_(a0 * p0 + a1 * p1 + a2 * p2, R(8) * (a0 + a1 + a2));
 }
 
+// Both states of a face: weno5 of f0..f4 and of the reversed f5..f1, through
+// the first and second differences that the two share.  With D_k = f_k -
+// f_{k-1} and S_k = D_{k+1} - D_k, the three candidates of the left state are
+// f2 + (7 D2 - 3 D1)/8, f2 + (D2 + 3 D3)/8 and f2 + (5 D3 - D4)/8, their
+// smoothness indicators 13/12 S^2 plus a quarter of (3 D2 - D1)^2, (D2 +
+// D3)^2 and (D4 - 3 D3)^2: interpolation.cpp:86-115 term by term, the weights
+// 1/16, 5/8, 5/16 as 0.1, 1, 0.5.  About 85 operations for the pair instead
+// of 110 (256^3, WENO5 + Roe: x-sweep 1.207 -> 1.072 ms, y 1.034 -> 0.886).
+// V: a scalar or a pair of lines; o: its operations.
+template <typename V, typename A>
+NS3D_HD void weno5_pair(const A &o, V f0, V f1, V f2, V f3, V f4, V f5, V &left, V &right) {
+    const V d1 = o.sub(f1, f0), d2 = o.sub(f2, f1), d3 = o.sub(f3, f2), d4 = o.sub(f4, f3), d5 = o.sub(f5, f4);
+    auto sq = [&](V a, V b) {  // eps + 13/12 (b - a)^2
+        const V s = o.sub(b, a);
+        return o.fma(o.mul(o.c(13.0 / 12.0), s), s, o.c(1e-6));
+    };
+    const V s1 = sq(d1, d2), s2 = sq(d2, d3), s3 = sq(d3, d4), s4 = sq(d4, d5);
+    // one side: g = the value nearest the face, e1 .. e4 the differences
+    // towards it and on, t0 .. t2 the three eps + 13/12 S^2
+    auto side = [&](V g, V e1, V e2, V e3, V e4, V t0, V t1, V t2) {
+        auto ind = [&](V u, V t) {  // (eps + beta)^2
+            const V b = o.fma(o.mul(o.c(0.25), u), u, t);
+            return o.mul(b, b);
+        };
+        const V m0 = ind(o.fma(o.c(3.0), e2, o.neg(e1)), t0), m1 = ind(o.add(e2, e3), t1),
+                m2 = ind(o.fma(o.c(-3.0), e3, e4), t2);
+        // alpha_k = d_k / m_k, all times m0 m1 m2 / d_1
+        const V a0 = o.mul(o.mul(o.c(0.1), m1), m2), a1 = o.mul(m0, m2), a2 = o.mul(o.mul(o.c(0.5), m0), m1);
+        const V p0 = o.fma(o.c(7.0), e2, o.mul(o.c(-3.0), e1)), p1 = o.fma(o.c(3.0), e3, e2), p2 = o.fma(o.c(5.0), e3, o.neg(e4));
+        const V num = o.fma(a0, p0, o.fma(a1, p1, o.mul(a2, p2)));
+        return o.add_quot(g, num, o.mul(o.c(8.0), o.add(a0, o.add(a1, a2))));
+    };
+    left = side(f2, d1, d2, d3, d4, s1, s2, s3);
+    right = side(f3, o.neg(d5), o.neg(d4), o.neg(d3), o.neg(d2), s4, s3, s2);
+}
+template <typename R>
+struct ScalarOps {
+    NS3D_HD R c(double x) const { return R(x); }
+    NS3D_HD R neg(R a) const { return -a; }
+    NS3D_HD R add(R a, R b) const { return a + b; }
+    NS3D_HD R sub(R a, R b) const { return a - b; }
+    NS3D_HD R mul(R a, R b) const { return a * b; }
+    NS3D_HD R fma(R a, R b, R d) const { return a * b + d; }
+    // g + a / b
+    NS3D_HD R add_quot(R g, R a, R b) const {
+#ifdef __CUDA_ARCH__
+        if constexpr (sizeof(R) == 8) return __fma_rn(a, rcp_fp64(b), g);
+#endif
+        return g + a / b;
+    }
+};
+
 // mdcd_linear_interpolate, interpolation.cpp:118-133.
 template <typename R>
 NS3D_HD R mdcd_linear(const R *c, R f0, R f1, R f2, R f3, R f4, R f5) {
@@ -263,6 +315,10 @@ NS3D_HD void face_pair(const SchemeParams<R> &sp, const R *f, R &L, R &Rr) {
         }
         return;
     }
+    if (it == I_WENO5) {
+        weno5_pair<R>(ScalarOps<R>(), f[0], f[1], f[2], f[3], f[4], f[5], L, Rr);
+        return;
+    }
     L = interp_side<R, INTERP>(sp, f, false);
     Rr = interp_side<R, INTERP>(sp, f, true);
 }
@@ -330,19 +386,18 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     l0 = l0 < delta ? (l0 * l0 + d2) * i2d : l0;
     lv = lv < delta ? (lv * lv + d2) * i2d : lv;
     l4 = l4 < delta ? (l4 * l4 + d2) * i2d : l4;
-    R k0 = (l0 - lv) * A0, k4 = (l4 - lv) * A4;
+    const R k0 = (l0 - lv) * A0, k4 = (l4 - lv) * A4, ks = k0 + k4, kd = (k4 - k0) * c;
     // R0 = (1, u-nc, v-nc, w-nc, H-cV), R4 = (1, u+nc, v+nc, w+nc, H+cV)
-    R cx = DIR == 0 ? c : R(0), cy = DIR == 1 ? c : R(0), cz = DIR == 2 ? c : R(0);
-    R D0 = lv * dU[0] + k0 + k4;
-    R D1 = lv * dU[1] + k0 * (ub - cx) + k4 * (ub + cx);
-    R D2 = lv * dU[2] + k0 * (vb - cy) + k4 * (vb + cy);
-    R D3 = lv * dU[3] + k0 * (wb - cz) + k4 * (wb + cz);
-    R D4 = lv * dU[4] + k0 * (Hb - c * V) + k4 * (Hb + c * V);
-    F[0] = R(0.5) * (FL[0] + FR[0]) - R(0.5) * D0;
-    F[1] = R(0.5) * (FL[1] + FR[1]) - R(0.5) * D1;
-    F[2] = R(0.5) * (FL[2] + FR[2]) - R(0.5) * D2;
-    F[3] = R(0.5) * (FL[3] + FR[3]) - R(0.5) * D3;
-    F[4] = R(0.5) * (FL[4] + FR[4]) - R(0.5) * D4;
+    R D0 = lv * dU[0] + ks;
+    R D1 = lv * dU[1] + ks * ub + (DIR == 0 ? kd : R(0));
+    R D2 = lv * dU[2] + ks * vb + (DIR == 1 ? kd : R(0));
+    R D3 = lv * dU[3] + ks * wb + (DIR == 2 ? kd : R(0));
+    R D4 = lv * dU[4] + ks * Hb + kd * V;
+    F[0] = R(0.5) * (FL[0] + FR[0] - D0);
+    F[1] = R(0.5) * (FL[1] + FR[1] - D1);
+    F[2] = R(0.5) * (FL[2] + FR[2] - D2);
+    F[3] = R(0.5) * (FL[3] + FR[3] - D3);
+    F[4] = R(0.5) * (FL[4] + FR[4] - D4);
 }
 
 // Rusanov_Riemann_solver, InviscousFlux.cpp:270-311.
