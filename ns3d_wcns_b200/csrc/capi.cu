@@ -500,7 +500,8 @@ template <typename R>
 int visc_launch(ns3d_handle *h, double *red, long *nblocks = nullptr) {
     ViscArgs<R> va = visc_args<R>(h);
     va.red = red;
-    dim3 g((va.L.nx + VTX - 1) / VTX, (va.L.ny + VTY - 1) / VTY, (va.zhi - va.zlo + VZC - 1) / VZC);
+    va.zc = visc_planes(va.L, va.zhi - va.zlo);
+    dim3 g((va.L.nx + VTX - 1) / VTX, (va.L.ny + VTY - 1) / VTY, (va.zhi - va.zlo + va.zc - 1) / va.zc);
     if (nblocks) *nblocks = (long)g.x * g.y * g.z;
     ViscMaps maps;
     for (int q = 0; q < 3; ++q) maps.m[q] = sizeof(R) == 8 ? h->tmW64[h->s0][q] : h->tmW32[q];
@@ -1043,7 +1044,7 @@ int ns3d_create(const ns3d_params *params, const ns3d_grid *grid, ns3d_handle **
     bytes += 2 * (((size_t)h->cfl_nblocks * 8 + 255) / 256 * 256);  // stage CFL minima, kinetic energy
     bytes += 256;                                              // device clock
     {
-        const long vb = (long)((grid->nx + VTX - 1) / VTX) * ((grid->ny + VTY - 1) / VTY) * ((grid->nz + VZC - 1) / VZC);
+        const long vb = (long)((grid->nx + VTX - 1) / VTX) * ((grid->ny + VTY - 1) / VTY) * ((grid->nz + VZC_MIN - 1) / VZC_MIN);
         h->visc_nblocks = vb;
         bytes += ((size_t)vb * 5 * 8 + 255) / 256 * 256;      // viscous-kernel diagnostics sums
     }

@@ -45,6 +45,7 @@ struct ViscArgs {
     double *red;
     int rlo, rhi;
     double vol;
+    int zc;                 // planes a block marches (visc_planes)
 };
 
 // choose_scheme, ViscousFlux.cpp:33-50 (idx relative to the first interior node)
@@ -75,7 +76,7 @@ __device__ __forceinline__ R sutherland(R mu0, R S, R T) {
     return mu0 * (T * sqrt(T)) * (R(1) + S) / (T + S);
 }
 
-constexpr int VTX = 32, VTY = 8, VH = NG, VZC = 32;
+constexpr int VTX = 32, VTY = 8, VH = NG, VZC = 32, VZC_MIN = 2;
 
 // First derivative of the window value f(o), o in [-3, 3], with a block-
 // uniform order; the offsets stay compile-time so the window lives in
@@ -101,12 +102,24 @@ __device__ __forceinline__ R dtile(F f, int order, const R *dinv) {
     return (-f(2) + R(8) * f(1) - R(8) * f(-1) + f(-2)) * dinv[1];
 }
 
-// A block owns a 32 x 8 column of nodes and marches up VZC planes: each
+// A block owns a 32 x 8 column of nodes and marches up zc planes: each
 // thread keeps its node's (u, v, w, T) of planes k-3 .. k+3 in registers and
 // loads one new plane per step (prefetched a step ahead); the x/y derivatives
 // read the plane's tile with its 3-cell halo, which one thread requests as
 // four TMA boxes a plane ahead (double buffer, mbarrier completion, bounded
 // waits).
+// Planes per block: 32, halved while that leaves the chip with fewer than two
+// blocks per SM.  A block waits about a microsecond for each plane, so a small
+// grid is as slow as its longest column (16^3: 24 us with 16 planes, 9 with 2;
+// 64^3: 39 us with 32 planes, 15 with 8), while every block loads six planes
+// of its own to start with.
+inline int visc_planes(const Layout &L, int planes) {
+    const long columns = (long)((L.nx + VTX - 1) / VTX) * ((L.ny + VTY - 1) / VTY);
+    int zc = VZC;
+    while (zc > VZC_MIN && columns * ((planes + zc - 1) / zc) < 2 * 148) zc /= 2;
+    return zc;
+}
+
 // Tensor maps of u, v, w, T of the state being differenced (3-D: x = padded
 // element index, y = ghost-inclusive row, z = ghost-inclusive plane).
 struct ViscMaps {
@@ -138,7 +151,7 @@ __global__ void __launch_bounds__(VTX * VTY) viscous_flux_kernel(ViscArgs<R> a, 
     if (a.done && *a.done) return;  // uniform over the grid
     const Layout &L = a.L;
     const int x0 = blockIdx.x * VTX, y0 = blockIdx.y * VTY;
-    const int kb = a.zlo + blockIdx.z * VZC, ke = min(kb + VZC, a.zhi);
+    const int kb = a.zlo + blockIdx.z * a.zc, ke = min(kb + a.zc, a.zhi);
     const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
     const int tid = threadIdx.y * VTX + threadIdx.x;
     const bool in = i < L.nx && j < L.ny;
