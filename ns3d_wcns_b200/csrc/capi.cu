@@ -298,6 +298,10 @@ struct ns3d_handle {
     double *rhs64[5] = {};
     double *T64 = nullptr;
     float *w32[5] = {};
+    // mixed: the FP32 primitives the stencils read.  Between steps w32; during
+    // a step the fused z-sweep writes each stage's result to a buffer of its
+    // own, in FP64 state planes that are free at that time (w32_buffer)
+    int w32_cur = 0;
     float *rhs32[5] = {};
     float *T32 = nullptr;
     void *visc[9] = {};  // double (plain) or float (mixed), interior layout
@@ -307,7 +311,7 @@ struct ns3d_handle {
     int *dev_err = nullptr;       // device error word (a bounded device wait ran out)
     // TMA tensor maps of (u, v, w) per state buffer and of T (FP64 path), or of
     // the FP32 primitives and T (mixed path)
-    CUtensorMap tmW64[3][3], tmT64, tmW32[3], tmT32;
+    CUtensorMap tmW64[3][3], tmT64, tmW32[7][3], tmT32;
     double *cfl_part = nullptr;   // per-block CFL minima written by the last RK stage
     double *ke_part = nullptr;    // per-block kinetic energy written by the last RK stage
     long cfl_nblocks = 0;         // capacity of cfl_part / ke_part
@@ -401,13 +405,23 @@ void prof_end(ns3d_handle *h) {
     h->prof_open = -1;
 }
 
+// FP32 primitive buffers of the mixed path: 0 = w32; 1 + b = the first half of
+// the planes of state buffer b (stage 1's result, in the buffer that receives
+// the step's result only in stage 3); 4 + b = their second half (stage 2's
+// result, beside the stage increments in the first half).
+float *w32_buffer(ns3d_handle *h, int which, int q) {
+    if (which == 0) return h->w32[q];
+    const int b = (which - 1) % 3;
+    return reinterpret_cast<float *>(h->S[b][q]) + (which >= 4 ? h->L64.plane : 0);
+}
+
 template <typename R>
 SweepArgs<R> sweep_args(ns3d_handle *h, int dir) {
     SweepArgs<R> a;
     const bool m = sizeof(R) == 4;
     for (int q = 0; q < 5; ++q) {
         if constexpr (sizeof(R) == 8) { a.W[q] = h->S[h->s0][q]; a.Rhs[q] = h->rhs64[q]; }
-        else { a.W[q] = h->w32[q]; a.Rhs[q] = h->rhs32[q]; }
+        else { a.W[q] = w32_buffer(h, h->w32_cur, q); a.Rhs[q] = h->rhs32[q]; }
     }
     a.L = m ? h->L32 : h->L64;
     a.periodic = h->bc.periodic[dir];
@@ -465,7 +479,7 @@ ViscArgs<R> visc_args(ns3d_handle *h) {
     ViscArgs<R> a;
     for (int q = 0; q < 5; ++q) {
         if constexpr (sizeof(R) == 8) a.W[q] = h->S[h->s0][q];
-        else a.W[q] = h->w32[q];
+        else a.W[q] = w32_buffer(h, h->w32_cur, q);
     }
     for (int q = 0; q < 9; ++q) a.V[q] = (R *)h->visc[q];
     if constexpr (sizeof(R) == 8) a.T = h->T64; else a.T = h->T32;
@@ -504,7 +518,7 @@ int visc_launch(ns3d_handle *h, double *red, long *nblocks = nullptr) {
     dim3 g((va.L.nx + VTX - 1) / VTX, (va.L.ny + VTY - 1) / VTY, (va.zhi - va.zlo + va.zc - 1) / va.zc);
     if (nblocks) *nblocks = (long)g.x * g.y * g.z;
     ViscMaps maps;
-    for (int q = 0; q < 3; ++q) maps.m[q] = sizeof(R) == 8 ? h->tmW64[h->s0][q] : h->tmW32[q];
+    for (int q = 0; q < 3; ++q) maps.m[q] = sizeof(R) == 8 ? h->tmW64[h->s0][q] : h->tmW32[h->w32_cur][q];
     maps.m[3] = sizeof(R) == 8 ? h->tmT64 : h->tmT32;
     prof_begin(h, "viscous_flux");
     const bool p6 = va.periodic[0] && va.periodic[1] && va.periodic[2];
@@ -559,6 +573,7 @@ int compute_rhs_async(ns3d_handle *h) {
 int stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, double dt) {
     cudaStream_t st = h->stream;
     h->visc_valid = false;
+    h->w32_cur = 0;  // the mixed kernel writes w32
     dim3 g = cell_grid(h->L64, true, STAGE_THREADS);
     double *cfl = stage == 3 ? h->cfl_part : nullptr;  // the next step's CFL bound
     if (!h->mixed) {
@@ -611,12 +626,14 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
         // rk3_async's buffers: (1: s0, s0 -> b1), (2: s0, b1 -> b2), (3: s0, b2 -> b1)
         const int free_buf = 3 - src0 - (stage == 2 ? srcc : dst);
         if (free_buf < 0 || free_buf > 2 || free_buf == src0 || (stage != 2 && free_buf == dst)) return NS3D_ERR_STATE;
+        // the stage's result: dst == free_buf in stage 2
+        const int next = stage == 1 ? 1 + dst : (stage == 2 ? 4 + dst : 0);
         FusedStage f{};
         f.stage = stage;
         for (int q = 0; q < 5; ++q) {
             f.U0[q] = h->S[src0][q]; f.Uout[q] = h->S[dst][q];
             f.D[q] = reinterpret_cast<float *>(h->S[free_buf][q]);  // FP32 layout inside an FP64 plane
-            f.W32out[q] = h->w32[q];  // in place (the sweep defers the cells its wrap re-reads)
+            f.W32out[q] = w32_buffer(h, next, q);
         }
         f.T32out = h->T32;
         f.L64 = h->L64;
@@ -629,13 +646,15 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
         f.keep_rhs = stage == 3 && h->P.keep_rhs;
         h->cfl_valid = false;
         h->rhs_complete = false;
+        const long z_blocks = sweep_z_blocks(sweep_args<float>(h, 2));
         int r = rhs_impl<float>(h, &f);
         if (r) return r;
+        h->w32_cur = next;
         h->rhs_complete = f.keep_rhs != 0;
         StageArgsMixed a;
         for (int q = 0; q < 5; ++q) {
             a.U0[q] = h->S[src0][q]; a.Uc[q] = nullptr; a.Rhs[q] = h->rhs32[q];
-            a.Uout[q] = h->S[dst][q]; a.Wout[q] = h->w32[q]; a.D[q] = f.D[q];
+            a.Uout[q] = h->S[dst][q]; a.Wout[q] = f.W32out[q]; a.D[q] = f.D[q];
         }
         a.L = h->L64; a.L32 = h->L32; a.b = h->bc; a.dt = dt; a.gamma = h->ph.gamma; a.stage = stage;
         a.Tout = h->T32; a.Rgas = h->ph.Rgas;
@@ -649,8 +668,7 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
         h->launches += 1;
         CK(h, cudaGetLastError(), "ghost kernel");
         if (stage == 3) {
-            const int gx = (h->L32.nx + SweepGeom<2, float>::NLINE - 1) / SweepGeom<2, float>::NLINE;
-            h->cfl_count = (long)gx * h->L32.ny;  // z-sweep blocks
+            h->cfl_count = z_blocks;
             h->cfl_valid = true;
         }
         return NS3D_OK;
@@ -701,6 +719,7 @@ int rk3_async(ns3d_handle *h, double dt) {
     const int s0 = h->s0, b1 = (s0 + 1) % 3, b2 = (s0 + 2) % 3;
     auto fail_reset = [&](int r) {  // back to the step's start buffer
         h->s0 = s0;
+        h->w32_cur = 0;
         return r;
     };
     int r;
@@ -993,8 +1012,16 @@ int ns3d_create(const ns3d_params *params, const ns3d_grid *grid, ns3d_handle **
     h->zlo = 0;
     h->zhi = grid->nz;
     if (ghost_count(h->L64) >= (1L << 31)) { delete h; return NS3D_ERR_SIZE; }  // 32-bit ghost decode
-    // the mixed path's FP32 stage increments live inside an FP64 state plane
-    if ((size_t)h->L32.plane * 4 > (size_t)h->L64.plane * 8) { delete h; return NS3D_ERR_CONFIG; }
+    if (h->mixed) {
+        // one pitch for both layouts: an FP32 array takes half an FP64 plane
+        // (stage increments and intermediate primitives live there), and the
+        // two layouts' element indexes differ by a constant
+        Layout &L = h->L64;
+        L.px = h->L32.px;
+        const long n = (long)L.sz * L.sy * L.px;
+        L.plane = (n + 63) / 64 * 64;
+        if (h->L32.plane > L.plane) { delete h; return NS3D_ERR_CONFIG; }
+    }
     // derived constants, initialization.cpp:170-172, 194-197
     Phys &ph = h->ph;
     ph.gamma = params->gamma;
@@ -1102,7 +1129,9 @@ int ns3d_create(const ns3d_params *params, const ns3d_grid *grid, ns3d_handle **
                 for (int q = 0; q < 3 && ok; ++q) ok = encode_plane_map(&h->tmW64[b][q], h->S[b][q + 1], true, h->L64);
             if (ok) ok = encode_plane_map(&h->tmT64, h->T64, true, h->L64);
         } else {
-            for (int q = 0; q < 3 && ok; ++q) ok = encode_plane_map(&h->tmW32[q], h->w32[q + 1], false, h->L32);
+            for (int b = 0; b < 7 && ok; ++b)
+                for (int q = 0; q < 3 && ok; ++q)
+                    ok = encode_plane_map(&h->tmW32[b][q], w32_buffer(h, b, q + 1), false, h->L32);
             if (ok) ok = encode_plane_map(&h->tmT32, h->T32, false, h->L32);
         }
         if (!ok) {
@@ -1262,6 +1291,7 @@ static int finish_upload(ns3d_handle *h, int b, bool apply_bc) {
     const int dst = (b + 1) % 3, dst2 = (b + 2) % 3;
     int r;
     h->visc_valid = false;
+    h->w32_cur = 0;
     if (!h->mixed) {
         if (!apply_bc) {
             dim3 g = cell_grid(h->L64, true, 128);
@@ -1810,6 +1840,7 @@ int ns3d_rk3_stage(ns3d_handle *h, int stage, double dt) {
     const int dst = stage == 2 ? b2 : b1;
     if ((r = rk_stage_async(h, stage, s0, srcc, dst, dt))) {
         h->s0 = s0;
+        h->w32_cur = 0;
         h->step_start = -1;
         return r;
     }
@@ -1830,7 +1861,7 @@ int ns3d_device_fields(ns3d_handle *h, int what, void *ptrs[5], long layout[6]) 
     if (what == NS3D_PRIMITIVE && !h->mixed) {
         for (int q = 0; q < 5; ++q) ptrs[q] = h->S[h->s0][q];
     } else if (what == NS3D_PRIMITIVE && h->mixed) {
-        for (int q = 0; q < 5; ++q) ptrs[q] = h->w32[q];
+        for (int q = 0; q < 5; ++q) ptrs[q] = w32_buffer(h, h->w32_cur, q);
         L = &h->L32; esz = 4;
     } else if (what == NS3D_CONSERVED && h->mixed) {
         for (int q = 0; q < 5; ++q) ptrs[q] = h->S[h->s0][q];

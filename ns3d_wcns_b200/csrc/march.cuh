@@ -112,21 +112,6 @@ __device__ __forceinline__ T march_ld(const R *p) { return *reinterpret_cast<con
 
 // ------------------------------------------------------------------ one face
 
-// Variable q of six (or five) cells, q known only at run time: selects over
-// the register window, for the rare paths that loop over the variables (one
-// copy of their code instead of five: the loop over the cells has to stay in
-// the instruction cache).
-template <int NP, typename T>
-__device__ __forceinline__ void march_pick(const T (*u)[5], int q, T *f) {
-#pragma unroll
-    for (int k = 0; k < NP; ++k) {
-        f[k] = u[k][0];
-#pragma unroll
-        for (int r = 1; r < 5; ++r)
-            if (q == r) f[k] = u[k][r];
-    }
-}
-
 // Variables whose detector does not clearly accept the linear scheme at one
 // cell, from its five points u[m][q]: bit q (and q + 5 for a float2's second
 // line).  FP64: the two sides of the cross-multiplied test (mdcd_smooth, both
@@ -156,37 +141,96 @@ __device__ __forceinline__ unsigned march_doubt(const T (*u)[5]) {
     return r;
 }
 
-// The face's states for the variables in doubt (rare): FP64 first takes the
-// exact decisions; one copy of the WENO branch serves every variable, line
-// and side.
+// Position of the nth set bit (nth < popc(mask)).
+__device__ __forceinline__ int march_nth_bit(unsigned mask, int nth) {
+    int pos = 0;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+        const int c = __popc((mask >> pos) & ((1u << s) - 1u));
+        if (nth >= c) { nth -= c; pos += s; }
+    }
+    return pos;
+}
+__device__ __forceinline__ double march_shfl(double v, int src, int) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ float march_shfl(float v, int src, int) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ float march_shfl(float2 v, int src, int line) {
+    const float x = __shfl_sync(0xffffffffu, v.x, src), y = __shfl_sync(0xffffffffu, v.y, src);
+    return line ? y : x;
+}
+
+// The states of the variables in doubt, for a warp in which some lane has
+// one: every (lane, variable, line) in doubt is a task, the tasks are dealt
+// out over the 32 lanes, each fetches its stencil by shuffles, takes the
+// exact decision (FP64) and evaluates both sides, and the results go back.
+// An under-resolved flow has a few tasks at most faces; one round then
+// replaces a divergent branch per variable and side, which the whole warp
+// would walk through (64^3 decaying turbulence, y-sweep: 60 -> 41 us).
 template <typename T>
 __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5], unsigned doubt, T *UL, T *UR) {
     using R = typename LaneOf<T>::R;
+    constexpr int NV = 5 * LaneOf<T>::N;
+    const int lane = threadIdx.x & 31;
+    int total = 0;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) total += __popc(__ballot_sync(0xffffffffu, (doubt >> v) & 1u));
 #pragma unroll 1
-    for (int q = 0; q < 5; ++q) {
-        if (!(doubt & (33u << q))) continue;
-        T f[6];
-        march_pick<6>(u, q, f);
-        if constexpr (sizeof(R) == 8) {
-            if (mdcd_smooth(f[0], f[1], f[2], f[3], f[4]) && mdcd_smooth(f[1], f[2], f[3], f[4], f[5])) continue;
+    for (int base = 0; base < total; base += 32) {
+        int var = -1, nth = 0, off = base + lane;  // this lane's task
+        unsigned mask = 0;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const unsigned b = __ballot_sync(0xffffffffu, (doubt >> v) & 1u);
+            const int c = __popc(b);
+            if (off >= 0 && off < c) { var = v; mask = b; nth = off; }
+            off -= c;
         }
-#pragma unroll 1
-        for (int h = 0; h < 2 * LaneOf<T>::N; ++h) {  // side, line
-            const int line = h >> 1;
-            if (!(doubt & ((line ? 32u : 1u) << q))) continue;
-            R g[6];
+        const int src = march_nth_bit(mask, nth) & 31, line = var >= 5, q0 = line ? var - 5 : var;
+        R g[6];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) g[k] = march_half((h & 1) ? f[5 - k] : f[k], line);
-            const R v = mdcd_weno_branch(m.a.sp.hd, g[0], g[1], g[2], g[3], g[4], g[5]);
+        for (int k = 0; k < 6; ++k) g[k] = R(0);
 #pragma unroll
-            for (int k = 0; k < 5; ++k)
-                if (k == q) {
-                    if (h & 1) march_set(UR[k], line, v);
-                    else march_set(UL[k], line, v);
-                }
+        for (int q = 0; q < 5; ++q) {
+            if (!__any_sync(0xffffffffu, q0 == q)) continue;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const R x = march_shfl(u[k][q], src, line);
+                if (q0 == q) g[k] = x;
+            }
+        }
+        bool keep = false;  // the linear states stay
+        if constexpr (sizeof(R) == 8)
+            keep = mdcd_smooth(g[0], g[1], g[2], g[3], g[4]) && mdcd_smooth(g[1], g[2], g[3], g[4], g[5]);
+        const R l = mdcd_weno_branch(m.a.sp.hd, g[0], g[1], g[2], g[3], g[4], g[5]);
+        const R r = mdcd_weno_branch(m.a.sp.hd, g[5], g[4], g[3], g[2], g[1], g[0]);
+        int from = -base;  // the task of this lane's variable v sits in lane `from` + its rank
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const unsigned b = __ballot_sync(0xffffffffu, (doubt >> v) & 1u);
+            if (!b) continue;
+            const int t = from + __popc(b & ((1u << lane) - 1u));
+            const R lv = __shfl_sync(0xffffffffu, l, t & 31), rv = __shfl_sync(0xffffffffu, r, t & 31);
+            const bool kv = __shfl_sync(0xffffffffu, (int)keep, t & 31);
+            if (((doubt >> v) & 1u) && t >= 0 && t < 32 && !kv) {
+                march_set(UL[v % 5], v / 5, lv);
+                march_set(UR[v % 5], v / 5, rv);
+            }
+            from += __popc(b);
         }
     }
 }
+
+// Paired arithmetic of two lines, for the templates of schemes.cuh
+struct PairOps {
+    __device__ __forceinline__ float2 c(double x) const { return p2((float)x); }
+    __device__ __forceinline__ float2 neg(float2 a) const { return make_float2(-a.x, -a.y); }
+    __device__ __forceinline__ float2 add(float2 a, float2 b) const { return add2(a, b); }
+    __device__ __forceinline__ float2 sub(float2 a, float2 b) const { return sub2(a, b); }
+    __device__ __forceinline__ float2 mul(float2 a, float2 b) const { return mul2(a, b); }
+    __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 d) const { return fma2(a, b, d); }
+    __device__ __forceinline__ float2 add_quot(float2 g, float2 a, float2 b) const {
+        return make_float2(g.x + a.x / b.x, g.y + a.y / b.y);
+    }
+};
 
 // Left and right states of the face between u[2] and u[3]; doubt: march_doubt
 // of the two cells (MDCD_HYBRID).
@@ -195,15 +239,10 @@ __device__ __forceinline__ void march_states(const MarchArgs<T> &m, const T (*u)
     if constexpr (INTERP == I_WENO5) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
-            if constexpr (LaneOf<T>::N == 2) {
-                UL[q] = make_float2(weno5(u[0][q].x, u[1][q].x, u[2][q].x, u[3][q].x, u[4][q].x),
-                                    weno5(u[0][q].y, u[1][q].y, u[2][q].y, u[3][q].y, u[4][q].y));
-                UR[q] = make_float2(weno5(u[5][q].x, u[4][q].x, u[3][q].x, u[2][q].x, u[1][q].x),
-                                    weno5(u[5][q].y, u[4][q].y, u[3][q].y, u[2][q].y, u[1][q].y));
-            } else {
-                UL[q] = weno5(u[0][q], u[1][q], u[2][q], u[3][q], u[4][q]);
-                UR[q] = weno5(u[5][q], u[4][q], u[3][q], u[2][q], u[1][q]);
-            }
+            if constexpr (LaneOf<T>::N == 2)
+                weno5_pair<T>(PairOps(), u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q], UL[q], UR[q]);
+            else
+                weno5_pair<T>(ScalarOps<T>(), u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q], UL[q], UR[q]);
         }
     } else {
 #pragma unroll
@@ -217,7 +256,7 @@ __device__ __forceinline__ void march_states(const MarchArgs<T> &m, const T (*u)
             }
         }
         if constexpr (INTERP == I_MDCD_HYBRID) {
-            if (doubt) march_weno<T>(m, u, doubt, UL, UR);
+            if (__any_sync(0xffffffffu, doubt != 0)) march_weno<T>(m, u, doubt, UL, UR);
         }
     }
 }
@@ -648,6 +687,22 @@ inline cudaError_t launch_march(const SweepArgs<typename LaneOf<T>::R> &a, cudaS
     march_kernel<DIR, T, INTERP, RS><<<grid, MARCH_NT, smem, st>>>(m);
     return cudaGetLastError();
 }
+
+template <int DIR, typename T>
+inline long march_blocks(const SweepArgs<typename LaneOf<T>::R> &a) {
+    MarchArgs<T> m;
+    const dim3 g = march_grid<DIR, T>(a, m);
+    return (long)g.x * g.y;
+}
+template <int DIR, typename R>
+inline long sweep_blocks(const SweepArgs<R> &a) {
+    return (long)((a.L.nx + SweepGeom<DIR, R>::NLINE - 1) / SweepGeom<DIR, R>::NLINE) * a.L.ny;
+}
+
+// Component-wise schemes march; characteristic reconstruction, whose bases
+// and projections want the registers, keeps the chunked kernel.
+inline bool march_takes(const SweepArgs<double> &a) { return !a.sp.char_recon; }
+inline bool march_takes(const SweepArgs<float> &a) { return !a.sp.char_recon && !sweep32_scalar_forced(); }
 
 // The scheme's instantiation: the interpolation always compiled in, the
 // Riemann solver for the schemes' usual partners.

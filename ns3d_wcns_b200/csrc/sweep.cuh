@@ -768,6 +768,7 @@ cudaError_t sweep_x(const SweepArgs<double> &, cudaStream_t);
 cudaError_t sweep_y(const SweepArgs<double> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<double> &, cudaStream_t);
 long sweep_z_blocks(const SweepArgs<double> &);
+long sweep_z_blocks(const SweepArgs<float> &);
 cudaError_t sweep_x(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_y(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<float> &, cudaStream_t);

@@ -4,7 +4,10 @@
 
 namespace ns3d {
 cudaError_t sweep_y(const SweepArgs<double> &a, cudaStream_t st) {
-    return a.sp.char_recon ? sweep_select<1, double>(a, st) : march_select<1, double>(a, st);
+    return march_takes(a) ? march_select<1, double>(a, st) : sweep_select<1, double>(a, st);
 }
-cudaError_t sweep_y(const SweepArgs<float> &a, cudaStream_t st) { return sweep_select_f32<1>(a, st); }
+cudaError_t sweep_y(const SweepArgs<float> &a, cudaStream_t st) {
+    if (!march_takes(a)) return sweep_select<1, float>(a, st);
+    return a.L.nx & 1 ? march_select<1, float>(a, st) : march_select<1, float2>(a, st);
+}
 }  // namespace ns3d

@@ -4,15 +4,19 @@
 
 namespace ns3d {
 cudaError_t sweep_z(const SweepArgs<double> &a, cudaStream_t st) {
-    return a.sp.char_recon ? sweep_select<2, double>(a, st) : march_select<2, double>(a, st);
+    return march_takes(a) ? march_select<2, double>(a, st) : sweep_select<2, double>(a, st);
 }
-cudaError_t sweep_z(const SweepArgs<float> &a, cudaStream_t st) { return sweep_select_f32<2>(a, st); }
+cudaError_t sweep_z(const SweepArgs<float> &a, cudaStream_t st) {
+    if (!march_takes(a)) return sweep_select<2, float>(a, st);
+    return a.L.nx & 1 ? march_select<2, float>(a, st) : march_select<2, float2>(a, st);
+}
 
 // blocks of the z-sweep: the partials its fused stage 3 writes
 long sweep_z_blocks(const SweepArgs<double> &a) {
-    if (a.sp.char_recon) return (long)((a.L.nx + SweepGeom<2, double>::NLINE - 1) / SweepGeom<2, double>::NLINE) * a.L.ny;
-    MarchArgs<double> m;
-    const dim3 g = march_grid<2, double>(a, m);
-    return (long)g.x * g.y;
+    return march_takes(a) ? march_blocks<2, double>(a) : sweep_blocks<2, double>(a);
+}
+long sweep_z_blocks(const SweepArgs<float> &a) {
+    if (!march_takes(a)) return sweep_blocks<2, float>(a);
+    return a.L.nx & 1 ? march_blocks<2, float>(a) : march_blocks<2, float2>(a);
 }
 }  // namespace ns3d
