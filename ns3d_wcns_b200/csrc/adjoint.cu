@@ -33,6 +33,13 @@ __device__ __forceinline__ int wrapn(int i, int n) { return i < 0 ? i + n : (i >
 struct Idx {
     int nx, ny, nz;
     __device__ __forceinline__ long at(int i, int j, int k) const { return ((long)k * ny + j) * nx + i; }
+    // cell number (below 2^31 cells) -> coordinates, in 32-bit arithmetic
+    __device__ __forceinline__ void split(long t, int &i, int &j, int &k) const {
+        const unsigned u = (unsigned)t, row = u / (unsigned)nx;
+        i = (int)(u - row * (unsigned)nx);
+        k = (int)(row / (unsigned)ny);
+        j = (int)(row - (unsigned)k * (unsigned)ny);
+    }
 };
 
 // interior (i,j,k) shifted by o along d, periodic
@@ -65,7 +72,8 @@ __global__ void __launch_bounds__(ADJ_T) adj_face_kernel(AdjArgs a) {
     const long nface = (long)I.nx * I.ny * I.nz;
     const long t = (long)blockIdx.x * blockDim.x + tid;
     if (t >= nface) return;
-    const int i = (int)(t % I.nx), j = (int)((t / I.nx) % I.ny), k = (int)(t / ((long)I.nx * I.ny));
+    int i, j, k;
+    I.split(t, i, j, k);
     // face j' + 1/2 along DIR with j' = the cell coordinate along DIR
     const double ih = a.inv_h[DIR];
     double Fb[5];
@@ -138,9 +146,10 @@ __global__ void __launch_bounds__(256) adj_line_kernel(AdjArgs a, int lpb, int f
     const long g = (long)blockIdx.x * lpb + l;
     const bool ok = g < nlines;
     int i, j, k;
-    if (DIR == 0) { i = c; j = (int)(g % I.ny); k = (int)(g / I.ny); }
-    else if (DIR == 1) { i = (int)(g % I.nx); j = c; k = (int)(g / I.nx); }
-    else { i = (int)(g % I.nx); j = (int)(g / I.nx); k = c; }
+    const unsigned across = DIR == 0 ? I.ny : I.nx, g_hi = (unsigned)g / across, g_lo = (unsigned)g - g_hi * across;
+    if (DIR == 0) { i = c; j = (int)g_lo; k = (int)g_hi; }
+    else if (DIR == 1) { i = (int)g_lo; j = c; k = (int)g_hi; }
+    else { i = (int)g_lo; j = (int)g_hi; k = c; }
     const long tc = ok ? I.at(i, j, k) : 0;
     if (ok) {
         double Uc[5];
@@ -225,7 +234,8 @@ __global__ void __launch_bounds__(128) adj_face_gather_kernel(AdjArgs a, int fir
     const long ncell = (long)I.nx * I.ny * I.nz;
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ncell) return;
-    const int i = (int)(t % I.nx), j = (int)((t / I.nx) % I.ny), k = (int)(t / ((long)I.nx * I.ny));
+    int i, j, k;
+    I.split(t, i, j, k);
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
         double s = first ? 0.0 : a.Ub[q][t];
@@ -241,7 +251,7 @@ __global__ void __launch_bounds__(128) adj_face_gather_kernel(AdjArgs a, int fir
 __device__ __forceinline__ void prim4(const AdjArgs &a, int i, int j, int k, double x[4]) {
     const long c = a.L.at(i + NG, j + NG, k + NG);
     x[0] = a.W[1][c]; x[1] = a.W[2][c]; x[2] = a.W[3][c];
-    x[3] = a.W[4][c] / (a.W[0][c] * a.Rgas);
+    x[3] = a.W[4][c] * rcp_fp64(a.W[0][c] * a.Rgas);
 }
 
 __global__ void __launch_bounds__(128) adj_visc_node_kernel(AdjArgs a) {
@@ -249,7 +259,8 @@ __global__ void __launch_bounds__(128) adj_visc_node_kernel(AdjArgs a) {
     const long ncell = (long)I.nx * I.ny * I.nz;
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ncell) return;
-    const int i = (int)(t % I.nx), j = (int)((t / I.nx) % I.ny), k = (int)(t / ((long)I.nx * I.ny));
+    int i, j, k;
+    I.split(t, i, j, k);
     // node-flux adjoint: transpose of D_d (antisymmetric) applied to rhs adjoints
     auto DT = [&](const double *r, int d) {
         double s = 0.0;
@@ -301,7 +312,8 @@ __global__ void __launch_bounds__(128) adj_visc_gather_kernel(AdjArgs a) {
     const long ncell = (long)I.nx * I.ny * I.nz;
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ncell) return;
-    const int i = (int)(t % I.nx), j = (int)((t / I.nx) % I.ny), k = (int)(t / ((long)I.nx * I.ny));
+    int i, j, k;
+    I.split(t, i, j, k);
     double xb[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -320,12 +332,12 @@ __global__ void __launch_bounds__(128) adj_visc_gather_kernel(AdjArgs a) {
     const long c = a.L.at(i + NG, j + NG, k + NG);
     const double rho = a.W[0][c], u = a.W[1][c], v = a.W[2][c], w = a.W[3][c], p = a.W[4][c];
     const double gm1 = a.gamma - 1.0;
-    const double E = p / gm1 + 0.5 * rho * (u * u + v * v + w * w);
-    const double irR = 1.0 / (rho * a.Rgas);
-    a.Ub[0][t] += -(u * xb[0] + v * xb[1] + w * xb[2]) / rho + xb[3] * gm1 * irR * (u * u + v * v + w * w - E / rho);
-    a.Ub[1][t] += xb[0] / rho - xb[3] * gm1 * u * irR;
-    a.Ub[2][t] += xb[1] / rho - xb[3] * gm1 * v * irR;
-    a.Ub[3][t] += xb[2] / rho - xb[3] * gm1 * w * irR;
+    const double E = p * rcp_fp64(gm1) + 0.5 * rho * (u * u + v * v + w * w);
+    const double ir = rcp_fp64(rho), irR = rcp_fp64(rho * a.Rgas);
+    a.Ub[0][t] += -(u * xb[0] + v * xb[1] + w * xb[2]) * ir + xb[3] * gm1 * irR * (u * u + v * v + w * w - E * ir);
+    a.Ub[1][t] += xb[0] * ir - xb[3] * gm1 * u * irR;
+    a.Ub[2][t] += xb[1] * ir - xb[3] * gm1 * v * irR;
+    a.Ub[3][t] += xb[2] * ir - xb[3] * gm1 * w * irR;
     a.Ub[4][t] += xb[3] * gm1 * irR;
 }
 
@@ -341,7 +353,8 @@ __global__ void ke_seed_kernel(AdjArgs a, double vol, double *const *Ub) {
     const Idx I{a.L.nx, a.L.ny, a.L.nz};
     const long ncell = (long)I.nx * I.ny * I.nz;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ncell; t += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % I.nx), j = (int)((t / I.nx) % I.ny), k = (int)(t / ((long)I.nx * I.ny));
+        int i, j, k;
+    I.split(t, i, j, k);
         const long c = a.L.at(i + NG, j + NG, k + NG);
         const double u = a.W[1][c], v = a.W[2][c], w = a.W[3][c];
         // J = sum 0.5 |m|^2 / rho * vol (postprocess.cpp:119-122)
@@ -356,7 +369,8 @@ __global__ void velocity_grad_kernel(AdjArgs a, const double *const *Ub, double 
     const Idx I{a.L.nx, a.L.ny, a.L.nz};
     const long ncell = (long)I.nx * I.ny * I.nz;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ncell; t += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(t % I.nx), j = (int)((t / I.nx) % I.ny), k = (int)(t / ((long)I.nx * I.ny));
+        int i, j, k;
+    I.split(t, i, j, k);
         const long c = a.L.at(i + NG, j + NG, k + NG);
         const double rho = a.W[0][c];
         for (int q = 0; q < 3; ++q) gvel[q][t] = rho * Ub[1 + q][t] + rho * a.W[1 + q][c] * Ub[4][t];

@@ -29,24 +29,7 @@ namespace adj {
 
 // ----------------------------------------------------------- interpolation
 
-// Forward WENO5 (same function as schemes.cuh's weno5) and its VJP:
-// f[0..4] -> q; fb[0..4] += dq/df * qb.
-template <typename R>
-NS3D_HD R weno5_fwd(const R *f) {
-    const R eps = R(1e-6), c13 = R(13.0 / 12.0);
-    R t0 = f[0] - R(2) * f[1] + f[2], u0 = f[0] - R(4) * f[1] + R(3) * f[2];
-    R t1 = f[1] - R(2) * f[2] + f[3], u1 = f[1] - f[3];
-    R t2 = f[2] - R(2) * f[3] + f[4], u2 = R(3) * f[2] - R(4) * f[3] + f[4];
-    R b0 = c13 * t0 * t0 + R(0.25) * u0 * u0, b1 = c13 * t1 * t1 + R(0.25) * u1 * u1;
-    R b2 = c13 * t2 * t2 + R(0.25) * u2 * u2;
-    R s0 = (eps + b0) * (eps + b0), s1 = (eps + b1) * (eps + b1), s2 = (eps + b2) * (eps + b2);
-    R a0 = R(1.0 / 16.0) * s1 * s2, a1 = R(5.0 / 8.0) * s0 * s2, a2 = R(5.0 / 16.0) * s0 * s1;
-    R p0 = R(3) * f[0] - R(10) * f[1] + R(15) * f[2];
-    R p1 = -f[1] + R(6) * f[2] + R(3) * f[3];
-    R p2 = R(3) * f[2] + R(6) * f[3] - f[4];
-    return (a0 * p0 + a1 * p1 + a2 * p2) / (R(8) * (a0 + a1 + a2));
-}
-
+// VJP of schemes.cuh's weno5: fb[0..4] += dq/df * qb.
 template <typename R>
 NS3D_HD void weno5_vjp(const R *f, R qb, R *fb) {
     const R eps = R(1e-6), c13 = R(13.0 / 12.0);
@@ -59,7 +42,8 @@ NS3D_HD void weno5_vjp(const R *f, R qb, R *fb) {
     R s0 = e0 * e0, s1 = e1 * e1, s2 = e2 * e2;
     R a0 = R(1.0 / 16.0) * s1 * s2, a1 = R(5.0 / 8.0) * s0 * s2, a2 = R(5.0 / 16.0) * s0 * s1;
     R A = a0 + a1 + a2;
-    R w0 = a0 / A, w1 = a1 / A, w2 = a2 / A;  // normalised weights
+    const R iA = rcp_(A);
+    R w0 = a0 * iA, w1 = a1 * iA, w2 = a2 * iA;  // normalised weights
     R p0 = (R(3) * f[0] - R(10) * f[1] + R(15) * f[2]) * R(0.125);
     R p1 = (-f[1] + R(6) * f[2] + R(3) * f[3]) * R(0.125);
     R p2 = (R(3) * f[2] + R(6) * f[3] - f[4]) * R(0.125);
@@ -72,9 +56,9 @@ NS3D_HD void weno5_vjp(const R *f, R qb, R *fb) {
     fb[3] += R(0.375) * pb1 + R(0.75) * pb2;
     fb[4] += R(-0.125) * pb2;
     // weights: alpha_k = d_k / e_k^2, d q / d beta_k = -2 w_k (p_k - q) / e_k
-    R bb0 = R(-2) * qb * w0 * (p0 - q) / e0;
-    R bb1 = R(-2) * qb * w1 * (p1 - q) / e1;
-    R bb2 = R(-2) * qb * w2 * (p2 - q) / e2;
+    R bb0 = quot_(R(-2) * qb * w0 * (p0 - q), e0);
+    R bb1 = quot_(R(-2) * qb * w1 * (p1 - q), e1);
+    R bb2 = quot_(R(-2) * qb * w2 * (p2 - q), e2);
     R tb, ub;
     tb = R(2) * c13 * t0 * bb0; ub = R(0.5) * u0 * bb0;
     fb[0] += tb + ub; fb[1] += R(-2) * tb - R(4) * ub; fb[2] += tb + R(3) * ub;
@@ -97,32 +81,33 @@ NS3D_HD void mdcd_weno_vjp(const R *f, const R *hd, R qb, R *fb) {
                      c13 * (t2 * t2) + R(0.25) * (u2 * u2), mdcd_beta3(f[0], f[1], f[2], f[3], f[4], f[5])};
     const R qk[4] = {R(3) * f[0] - R(10) * f[1] + R(15) * f[2], -f[1] + R(6) * f[2] + R(3) * f[3],
                      R(3) * f[2] + R(6) * f[3] - f[4], R(15) * f[3] - R(10) * f[4] + R(3) * f[5]};
-    const R D = be[3] - (be[0] + R(4) * be[1] + be[2]) / R(6);
+    const R D = be[3] - (be[0] + R(4) * be[1] + be[2]) * R(1.0 / 6.0);
     const R tau = fabs(D);
-    R g[4], al[4], A = R(0), Q = R(0);
+    R g[4], al[4], ib[4], A = R(0), Q = R(0);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        g[k] = R(20) + tau / (be[k] + es);
+        ib[k] = rcp_(be[k] + es);
+        g[k] = R(20) + tau * ib[k];
         al[k] = hd[k] * (g[k] * g[k]);
         A += al[k];
         Q += al[k] * qk[k];
     }
-    const R q = Q / (R(8) * A);
+    const R iA = rcp_(A);
+    const R q = R(0.125) * Q * iA;
     R qkb[4], beb[4], taub = R(0);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        qkb[k] = qb * al[k] / (R(8) * A);
-        const R alb = qb * (qk[k] * R(0.125) - q) / A;
+        qkb[k] = R(0.125) * qb * al[k] * iA;
+        const R alb = qb * (qk[k] * R(0.125) - q) * iA;
         const R gb = alb * R(2) * hd[k] * g[k];
-        const R ib = R(1) / (be[k] + es);
-        taub += gb * ib;
-        beb[k] = -gb * tau * ib * ib;
+        taub += gb * ib[k];
+        beb[k] = -gb * tau * ib[k] * ib[k];
     }
     const R Db = D >= R(0) ? taub : -taub;
     beb[3] += Db;
-    beb[0] -= Db / R(6);
-    beb[1] -= R(4) * Db / R(6);
-    beb[2] -= Db / R(6);
+    beb[0] -= Db * R(1.0 / 6.0);
+    beb[1] -= Db * R(4.0 / 6.0);
+    beb[2] -= Db * R(1.0 / 6.0);
     // candidates
     fb[0] += R(3) * qkb[0];
     fb[1] += R(-10) * qkb[0] - qkb[1];
@@ -138,7 +123,7 @@ NS3D_HD void mdcd_weno_vjp(const R *f, const R *hd, R qb, R *fb) {
     tb = R(2) * c13 * t2 * beb[2]; ub = R(0.5) * u2 * beb[2];
     fb[2] += tb + R(3) * ub; fb[3] += R(-2) * tb - R(4) * ub; fb[4] += tb + ub;
     // beta3: gradient of the quadratic form of interpolation.cpp:193-200
-    const R b3 = beb[3] / R(120960);
+    const R b3 = beb[3] * R(1.0 / 120960.0);
     fb[0] += b3 * (R(543598) * f[0] - R(2380800) * f[1] + R(4086352) * f[2] - R(3462252) * f[3] +
                    R(1458762) * f[4] - R(245620) * f[5]);
     fb[1] += b3 * (R(-2380800) * f[0] + R(11306634) * f[1] - R(20427884) * f[2] + R(17905032) * f[3] -
@@ -161,8 +146,7 @@ template <typename R, int INTERP>
 NS3D_HD void interp_pair_fwd(const R *f, const R *lin, const R *hd, R &l, R &r) {
     const R fr[6] = {f[5], f[4], f[3], f[2], f[1], f[0]};
     if constexpr (INTERP == 0) {
-        l = weno5_fwd(f);
-        r = weno5_fwd(fr);
+        weno5_pair<R>(ScalarOps<R>(), f[0], f[1], f[2], f[3], f[4], f[5], l, r);
         return;
     }
     if constexpr (INTERP == 3) {
@@ -217,7 +201,7 @@ struct SideF {
 template <typename R>
 NS3D_HD SideF<R> side_fwd(const R *U, R g) {
     SideF<R> s;
-    s.r = U[0]; s.ir = R(1) / s.r;
+    s.r = U[0]; s.ir = rcp_(s.r);
     s.u = U[1] * s.ir; s.v = U[2] * s.ir; s.w = U[3] * s.ir; s.E = U[4];
     s.q2 = s.u * s.u + s.v * s.v + s.w * s.w;
     s.p = (s.E - R(0.5) * s.r * s.q2) * (g - R(1));
@@ -267,7 +251,7 @@ NS3D_HD void pflux_vjp(const SideF<R> &s, const R *Fb, R &ub, R &vb, R &wb, R &p
 
 // entropy fix of Roe_Riemann_solver (InviscousFlux.cpp:364-373) on |lambda|
 template <typename R>
-NS3D_HD R efix(R l, R d) { return l < d ? (l * l + d * d) / (R(2) * d) : l; }
+NS3D_HD R efix(R l, R d) { return l < d ? quot_(l * l + d * d, R(2) * d) : l; }
 
 // Roe flux: same function as schemes.cuh roe_flux; VJP accumulates ULb, URb.
 template <int DIR, typename R>
@@ -275,13 +259,13 @@ NS3D_HD void roe_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
     const R gm1 = g - R(1), kfac = g / gm1;
     SideF<R> L = side_fwd(UL, g), Rs = side_fwd(UR, g);
     R HL = R(0.5) * L.q2 + kfac * L.p * L.ir, HR = R(0.5) * Rs.q2 + kfac * Rs.p * Rs.ir;
-    R sL = sqrt(L.r), sR = sqrt(Rs.r);
-    R den = R(1) / (sL + sR);
+    R sL = sqrt_(L.r), sR = sqrt_(Rs.r);
+    R den = rcp_(sL + sR);
     R ub = (sL * L.u + sR * Rs.u) * den, vb = (sL * L.v + sR * Rs.v) * den, wb = (sL * L.w + sR * Rs.w) * den;
     R Hb = (sL * HL + sR * HR) * den;
     R q2b = ub * ub + vb * vb + wb * wb;
     R c2 = gm1 * (Hb - R(0.5) * q2b);
-    R c = sqrt(c2);
+    R c = sqrt_(c2);
     R V = DIR == 0 ? ub : (DIR == 1 ? vb : wb);
     R phi = R(0.5) * gm1 * q2b;
     R dU[5];
@@ -290,7 +274,7 @@ NS3D_HD void roe_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
     const R dUn = dU[1 + DIR];
     R t = phi * dU[0] + gm1 * (dU[4] - ub * dU[1] - vb * dU[2] - wb * dU[3]);
     R s = c * (V * dU[0] - dUn);
-    R i2c2 = R(1) / (R(2) * c2);
+    R i2c2 = rcp_(R(2) * c2);
     R A0 = (t + s) * i2c2, A4 = (t - s) * i2c2;
     R l0 = fabs(V - c), lv = fabs(V), l4 = fabs(V + c);
     R delta = R(0.1) * (lv + c);
@@ -319,10 +303,11 @@ NS3D_HD void roe_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
     R A0b = k0b * (l0f - lvf), A4b = k4b * (l4f - lvf);
     // entropy fix
     R deltab = R(0);
+    const R idelta = rcp_(delta);
     auto fixb = [&](R l, R lfb) -> R {  // returns lb, accumulates deltab
         if (l < delta) {
-            deltab += lfb * (R(0.5) - l * l / (R(2) * delta * delta));
-            return lfb * l / delta;
+            deltab += lfb * (R(0.5) - R(0.5) * l * l * idelta * idelta);
+            return lfb * l * idelta;
         }
         return lfb;
     };
@@ -348,7 +333,7 @@ NS3D_HD void roe_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
     ubb -= tb * gm1 * dU[1]; vbb -= tb * gm1 * dU[2]; wbb -= tb * gm1 * dU[3];
     R q2bb = R(0.5) * gm1 * phib;
     if (DIR == 0) ubb += Vb; else if (DIR == 1) vbb += Vb; else wbb += Vb;
-    c2b += cb / (R(2) * c);
+    c2b += quot_(cb, R(2) * c);
     Hbb += gm1 * c2b;
     q2bb -= R(0.5) * gm1 * c2b;
     ubb += R(2) * ub * q2bb; vbb += R(2) * vb * q2bb; wbb += R(2) * wb * q2bb;
@@ -361,7 +346,7 @@ NS3D_HD void roe_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
     sRb -= denb * den * den;
     R uLb = ubb * sL * den, vLb = vbb * sL * den, wLb = wbb * sL * den, HLb = Hbb * sL * den;
     R uRb = ubb * sR * den, vRb = vbb * sR * den, wRb = wbb * sR * den, HRb = Hbb * sR * den;
-    R rLb = sLb / (R(2) * sL), rRb = sRb / (R(2) * sR);
+    R rLb = quot_(sLb, R(2) * sL), rRb = quot_(sRb, R(2) * sR);
     // H = 0.5 q2 + kfac p ir
     R pLb = kfac * L.ir * HLb, pRb = kfac * Rs.ir * HRb;
     uLb += L.u * HLb; vLb += L.v * HLb; wLb += L.w * HLb;   // d(0.5 q2)/du = u
@@ -383,7 +368,7 @@ template <int DIR, typename R>
 NS3D_HD void rusanov_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb) {
     SideF<R> L = side_fwd(UL, g), Rs = side_fwd(UR, g);
     R unL = DIR == 0 ? L.u : (DIR == 1 ? L.v : L.w), unR = DIR == 0 ? Rs.u : (DIR == 1 ? Rs.v : Rs.w);
-    R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rs.p * Rs.ir);
+    R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rs.p * Rs.ir);
     R sl = fabs(unL) + aL, sr = fabs(unR) + aR;
     bool left = !(sl < sr);  // std::max(a,b) returns a unless a < b
     R smax = left ? sl : sr;
@@ -396,19 +381,19 @@ NS3D_HD void rusanov_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *
         ULb[n] += R(0.5) * smax * Fb[n];
     }
     R uLb = 0, vLb = 0, wLb = 0, pLb = 0, ELb = 0, rLb = 0, uRb = 0, vRb = 0, wRb = 0, pRb = 0, ERb = 0, rRb = 0;
-    // smax = |un| + sqrt(g p / r)
+    // smax = |un| + sqrt_(g p / r)
     if (left) {
         R unb = (unL >= R(0) ? R(1) : R(-1)) * smaxb;
         if (DIR == 0) uLb += unb; else if (DIR == 1) vLb += unb; else wLb += unb;
         R ab = smaxb, x = g * L.p * L.ir;
-        R xb = ab / (R(2) * aL);
+        R xb = quot_(ab, R(2) * aL);
         pLb += xb * g * L.ir;
         rLb += -(xb * g * L.p) * L.ir * L.ir;
         (void)x;
     } else {
         R unb = (unR >= R(0) ? R(1) : R(-1)) * smaxb;
         if (DIR == 0) uRb += unb; else if (DIR == 1) vRb += unb; else wRb += unb;
-        R xb = smaxb / (R(2) * aR);
+        R xb = quot_(smaxb, R(2) * aR);
         pRb += xb * g * Rs.ir;
         rRb += -(xb * g * Rs.p) * Rs.ir * Rs.ir;
     }
@@ -423,7 +408,7 @@ template <int DIR, typename R>
 NS3D_HD void hll_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb) {
     SideF<R> L = side_fwd(UL, g), Rs = side_fwd(UR, g);
     R unL = DIR == 0 ? L.u : (DIR == 1 ? L.v : L.w), unR = DIR == 0 ? Rs.u : (DIR == 1 ? Rs.v : Rs.w);
-    R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rs.p * Rs.ir);
+    R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rs.p * Rs.ir);
     R a = unL - aL, b = unR - aR;
     bool sl_right = b < a;  // SL = min -> b when b < a
     R SL = sl_right ? b : a;
@@ -442,7 +427,7 @@ NS3D_HD void hll_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
 #pragma unroll
         for (int n = 0; n < 5; ++n) FRb[n] = Fb[n];
     } else {
-        R id = R(1) / (SR - SL);
+        R id = rcp_(SR - SL);
         R SLb = 0, SRb = 0;
 #pragma unroll
         for (int n = 0; n < 5; ++n) {
@@ -461,12 +446,12 @@ NS3D_HD void hll_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb)
             // speed = un + sgn_a * a
             if (!rightside) {
                 if (DIR == 0) uLb += sb; else if (DIR == 1) vLb += sb; else wLb += sb;
-                R xb = sgn_a * sb / (R(2) * aL);
+                R xb = quot_(sgn_a * sb, R(2) * aL);
                 pLb += xb * g * L.ir;
                 rLb += -(xb * g * L.p) * L.ir * L.ir;
             } else {
                 if (DIR == 0) uRb += sb; else if (DIR == 1) vRb += sb; else wRb += sb;
-                R xb = sgn_a * sb / (R(2) * aR);
+                R xb = quot_(sgn_a * sb, R(2) * aR);
                 pRb += xb * g * Rs.ir;
                 rRb += -(xb * g * Rs.p) * Rs.ir * Rs.ir;
             }
@@ -489,7 +474,7 @@ template <int DIR, typename R>
 NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb) {
     SideF<R> L = side_fwd(UL, g), Rs = side_fwd(UR, g);
     const R unL = DIR == 0 ? L.u : (DIR == 1 ? L.v : L.w), unR = DIR == 0 ? Rs.u : (DIR == 1 ? Rs.v : Rs.w);
-    const R aL = sqrt(g * L.p * L.ir), aR = sqrt(g * Rs.p * Rs.ir);
+    const R aL = sqrt_(g * L.p * L.ir), aR = sqrt_(g * Rs.p * Rs.ir);
     R a = unL - aL, b = unR - aR;
     const bool sl_right = b < a;
     const R SL = sl_right ? b : a;
@@ -510,9 +495,9 @@ NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb
     const R den = Rs.r * (SR - unR) - L.r * (SL - unL);
     const bool batten = fabs(den) > R(1e-12);
     R SM;
-    const R sqL = sqrt(L.r), sqR = sqrt(Rs.r);
-    if (batten) SM = num / den;
-    else SM = (sqL * unL + sqR * unR) / (sqL + sqR);
+    const R sqL = sqrt_(L.r), sqR = sqrt_(Rs.r);
+    if (batten) SM = quot_(num, den);
+    else SM = quot_(sqL * unL + sqR * unR, sqL + sqR);
     // the upwind side K and its star state
     const bool left = SM >= R(0);
     const SideF<R> &K = left ? L : Rs;
@@ -520,8 +505,9 @@ NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb
     R *UKb = left ? ULb : URb;
     const R unK = left ? unL : unR, Sk = left ? SL : SR;
     const R dk = Sk - unK, W = Sk - SM, P = K.r * dk;
-    const R rs = K.r * dk / W;
-    const R Z = K.p / P, X = SM - unK, Y = SM + Z;
+    const R iW = rcp_(W), iP = rcp_(P);
+    const R rs = K.r * dk * iW;
+    const R Z = K.p * iP, X = SM - unK, Y = SM + Z;
     const R Es = K.E * K.ir + X * Y;
     const R vs[5] = {R(1), DIR == 0 ? SM : K.u, DIR == 1 ? SM : K.v, DIR == 2 ? SM : K.w, Es};
     // F_n = FK_n + Sk (rs vs_n - UK_n)
@@ -544,14 +530,14 @@ NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb
     const R Xb = Esb * Y, Yb = Esb * X;
     SMb += Xb + Yb;
     unKb -= Xb;
-    pKb += Yb / P;
-    const R Pb = -Yb * K.p / (P * P);
+    pKb += Yb * iP;
+    const R Pb = -Yb * K.p * iP * iP;
     rKb += Pb * dk;
     dkb += Pb * K.r;
     // rs = r dk / (Sk - SM)
-    rKb += rsb * dk / W;
-    dkb += rsb * K.r / W;
-    const R Wb = -rsb * K.r * dk / (W * W);
+    rKb += rsb * dk * iW;
+    dkb += rsb * K.r * iW;
+    const R Wb = -rsb * K.r * dk * iW * iW;
     Skb += Wb;
     SMb -= Wb;
     // dk = Sk - un
@@ -568,7 +554,7 @@ NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb
     R SLb = left ? Skb : R(0), SRb = left ? R(0) : Skb;
     R unLb = 0, unRb = 0;
     if (batten) {
-        const R numb = SMb / den, denb = -SMb * SM / den;
+        const R iden = rcp_(den), numb = SMb * iden, denb = -SMb * SM * iden;
         rRb += numb * unR * (SR - unR) + denb * (SR - unR);
         unRb += numb * Rs.r * (SR - R(2) * unR) - denb * Rs.r;
         SRb += numb * Rs.r * unR + denb * Rs.r;
@@ -589,9 +575,9 @@ NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb
     R aLb = 0, aRb = 0;
     if (sl_right) { unRb += SLb; aRb -= SLb; } else { unLb += SLb; aLb -= SLb; }
     if (sr_right) { unRb += SRb; aRb += SRb; } else { unLb += SRb; aLb += SRb; }
-    // a = sqrt(g p ir)
-    if (aL > R(0)) { const R xb = aLb / (R(2) * aL); pLb += xb * g * L.ir; irLb += xb * g * L.p; }
-    if (aR > R(0)) { const R xb = aRb / (R(2) * aR); pRb += xb * g * Rs.ir; irRb += xb * g * Rs.p; }
+    // a = sqrt_(g p ir)
+    if (aL > R(0)) { const R xb = quot_(aLb, R(2) * aL); pLb += xb * g * L.ir; irLb += xb * g * L.p; }
+    if (aR > R(0)) { const R xb = quot_(aRb, R(2) * aR); pRb += xb * g * Rs.ir; irRb += xb * g * Rs.p; }
     if (DIR == 0) { uLb += unLb; uRb += unRb; }
     else if (DIR == 1) { vLb += unLb; vRb += unRb; }
     else { wLb += unLb; wRb += unRb; }
@@ -665,7 +651,7 @@ NS3D_HD void face_vjp(int interp, int rcode, const R *lin, const R *hd, R g, con
 template <typename R>
 NS3D_HD void visc_flux_all(R mu0, R S, R cpr, const R *x, const R g[4][3], R V[9]) {
     const R T = x[3];
-    const R mu = mu0 * (T * sqrt(T)) * (R(1) + S) / (T + S);
+    const R mu = quot_(mu0 * (T * sqrt_(T)) * (R(1) + S), T + S);
     const R div = g[0][0] + g[1][1] + g[2][2];
     const R m2 = R(2) * mu, m23 = R(2.0 / 3.0) * mu * div;
     const R txx = m2 * g[0][0] - m23, tyy = m2 * g[1][1] - m23, tzz = m2 * g[2][2] - m23;
@@ -680,9 +666,10 @@ NS3D_HD void visc_flux_all(R mu0, R S, R cpr, const R *x, const R g[4][3], R V[9
 template <typename R>
 NS3D_HD void visc_flux_vjp(R mu0, R S, R cpr, const R *x, const R g[4][3], const R *Vb, R *xb, R gb[4][3]) {
     const R T = x[3];
-    const R sq = sqrt(T);
+    const R sq = sqrt_(T);
     const R num = mu0 * (T * sq) * (R(1) + S);
-    const R mu = num / (T + S);
+    const R its = rcp_(T + S);
+    const R mu = num * its;
     const R div = g[0][0] + g[1][1] + g[2][2];
     const R txx = R(2) * mu * g[0][0] - R(2.0 / 3.0) * mu * div;
     const R tyy = R(2) * mu * g[1][1] - R(2.0 / 3.0) * mu * div;
@@ -709,7 +696,7 @@ NS3D_HD void visc_flux_vjp(R mu0, R S, R cpr, const R *x, const R g[4][3], const
     gb[0][2] += mu * txzb; gb[2][0] += mu * txzb;
     gb[1][2] += mu * tyzb; gb[2][1] += mu * tyzb;
     // mu = mu0 T^1.5 (1+S)/(T+S)
-    const R dmu = mu0 * (R(1) + S) * (R(1.5) * sq * (T + S) - T * sq) / ((T + S) * (T + S));
+    const R dmu = mu0 * (R(1) + S) * (R(1.5) * sq * (T + S) - T * sq) * its * its;
     xb[3] += mub * dmu;
     (void)num;
 }
