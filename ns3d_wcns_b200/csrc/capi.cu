@@ -345,6 +345,8 @@ struct ns3d_handle {
     // layout), face-VJP scratch G, viscous scratch X, velocity gradient
     void *adj_pool = nullptr;
     size_t adj_bytes = 0;
+    double *adj_store = nullptr;  // stage states and checkpoints kept between calls (adjoint_store)
+    size_t adj_store_bytes = 0;
     double *ab[4][5] = {};
     double *adjG[30] = {};
     double *adjX[16] = {};
@@ -821,6 +823,41 @@ int ensure_adjoint(ns3d_handle *h) {
     return NS3D_OK;
 }
 
+// Device memory for the stage states and checkpoints of an adjoint call.  Up
+// to ADJ_KEEP_BYTES stay with the handle (an allocation and its release cost
+// a call on a 64^3 grid a third of its time); more is the call's own, freed
+// by adjoint_store_done.  One call at a time per handle uses it.
+constexpr size_t ADJ_KEEP_BYTES = (size_t)2 << 30;
+int adjoint_store(ns3d_handle *h, size_t bytes, double **out) {
+    if (bytes <= h->adj_store_bytes) { *out = h->adj_store; return NS3D_OK; }
+    double *p = nullptr;
+    if (bytes <= ADJ_KEEP_BYTES && h->adj_store) {
+        CK(h, cudaStreamSynchronize(h->stream), "synchronize");
+        cudaFree(h->adj_store);
+        h->adj_store = nullptr;
+        h->adj_store_bytes = 0;
+    }
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess && h->adj_store) {  // what is kept may be what is missing
+        cudaGetLastError();
+        CK(h, cudaStreamSynchronize(h->stream), "synchronize");
+        cudaFree(h->adj_store);
+        h->adj_store = nullptr;
+        h->adj_store_bytes = 0;
+        e = cudaMalloc(&p, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(h, NS3D_ERR_CUDA, "stage states and checkpoints: out of device memory");
+    }
+    if (bytes <= ADJ_KEEP_BYTES) { h->adj_store = p; h->adj_store_bytes = bytes; }
+    *out = p;
+    return NS3D_OK;
+}
+void adjoint_store_done(ns3d_handle *h, double *p) {
+    if (p && p != h->adj_store) cudaFree(p);
+}
+
 AdjArgs adj_args(ns3d_handle *h, double *const W[5], const double *const Rb[5], double *const Ub[5]) {
     AdjArgs a;
     for (int q = 0; q < 5; ++q) { a.W[q] = W[q]; a.Rb[q] = Rb[q]; a.Ub[q] = Ub[q]; }
@@ -884,12 +921,13 @@ int rk3_async_store(ns3d_handle *h, double dt, double *const st[3][5]) {
     const size_t bytes = (size_t)h->L64.plane * 8;
     const int s0 = h->s0, b1 = (s0 + 1) % 3, b2 = (s0 + 2) % 3;
     int r;
-    for (int q = 0; q < 5; ++q) CK(h, cudaMemcpyAsync(st[0][q], h->S[s0][q], bytes, cudaMemcpyDeviceToDevice, h->stream), "store");
+    // the five planes of a state lie one after another, here and in the store
+    CK(h, cudaMemcpyAsync(st[0][0], h->S[s0][0], 5 * bytes, cudaMemcpyDeviceToDevice, h->stream), "store");
     if ((r = rk_stage_async(h, 1, s0, s0, b1, dt))) return r;
-    for (int q = 0; q < 5; ++q) CK(h, cudaMemcpyAsync(st[1][q], h->S[b1][q], bytes, cudaMemcpyDeviceToDevice, h->stream), "store");
+    CK(h, cudaMemcpyAsync(st[1][0], h->S[b1][0], 5 * bytes, cudaMemcpyDeviceToDevice, h->stream), "store");
     h->s0 = b1;
     if ((r = rk_stage_async(h, 2, s0, b1, b2, dt))) { h->s0 = s0; return r; }
-    for (int q = 0; q < 5; ++q) CK(h, cudaMemcpyAsync(st[2][q], h->S[b2][q], bytes, cudaMemcpyDeviceToDevice, h->stream), "store");
+    CK(h, cudaMemcpyAsync(st[2][0], h->S[b2][0], 5 * bytes, cudaMemcpyDeviceToDevice, h->stream), "store");
     h->s0 = b2;
     if ((r = rk_stage_async(h, 3, s0, b2, b1, dt))) { h->s0 = s0; return r; }
     h->s0 = b1;
@@ -1163,6 +1201,7 @@ int ns3d_destroy(ns3d_handle *h) {
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     if (h->pool) cudaFree(h->pool);
     if (h->adj_pool) cudaFree(h->adj_pool);
+    if (h->adj_store) cudaFree(h->adj_store);
     delete h;
     return NS3D_OK;
 }
@@ -1908,15 +1947,14 @@ int ns3d_vjp_rk3_step(ns3d_handle *h, double dt, const double *const ubar_next[5
     // stage states of the step from the current state; the state is restored
     const size_t bytes = (size_t)h->L64.plane * 8;
     double *buf = nullptr;
-    CK(h, cudaMalloc(&buf, 15 * bytes), "stage buffers");
+    if ((r = adjoint_store(h, 15 * bytes, &buf))) return r;
     double *st[3][5];
     for (int b = 0; b < 3; ++b)
         for (int q = 0; q < 5; ++q) st[b][q] = buf + (size_t)(5 * b + q) * h->L64.plane;
     const int s_keep = h->s0;
     r = rk3_async_store(h, dt, st);
     if (!r) {
-        for (int q = 0; q < 5; ++q)
-            cudaMemcpyAsync(h->S[s_keep][q], st[0][q], bytes, cudaMemcpyDeviceToDevice, h->stream);
+        cudaMemcpyAsync(h->S[s_keep][0], st[0][0], 5 * bytes, cudaMemcpyDeviceToDevice, h->stream);
         h->s0 = s_keep;
         h->cfl_valid = false;
         r = refresh_T(h);
@@ -1925,7 +1963,7 @@ int ns3d_vjp_rk3_step(ns3d_handle *h, double dt, const double *const ubar_next[5
     if (!r) r = vjp_step_async(h, st[0], st[1], st[2], dt);
     if (!r) r = download_interior_slot(h, 0, ubar);
     cudaStreamSynchronize(h->stream);
-    cudaFree(buf);
+    adjoint_store_done(h, buf);
     return r;
 }
 
@@ -1946,7 +1984,7 @@ int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int check
     // checkpoints (nck states) + one segment of stage states (ce x 3 states)
     const size_t store_bytes = (size_t)(nck + 3 * ce) * 5 * bytes;
     double *store = nullptr;
-    CK(h, cudaMalloc(&store, store_bytes), "checkpoint storage");
+    if ((r = adjoint_store(h, store_bytes, &store))) return r;
     auto ck = [&](int c, int q) { return store + ((size_t)c * 5 + q) * plane; };
     auto seg = [&](int step, int stage, int q) { return store + ((size_t)(nck + 3 * step + stage) * 5 + q) * plane; };
     cudaEvent_t e0, e1, em, e2;
@@ -1957,9 +1995,8 @@ int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int check
     // ---- forward with checkpoints every ce steps
     for (int n = 0; n < nsteps && !r; ++n) {
         if (n % ce == 0)
-            for (int q = 0; q < 5; ++q)
-                if (cudaMemcpyAsync(ck(n / ce, q), h->S[h->s0][q], bytes, cudaMemcpyDeviceToDevice, h->stream))
-                    r = fail(h, NS3D_ERR_CUDA, "checkpoint copy");
+            if (cudaMemcpyAsync(ck(n / ce, 0), h->S[h->s0][0], 5 * bytes, cudaMemcpyDeviceToDevice, h->stream))
+                r = fail(h, NS3D_ERR_CUDA, "checkpoint copy");
         if (r) break;
         const int n0_last = (nck - 1) * ce;
         if (n >= n0_last) {
@@ -1992,8 +2029,7 @@ int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int check
         const int n0 = c * ce, n1 = (n0 + ce < nsteps) ? n0 + ce : nsteps;
         const bool stored = c == nck - 1;  // stage states kept by the forward pass
         if (!stored) {
-            for (int q = 0; q < 5; ++q)
-                cudaMemcpyAsync(h->S[h->s0][q], ck(c, q), bytes, cudaMemcpyDeviceToDevice, h->stream);
+            cudaMemcpyAsync(h->S[h->s0][0], ck(c, 0), 5 * bytes, cudaMemcpyDeviceToDevice, h->stream);
             r = refresh_T(h);
         }
         for (int n = n0; n < n1 && !r && !stored; ++n) {
@@ -2012,8 +2048,7 @@ int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int check
     cudaEventRecord(e2, h->stream);
     if (!r) {
         // initial state back into the handle, gradient w.r.t. the initial velocity
-        for (int q = 0; q < 5; ++q)
-            cudaMemcpyAsync(h->S[s_init][q], ck(0, q), bytes, cudaMemcpyDeviceToDevice, h->stream);
+        cudaMemcpyAsync(h->S[s_init][0], ck(0, 0), 5 * bytes, cudaMemcpyDeviceToDevice, h->stream);
         h->s0 = s_init;
         h->cfl_valid = false;
         AdjArgs a = adj_args(h, h->S[h->s0], h->ab[3], h->ab[0]);
@@ -2031,7 +2066,7 @@ int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int check
     cudaEventElapsedTime(&fwd_ms, e0, e1);
     cudaEventElapsedTime(&adj_ms, em, e2);
     cudaEventDestroy(e0); cudaEventDestroy(e1); cudaEventDestroy(em); cudaEventDestroy(e2);
-    cudaFree(store);
+    adjoint_store_done(h, store);
     if (r) return r;
     *J = Jv;
     if (stats) {
