@@ -765,6 +765,16 @@ __global__ void batch_scatter_interior(const double *src, double *dst, Layout L)
     dst[L.at(i + NG, j + NG, k + NG)] = src[((long)k * L.ny + j) * L.nx + i];
 }
 
+// the five primitive fields of the problem's current buffer, unpadded and one after another
+__global__ void batch_pack_kernel(const double *base, double *dst, Layout L, const int *state) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
+    if (i >= L.sx) return;
+    const int buf = *state < 0 || *state > 2 ? 0 : *state;
+    const long n = (long)L.sx * L.sy * L.sz, o = ((long)k * L.sy + j) * L.sx + i, c = L.at(i, j, k);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) dst[q * n + o] = base[(5 * buf + q) * L.plane + c];
+}
+
 // ghost fill of one problem's freshly uploaded state (stage 0 of stage_kernel64)
 __global__ void batch_fill_kernel(const double *const *Wc, double *const *Wout, Layout L, BcInfo b) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, k = blockIdx.z;
@@ -817,6 +827,8 @@ struct ns3d_batch {
     cudaGraphExec_t graph = nullptr;
     int graph_max_steps = -1;
     SchemeParams<double> sp;
+    double *pinned = nullptr;    // host side of ns3d_batch_download, allocated by its first call
+    size_t pinned_n = 0;
     std::string err;
     std::vector<double> init;    // copy of the uploaded pool (for re-runs after tuning)
 };
@@ -1196,6 +1208,7 @@ int ns3d_batch_destroy(ns3d_batch *b) {
     if (b->meta) cudaFree(b->meta);
     if (b->wave) cudaFree(b->wave);
     if (b->w_ghosts) cudaFree(b->w_ghosts);
+    if (b->pinned) cudaFreeHost(b->pinned);
     delete b;
     return NS3D_OK;
 }
@@ -1324,14 +1337,34 @@ int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]) {
     cudaSetDevice(b->device);
     const int s = b->order[problem];
     const Inst &I = b->inst[s];
-    int buf = 0;
-    BCK(b, cudaMemcpy(&buf, b->d_state + s, 4, cudaMemcpyDeviceToHost), "query");
-    if (buf < 0 || buf > 2) buf = 0;
     const Layout &L = I.L;
-    for (int q = 0; q < 5; ++q) {
-        const double *src = b->pool + I.base + (long)(5 * buf + q) * L.plane;
-        BCK(b, cudaMemcpy2D(out[q], (size_t)L.sx * 8, src + L.off, (size_t)L.px * 8, (size_t)L.sx * 8,
-                            (size_t)L.sy * L.sz, cudaMemcpyDeviceToHost), "download");
+    // the five fields packed on the device into the problem's face-flux area
+    // (dead between runs), one copy through a pinned buffer kept with the
+    // batch: a pitched copy per field into pageable memory took 1.4 ms for a
+    // 750 x 4 x 4 tube, this 1.1 (the rest is the first touch of new host pages)
+    const size_t n = (size_t)L.sx * L.sy * L.sz;
+    if (!b->pinned) {
+        size_t most = 0;
+        for (const Inst &J : b->inst) most = std::max(most, (size_t)J.L.sx * J.L.sy * J.L.sz);
+        b->pinned_n = std::min(5 * most, (size_t)8 << 20);  // doubles, 64 MB at most
+        if (cudaHostAlloc((void **)&b->pinned, b->pinned_n * 8, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            b->pinned = nullptr;
+            return bfail(b, NS3D_ERR_OOM, "pinned download buffer");
+        }
+    }
+    double *stg = b->pool + I.base + 15L * L.plane;
+    batch_pack_kernel<<<dim3((L.sx + 127) / 128, L.sy, L.sz), 128, 0, b->stream>>>(b->pool + I.base, stg, L, b->d_state + s);
+    BCK(b, cudaGetLastError(), "pack");
+    for (size_t at = 0; at < 5 * n; at += b->pinned_n) {
+        const size_t end = std::min(5 * n, at + b->pinned_n);
+        BCK(b, cudaMemcpyAsync(b->pinned, stg + at, (end - at) * 8, cudaMemcpyDeviceToHost, b->stream), "download");
+        BCK(b, cudaStreamSynchronize(b->stream), "synchronize");
+        for (size_t c = at; c < end;) {  // field by field
+            const size_t q = c / n, stop = std::min(end, (q + 1) * n);
+            std::memcpy(out[q] + (c - q * n), b->pinned + (c - at), (stop - c) * 8);
+            c = stop;
+        }
     }
     return NS3D_OK;
 }
