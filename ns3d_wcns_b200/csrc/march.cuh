@@ -62,26 +62,9 @@ __device__ __forceinline__ void march_cons(float gamma, const float2 *w, float2 
     for (int q = 0; q < 5; ++q) U[q] = make_float2(a[q], b[q]);
 }
 
-__device__ __forceinline__ double march_sub(double a, double b) { return a - b; }
-__device__ __forceinline__ float march_sub(float a, float b) { return a - b; }
-__device__ __forceinline__ float2 march_sub(float2 a, float2 b) { return sub2(a, b); }
 __device__ __forceinline__ double march_add(double a, double b) { return a + b; }
 __device__ __forceinline__ float march_add(float a, float b) { return a + b; }
 __device__ __forceinline__ float2 march_add(float2 a, float2 b) { return add2(a, b); }
-__device__ __forceinline__ double march_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float march_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float2 march_fma(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
-__device__ __forceinline__ double march_neg(double a) { return -a; }
-__device__ __forceinline__ float march_neg(float a) { return -a; }
-__device__ __forceinline__ float2 march_neg(float2 a) { return make_float2(-a.x, -a.y); }
-// r + c0 (p1 - m1) + c1 (p2 - m2) + c2 (p3 - m3): the differences first, so a
-// uniform field leaves r as it is
-template <typename T>
-__device__ __forceinline__ T march_diff3(const T *c, T p1, T m1, T p2, T m2, T p3, T m3, T r) {
-    r = march_fma(c[2], march_sub(p3, m3), r);
-    r = march_fma(c[1], march_sub(p2, m2), r);
-    return march_fma(c[0], march_sub(p1, m1), r);
-}
 template <typename R, typename F>
 __device__ __forceinline__ R march_visc_edge(R, F v, int order, const R *dinv) {
     return dstencil_inv<R>(v, order, dinv);
@@ -218,19 +201,6 @@ __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5
         }
     }
 }
-
-// Paired arithmetic of two lines, for the templates of schemes.cuh
-struct PairOps {
-    __device__ __forceinline__ float2 c(double x) const { return p2((float)x); }
-    __device__ __forceinline__ float2 neg(float2 a) const { return make_float2(-a.x, -a.y); }
-    __device__ __forceinline__ float2 add(float2 a, float2 b) const { return add2(a, b); }
-    __device__ __forceinline__ float2 sub(float2 a, float2 b) const { return sub2(a, b); }
-    __device__ __forceinline__ float2 mul(float2 a, float2 b) const { return mul2(a, b); }
-    __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 d) const { return fma2(a, b, d); }
-    __device__ __forceinline__ float2 add_quot(float2 g, float2 a, float2 b) const {
-        return make_float2(g.x + a.x / b.x, g.y + a.y / b.y);
-    }
-};
 
 // Left and right states of the face between u[2] and u[3]; doubt: march_doubt
 // of the two cells (MDCD_HYBRID).
@@ -555,7 +525,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
                     auto F = [&](unsigned o) { return *at(S::FL + o + q * S::slot); };
                     const T ro = rmw ? *slot(S::RO, q) : march_const<T>(0.0);
                     // faces cu - 1/2 and cu + 1/2 are f - 3 and f - 2
-                    rq[q] = march_diff3(m.dc, F(o2), F(o3), F(o1), F(o4), F(fo), fn[q], ro);
+                    rq[q] = diff3(m.dc, F(o2), F(o3), F(o1), F(o4), F(fo), fn[q], ro);
                 }
             }
             const bool edge = !per && (cu - NG < 3 || cu - NG >= n - 3);
@@ -565,7 +535,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     auto v = [&](unsigned o) { return *at(S::V + o + q * S::slot); };
-                    rq[q + 1] = march_diff3(m.vc, v(v4), v(v2), v(v5), v(v1), v(v6), v(vo), rq[q + 1]);
+                    rq[q + 1] = diff3(m.vc, v(v4), v(v2), v(v5), v(v1), v(v6), v(vo), rq[q + 1]);
                 }
             } else if (visc) {
 #pragma unroll 1
@@ -666,13 +636,7 @@ inline cudaError_t launch_march(const SweepArgs<typename LaneOf<T>::R> &a, cudaS
         else return v;
     };
     for (int k = 0; k < 6; ++k) m.lin[k] = both(a.sp.lin[k]);
-    // the right-hand side takes minus the divergence: face differences (left
-    // minus right face), node differences (right minus left)
-    const double dc[3] = {75.0 / 64.0, -25.0 / 384.0, 3.0 / 640.0}, vc[3] = {45.0, -9.0, 1.0};
-    for (int k = 0; k < 3; ++k) {
-        m.dc[k] = both((R)(dc[k] * (double)a.inv_h));
-        m.vc[k] = both((R)(vc[k] * (double)a.dinv[2]));
-    }
+    for (int k = 0; k < 3; ++k) { m.dc[k] = both(a.dc[k]); m.vc[k] = both(a.vc[k]); }
     const dim3 grid = march_grid<DIR, T>(a, m);
     const int smem = (int)MarchSmem<DIR, T>::bytes;
     static unsigned configured = 0;  // one bit per device ordinal
@@ -696,7 +660,9 @@ inline long march_blocks(const SweepArgs<typename LaneOf<T>::R> &a) {
 }
 template <int DIR, typename R>
 inline long sweep_blocks(const SweepArgs<R> &a) {
-    return (long)((a.L.nx + SweepGeom<DIR, R>::NLINE - 1) / SweepGeom<DIR, R>::NLINE) * a.L.ny;
+    int len;
+    const dim3 g = sweep_grid<DIR, R>(a, len);
+    return (long)g.x * g.y * g.z;
 }
 
 // Component-wise schemes march; characteristic reconstruction, whose bases

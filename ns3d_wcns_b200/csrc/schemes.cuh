@@ -233,7 +233,9 @@ NS3D_HD bool mdcd_smooth_fast(R fm2, R fm1, R f0, R fp1, R fp2, bool &near) {
     const R eps = R(0.9 * 0.4 / (1.0 - 0.9 * 0.4) * 1e-4);
     R a = fabs(f0 - fm1) + fabs(f0 - R(2) * fm1 + fm2);
     R b = fabs(f0 - fp1) + fabs(f0 - R(2) * fp1 + fp2);
-    const R lhs = R(2) * a * b + eps, rhs = R(0.4) * (a * a + b * b + eps);
+    // (FP64: both sides times 5/2, two instructions fewer)
+    const R lhs = sizeof(R) == 8 ? R(5) * a * b + R(2.5) * eps : R(2) * a * b + eps;
+    const R rhs = sizeof(R) == 8 ? a * a + (b * b + eps) : R(0.4) * (a * a + b * b + eps);
     if constexpr (sizeof(R) == 8) {
         // where near stays clear the high words decide (both sides are positive)
         const int d = f64_hi_word(lhs) - f64_hi_word(rhs);

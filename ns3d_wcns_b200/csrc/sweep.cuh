@@ -77,12 +77,14 @@ struct SweepArgs {
     Layout L;
     int periodic;       // this direction
     int outflow_lo, outflow_hi;  // ghost faces copy the boundary face (else zero)
-    R inv_h;            // 1/h of this direction
     R dinv[3];          // 1/(2h), 1/(12h), 1/(60h): the viscous stencils' divisors
+    R dc[3];            // half-node difference: 75/64, -25/384, 3/640 over h
+    R vc[3];            // 6th-order derivative: 45, -9, 1 over 60 h
     SchemeParams<R> sp;
     int first;          // 1: write (first direction), 0: accumulate
     int visc;           // 1: add the viscous divergence term
     const int *done;    // non-null: skip the launch while *done (device time loop)
+    int seg_len;        // cells of a line per block (chunked kernels; gridDim.z segments)
     int zlo, zhi;       // owned interior z-planes [zlo, zhi): the x/y sweeps run over them, the
                         // z-sweep updates only them (the rest of a z-slab's planes are halo)
     FusedStage fs;      // z-sweep only
@@ -148,6 +150,17 @@ __device__ __forceinline__ void to_conserved(const SweepArgs<R> &a, R r, R u, R 
     } else {
         p2c_f(r, u, v, w, p, a.sp.gamma - 1.f, U);
     }
+}
+
+// r + c0 (p1 - m1) + c1 (p2 - m2) + c2 (p3 - m3): the half-node difference
+// (InviscousFlux.cpp:990-992) and the 6th-order derivative added to a
+// right-hand side, the differences first so that a uniform field leaves r as
+// it is
+template <typename R>
+__device__ __forceinline__ R diff3(const R *c, R p1, R m1, R p2, R m2, R p3, R m3, R r) {
+    r += c[2] * (p3 - m3);
+    r += c[1] * (p2 - m2);
+    return r + c[0] * (p1 - m1);
 }
 
 // first derivative along the line, ViscousFlux.cpp:15-29 with the order of
@@ -266,10 +279,13 @@ sweep_kernel(SweepArgs<R> a) {
     const bool per = a.periodic != 0;
     const bool visc = a.visc != 0;
     const bool rmw = a.first == 0;
-    const int fb = per ? 0 : NG - 1;           // first face computed from cells
-    const int fe = per ? n + 5 : n + NG;       // one past the last computed face
-    const int cell_end = per ? n + 8 : n + 6;  // one past the last cell needed
-    const int chunk_end = n + NG + 2;          // chunks run while fc - 2 < n + NG
+    // the segment's cells [c0, c1) need the faces c0 - 3 .. c1 + 1
+    const int c0 = NG + blockIdx.z * a.seg_len, c1 = min(c0 + a.seg_len, n + NG);
+    const int fb = per ? c0 - NG : max(c0 - NG, NG - 1);       // first face computed from cells
+    const int fe = min(c1 + 2, per ? n + 5 : n + NG);          // one past the last computed face
+    const int cell_end = min(c1 + 5, per ? n + 8 : n + 6);     // one past the last cell needed
+    const int chunk_end = c1 + 2;                              // chunks run while fc - 2 < c1
+    const bool whole = gridDim.z == 1;
     const bool char_rt = CHAR == RUNTIME ? (a.sp.char_recon != 0) : (CHAR != 0);
     const int ti = G::tidx(line, slot);
 
@@ -328,7 +344,7 @@ sweep_kernel(SweepArgs<R> a) {
         // cell updated by this thread in this chunk; its old RHS (plain
         // loads, consumed after the face phase)
         const int cu = fc - 2 + slot;
-        const bool upd = line_ok && cu >= NG && cu < n + NG && (DIR != 2 || (cu - NG >= a.zlo && cu - NG < a.zhi));
+        const bool upd = line_ok && cu >= c0 && cu < c1 && (DIR != 2 || (cu - NG >= a.zlo && cu - NG < a.zhi));
         const long cid = lbase + cu * lstride;
         R rold[5];
 #pragma unroll
@@ -390,7 +406,7 @@ sweep_kernel(SweepArgs<R> a) {
             // centre and takes the other from the lane before it (lane 0: from
             // lane 31 of the previous chunk; in the first chunk it evaluates
             // both).  Same values as evaluating both centres per face.
-            if (line_ok && per && fc >= n) {
+            if (line_ok && per && whole && fc >= n) {
                 // the last chunk of a periodic line holds only faces n .. n+4
                 // (fc >= n: uniform over the block): copies of faces 0 .. 4
                 if (f < fe) {
@@ -442,7 +458,7 @@ sweep_kernel(SweepArgs<R> a) {
                     const int s = G::template idx<NF>(line, slot + 5);
 #pragma unroll
                     for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
-                    if (per && f < 5) {  // first chunk (fb = 0 on periodic lines)
+                    if (per && whole && f < 5) {  // first chunk (fb = 0 on periodic lines)
 #pragma unroll
                         for (int q = 0; q < 5; ++q) sWrapF[(q * NL + line) * 5 + f] = F[q];
                     }
@@ -578,23 +594,20 @@ sweep_kernel(SweepArgs<R> a) {
             // faces (Outflow copy of the boundary face, else zero) and the
             // reduced viscous orders apply; everywhere else one straight path
             const bool edge = !per && (cu - NG < 3 || cu - NG >= n - 3);
-            R d[5], vd[4] = {R(0), R(0), R(0), R(0)};
+            R rq[5];
             if (!edge) {
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
                     const R *fq = sF + q * NL * NF;
                     auto F_ = [&](int m) { return fq[G::template idx<NF>(line, slot + m)]; };
-                    // diff_6th_central_half, InviscousFlux.cpp:990-992
-                    d[q] = ((F_(3) - F_(2)) * R(75.0 / 64.0) + (F_(4) - F_(1)) * R(-25.0 / 384.0) +
-                            (F_(5) - F_(0)) * R(3.0 / 640.0)) * a.inv_h;
+                    rq[q] = diff3(a.dc, F_(2), F_(3), F_(1), F_(4), F_(0), F_(5), rold[q]);
                 }
                 if (visc) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const R *vq = sV + q * NL * NV;
                         auto V_ = [&](int off) { return vq[G::template idx<NV>(line, slot + 3 + off)]; };
-                        vd[q] = (V_(3) - R(9) * V_(2) + R(45) * V_(1) - R(45) * V_(-1) + R(9) * V_(-2) - V_(-3)) *
-                                a.dinv[2];
+                        rq[q + 1] = diff3(a.vc, V_(1), V_(-1), V_(2), V_(-2), V_(3), V_(-3), rq[q + 1]);
                     }
                 }
             } else {
@@ -611,23 +624,16 @@ sweep_kernel(SweepArgs<R> a) {
                         else if (ff > n + NG - 1) { if (a.outflow_hi) pm = pf_hi; else zero = true; }
                         fv[m] = zero ? R(0) : sF[q * NL * NF + G::template idx<NF>(line, pm)];
                     }
-                    d[q] = ((fv[3] - fv[2]) * R(75.0 / 64.0) + (fv[4] - fv[1]) * R(-25.0 / 384.0) +
-                            (fv[5] - fv[0]) * R(3.0 / 640.0)) * a.inv_h;
+                    rq[q] = diff3(a.dc, fv[2], fv[3], fv[1], fv[4], fv[0], fv[5], rold[q]);
                 }
                 if (visc) {
                     const int o = visc_order(cu - NG, n, false);
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
-                        vd[q] = dstencil_inv<R>(
+                        rq[q + 1] += dstencil_inv<R>(
                             [&](int off) { return sV[q * NL * NV + G::template idx<NV>(line, slot + 3 + off)]; },
                             o, a.dinv);
                 }
-            }
-            R rq[5];
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                rq[q] = rold[q] - d[q];
-                if (q > 0) rq[q] += vd[q - 1];
             }
             bool fused = false;
             if constexpr (DIR == 2 && sizeof(R) == 8) {
@@ -738,18 +744,44 @@ sweep_kernel(SweepArgs<R> a) {
     }
     if (DIR == 2 && a.fs.stage == 3)  // uniform: every thread of the block arrives
         block_speed_sum_n<CH>(cfl_acc, ke_acc - ke_c, a.fs.dx,
-                              a.fs.cfl_part + (long)blockIdx.y * gridDim.x + blockIdx.x,
-                              a.fs.ke_part + (long)blockIdx.y * gridDim.x + blockIdx.x);
+                              a.fs.cfl_part + ((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x,
+                              a.fs.ke_part + ((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+}
+
+// Cells per block of a chunked sweep: chunks of C faces on `blocks` bundles of
+// lines, two blocks resident per SM.  A bundle marches its chunks one after
+// another, so few bundles leave most of the chip idle; a segment of k chunks
+// updates k C - 5 cells.  Picks the k with the least rounds x (chunks + the
+// fixed cost of a block, about half a chunk).
+inline int sweep_segment(long blocks, int n, int C) {
+    int best = n;
+    double least = 1e300;
+    const int all = (n + 5 + C - 1) / C;
+    for (int k = all; k >= 1; --k) {
+        const int len = k == all ? n : k * C - 5;
+        if (len < 1) break;
+        const long rounds = (blocks * ((n + len - 1) / len) + 2 * 148 - 1) / (2 * 148);
+        const double t = rounds * (k + 0.5);
+        if (t < least * 0.98) { least = t; best = len; }
+    }
+    return best;
+}
+
+template <int DIR, typename R>
+inline dim3 sweep_grid(const SweepArgs<R> &a, int &seg_len) {
+    using G = SweepGeom<DIR, R>;
+    const int n = DIR == 0 ? a.L.nx : (DIR == 1 ? a.L.ny : a.L.nz);
+    dim3 grid(((DIR == 0 ? a.L.ny : a.L.nx) + G::NLINE - 1) / G::NLINE, DIR == 2 ? a.L.ny : a.zhi - a.zlo);
+    seg_len = sweep_segment((long)grid.x * grid.y, n, G::C);
+    grid.z = (n + seg_len - 1) / seg_len;
+    return grid;
 }
 
 template <int DIR, typename R, int INTERP, int RS, int CHAR>
-inline cudaError_t launch_sweep(const SweepArgs<R> &a, cudaStream_t st) {
+inline cudaError_t launch_sweep(SweepArgs<R> a, cudaStream_t st) {
     using G = SweepGeom<DIR, R>;
     dim3 block(DIR == 0 ? G::C : G::NLINE, DIR == 0 ? G::NLINE : G::C);
-    dim3 grid;
-    if (DIR == 0) grid = dim3((a.L.ny + G::NLINE - 1) / G::NLINE, a.zhi - a.zlo);
-    else if (DIR == 1) grid = dim3((a.L.nx + G::NLINE - 1) / G::NLINE, a.zhi - a.zlo);
-    else grid = dim3((a.L.nx + G::NLINE - 1) / G::NLINE, a.L.ny);
+    const dim3 grid = sweep_grid<DIR, R>(a, a.seg_len);
     const size_t smem = sweep_smem_bytes<DIR, R, CHAR != 0>();
     static unsigned configured = 0;  // one bit per device ordinal
     int dev = 0;

@@ -51,10 +51,31 @@ __device__ __forceinline__ void cp_async16(double2 *smem_dst, const double *gsrc
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
 
+// Paired arithmetic of two lines, for the templates of schemes.cuh
+struct PairOps {
+    __device__ __forceinline__ float2 c(double x) const { return p2((float)x); }
+    __device__ __forceinline__ float2 neg(float2 a) const { return make_float2(-a.x, -a.y); }
+    __device__ __forceinline__ float2 add(float2 a, float2 b) const { return add2(a, b); }
+    __device__ __forceinline__ float2 sub(float2 a, float2 b) const { return sub2(a, b); }
+    __device__ __forceinline__ float2 mul(float2 a, float2 b) const { return mul2(a, b); }
+    __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 d) const { return fma2(a, b, d); }
+    __device__ __forceinline__ float2 add_quot(float2 g, float2 a, float2 b) const {
+        return make_float2(g.x + a.x / b.x, g.y + a.y / b.y);
+    }
+};
+
 // MDCD linear coefficients, each duplicated into both halves
 struct PairConsts {
     float2 lin[6];
+    float2 dc[3], vc[3];  // SweepArgs::dc, vc
 };
+
+__device__ __forceinline__ float2 diff3(const float2 *c, float2 p1, float2 m1, float2 p2_, float2 m2, float2 p3, float2 m3,
+                                        float2 r) {
+    r = fma2(c[2], sub2(p3, m3), r);
+    r = fma2(c[1], sub2(p2_, m2), r);
+    return fma2(c[0], sub2(p1, m1), r);
+}
 
 // sum_k c_k f_k (mdcd_linear) for both lines
 __device__ __forceinline__ float2 mdcd_linear2(const float2 *c, float2 f0, float2 f1, float2 f2, float2 f3,
@@ -254,10 +275,13 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
     const bool per = a.periodic != 0;
     const bool visc = a.visc != 0;
     const bool rmw = a.first == 0;
-    const int fb = per ? 0 : NG - 1;
-    const int fe = per ? n + 5 : n + NG;
-    const int cell_end = per ? n + 8 : n + 6;
-    const int chunk_end = n + NG + 2;
+    // the segment's cells [c0, c1), as in sweep_kernel
+    const int c0 = NG + blockIdx.z * a.seg_len, c1 = min(c0 + a.seg_len, n + NG);
+    const int fb = per ? c0 - NG : max(c0 - NG, NG - 1);
+    const int fe = min(c1 + 2, per ? n + 5 : n + NG);
+    const int cell_end = min(c1 + 5, per ? n + 8 : n + 6);
+    const int chunk_end = c1 + 2;
+    const bool whole = gridDim.z == 1;
     const int ti = G::tidx(pr, slot);
     const float gm1 = a.sp.gamma - 1.f;
     // z with nx a multiple of 4: the even pair copies its own and the next
@@ -336,7 +360,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
     for (int fc = fb; fc < chunk_end; fc += C) {
         // cell updated by this thread (both lines) in this chunk
         const int cu = fc - 2 + slot;
-        const bool upd = line_ok && cu >= NG && cu < n + NG && (DIR != 2 || (cu - NG >= a.zlo && cu - NG < a.zhi));
+        const bool upd = line_ok && cu >= c0 && cu < c1 && (DIR != 2 || (cu - NG >= a.zlo && cu - NG < a.zhi));
         const long cid = lbase + cu * lstride;
         if (rmw && upd) {
 #pragma unroll
@@ -377,7 +401,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
 
         // ---- face f = fc + slot of both lines: cell positions slot .. slot+5
         const int f = fc + slot;
-        if (DIR == 0 && per && fc >= n) {
+        if (DIR == 0 && per && whole && fc >= n) {
             // the last chunk of a periodic x-line holds only faces n .. n+4
             // (fc >= n: uniform over the block): copies of faces 0 .. 4
             if (line_ok && f < fe) {
@@ -406,6 +430,8 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
                     mdcd_smooth2(sq[1], sq[2], sq[3], sq[4], sq[5], a3, b3);
                     wa |= ((a2 && a3) ? 0u : 1u) << q;
                     wb |= ((b2 && b3) ? 0u : 1u) << q;
+                } else if constexpr (INTERP == I_WENO5) {
+                    weno5_pair<float2>(PairOps(), sq[0], sq[1], sq[2], sq[3], sq[4], sq[5], UL[q], UR[q]);
                 } else if constexpr (INTERP != I_MDCD_LINEAR) {
                     float sa[6], sb[6];
 #pragma unroll
@@ -448,7 +474,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
 #pragma unroll
                 for (int q = 0; q < 5; ++q) sF[q * NP * NF + s] = make_float2(Fa[q], Fb[q]);
             }
-            if (DIR == 0 && per && f < 5) {  // first chunk (fb = 0 on periodic lines)
+            if (DIR == 0 && per && whole && f < 5) {  // first chunk (fb = 0 on periodic lines)
 #pragma unroll
                 for (int q = 0; q < 5; ++q) sWrapF[(q * NP + pr) * 5 + f] = sF[q * NP * NF + s];
             }
@@ -463,28 +489,20 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
         //      slot+5, node fluxes cu-3 .. cu+3 at visc positions slot .. slot+6
         if (upd) {
             const bool edge = !per && (cu - NG < 3 || cu - NG >= n - 3);
-            float2 d[5], vd[4] = {p2(0.f), p2(0.f), p2(0.f), p2(0.f)};
+            float2 rq[5];
             if (!edge) {
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
                     const float2 *fq = sF + q * NP * NF;
                     auto F_ = [&](int m) { return fq[G::template idx<NF>(pr, slot + m)]; };
-                    // diff_6th_central_half, InviscousFlux.cpp:990-992
-                    float2 t = mul2(sub2(F_(3), F_(2)), p2(float(75.0 / 64.0)));
-                    t = fma2(sub2(F_(4), F_(1)), p2(float(-25.0 / 384.0)), t);
-                    t = fma2(sub2(F_(5), F_(0)), p2(float(3.0 / 640.0)), t);
-                    d[q] = mul2(t, p2(a.inv_h));
+                    rq[q] = diff3(pc.dc, F_(2), F_(3), F_(1), F_(4), F_(0), F_(5), rold[q]);
                 }
                 if (visc) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const float2 *vq = sV + q * NP * NV;
                         auto V_ = [&](int off) { return vq[G::template idx<NV>(pr, slot + 3 + off)]; };
-                        float2 t = fma2(p2(-9.f), V_(2), V_(3));
-                        t = fma2(p2(45.f), V_(1), t);
-                        t = fma2(p2(-45.f), V_(-1), t);
-                        t = fma2(p2(9.f), V_(-2), t);
-                        vd[q] = mul2(sub2(t, V_(-3)), p2(a.dinv[2]));
+                        rq[q + 1] = diff3(pc.vc, V_(1), V_(-1), V_(2), V_(-2), V_(3), V_(-3), rq[q + 1]);
                     }
                 }
             } else {
@@ -503,28 +521,21 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
                         else if (ff > n + NG - 1) { if (a.outflow_hi) pm = pf_hi; else zero = true; }
                         fv[m] = zero ? p2(0.f) : sF[q * NP * NF + G::template idx<NF>(pr, pm)];
                     }
-                    float2 t = mul2(sub2(fv[3], fv[2]), p2(float(75.0 / 64.0)));
-                    t = fma2(sub2(fv[4], fv[1]), p2(float(-25.0 / 384.0)), t);
-                    t = fma2(sub2(fv[5], fv[0]), p2(float(3.0 / 640.0)), t);
-                    d[q] = mul2(t, p2(a.inv_h));
+                    rq[q] = diff3(pc.dc, fv[2], fv[3], fv[1], fv[4], fv[0], fv[5], rold[q]);
                 }
                 if (visc) {
                     const int o = visc_order(cu - NG, n, false);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const float2 *vq = sV + q * NP * NV;
-                        vd[q].x = dstencil_inv<float>(
+                        float2 vd;
+                        vd.x = dstencil_inv<float>(
                             [&](int off) { return vq[G::template idx<NV>(pr, slot + 3 + off)].x; }, o, a.dinv);
-                        vd[q].y = dstencil_inv<float>(
+                        vd.y = dstencil_inv<float>(
                             [&](int off) { return vq[G::template idx<NV>(pr, slot + 3 + off)].y; }, o, a.dinv);
+                        rq[q + 1] = add2(rq[q + 1], vd);
                     }
                 }
-            }
-            float2 rq[5];
-#pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                rq[q] = sub2(rold[q], d[q]);
-                if (q > 0) rq[q] = add2(rq[q], vd[q - 1]);
             }
             bool fused = false;
             if constexpr (DIR == 2) {
@@ -649,10 +660,13 @@ __global__ void __launch_bounds__(256, pair_min_blocks<DIR>()) sweep_pair_kernel
 }
 
 template <int DIR, int INTERP, int RS>
-inline cudaError_t launch_pair(const SweepArgs<float> &a, cudaStream_t st) {
+inline cudaError_t launch_pair(SweepArgs<float> a, cudaStream_t st) {
     using G = PairGeom<DIR>;
+    const int n = DIR == 0 ? a.L.nx : (DIR == 1 ? a.L.ny : a.L.nz);
     dim3 block(DIR == 0 ? G::C : G::NP, DIR == 0 ? G::NP : G::C);
     dim3 grid(((DIR == 0 ? a.L.ny : a.L.nx) + G::NL - 1) / G::NL, DIR == 2 ? a.L.ny : a.zhi - a.zlo);
+    a.seg_len = sweep_segment((long)grid.x * grid.y, n, G::C);
+    grid.z = (n + a.seg_len - 1) / a.seg_len;
     const size_t smem = pair_smem_bytes<DIR>();
     static unsigned configured = 0;  // one bit per device ordinal
     int dev = 0;
@@ -665,6 +679,7 @@ inline cudaError_t launch_pair(const SweepArgs<float> &a, cudaStream_t st) {
     }
     PairConsts pc;
     for (int k = 0; k < 6; ++k) pc.lin[k] = make_float2(a.sp.lin[k], a.sp.lin[k]);
+    for (int k = 0; k < 3; ++k) { pc.dc[k] = make_float2(a.dc[k], a.dc[k]); pc.vc[k] = make_float2(a.vc[k], a.vc[k]); }
     sweep_pair_kernel<DIR, INTERP, RS><<<grid, block, smem, st>>>(a, pc);
     return cudaGetLastError();
 }
