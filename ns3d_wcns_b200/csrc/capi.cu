@@ -3,6 +3,7 @@
 // compute_total_energy, and the reductions.
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -175,30 +176,25 @@ __global__ void __launch_bounds__(RED_THREADS) residual_kernel(const double *con
     block_sum_max<5>(sq, mx, partials + 10 * blockIdx.x);
 }
 
-// Fixed-order combination of the residual partials: sums of values 0-4,
-// maxima of values 5-9.
-__global__ void residual_combine_kernel(const double *partials, int nblocks, double *out) {
-    if (threadIdx.x >= 10) return;
-    const int q = threadIdx.x;
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) {
-        const double x = partials[(long)b * 10 + q];
-        s = q < 5 ? s + x : fmax(s, x);
-    }
-    out[q] = s;
-}
-
-// Fixed-order combination of per-block partials (nv values per block).
-// mode 0: sums, mode 1: minimum of value 0.
-__global__ void combine_kernel(const double *partials, int nblocks, int nv, int mode, double *out) {
-    if (threadIdx.x >= nv) return;
-    const int q = threadIdx.x;
+// Combination of n rows of nv partials in a fixed order, one warp per value:
+// each lane a strided share, then the lanes (a serial loop over 592 rows took
+// 20-25 us).  Values below first_max are summed, those from it on maximised;
+// mode 1: minimum.
+__global__ void combine_kernel(const double *partials, int n, int nv, int first_max, int mode, double *out) {
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (q >= nv) return;
+    const bool mx = q >= first_max;
     double s = mode == 1 ? 1e300 : 0.0;
-    for (int b = 0; b < nblocks; ++b) {
+    for (int b = lane; b < n; b += 32) {
         const double x = partials[(long)b * nv + q];
-        s = mode == 1 ? fmin(s, x) : s + x;
+        s = mode == 1 ? fmin(s, x) : (mx ? fmax(s, x) : s + x);
     }
-    out[q] = s;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const double x = __shfl_down_sync(0xffffffffu, s, o);
+        s = mode == 1 ? fmin(s, x) : (mx ? fmax(s, x) : s + x);
+    }
+    if (lane == 0) out[q] = s;
 }
 
 // Interior upload helpers: host interior block (nx*ny*nz) -> padded state.
@@ -370,6 +366,12 @@ int cuda_fail(ns3d_handle *h, cudaError_t e, const char *what) {
         cudaError_t e_ = (call);                            \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, what); \
     } while (0)
+
+// Blocks of the grid-stride reductions: a cell per thread, at most red_blocks
+int red_grid(const ns3d_handle *h) {
+    const long cells = (long)h->L64.nx * h->L64.ny * (h->zhi - h->zlo);
+    return (int)std::min((long)h->red_blocks, (cells + RED_THREADS - 1) / RED_THREADS);
+}
 
 dim3 cell_grid(const Layout &L, bool with_ghosts, int bx = 128) {
     int nx = with_ghosts ? L.sx : L.nx;
@@ -739,10 +741,25 @@ int rk3_async(ns3d_handle *h, double dt) {
     return NS3D_OK;
 }
 
+// Blocks of the first of two combining launches over n per-block values; 1:
+// one launch suffices (a few thousand values take one block no longer than a
+// launch does).
+int combine_blocks(const ns3d_handle *h, long n) {
+    return n <= 4096 ? 1 : (int)std::min((long)h->red_blocks, (n + 255) / 256);
+}
+
+// The minimum of the CFL bounds that the last stage's blocks left.
+void combine_cfl(ns3d_handle *h, double *out) {
+    const int nb = combine_blocks(h, h->cfl_count);
+    if (nb > 1) min_combine_kernel<<<nb, 256, 0, h->stream>>>(h->cfl_part, h->cfl_count, h->partials);
+    min_combine_kernel<<<1, 256, 0, h->stream>>>(nb > 1 ? h->partials : h->cfl_part, nb > 1 ? nb : h->cfl_count, out);
+    h->launches += nb > 1 ? 2 : 1;
+}
+
 int reduce_combine(ns3d_handle *h, int nv, int mode, double *host_out, const double *part = nullptr,
                    long nblocks = 0) {
-    combine_kernel<<<1, 32, 0, h->stream>>>(part ? part : h->partials, part ? (int)nblocks : h->red_blocks, nv, mode,
-                                            h->scalars);
+    combine_kernel<<<1, 32 * nv, 0, h->stream>>>(part ? part : h->partials, part ? (int)nblocks : red_grid(h), nv, nv, mode,
+                                                 h->scalars);
     h->launches += 1;
     CK(h, cudaGetLastError(), "combine");
     CK(h, cudaMemcpyAsync(host_out, h->scalars, sizeof(double) * nv, cudaMemcpyDeviceToHost, h->stream), "copy scalars");
@@ -752,9 +769,9 @@ int reduce_combine(ns3d_handle *h, int nv, int mode, double *host_out, const dou
 
 int check_state(ns3d_handle *h) {
     if (!h->mixed)
-        check_kernel<double><<<h->red_blocks, RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->partials, h->zlo, h->zhi - h->zlo);
+        check_kernel<double><<<red_grid(h), RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->partials, h->zlo, h->zhi - h->zlo);
     else
-        check_kernel<float><<<h->red_blocks, RED_THREADS, 0, h->stream>>>((const float *const *)(h->dptr + 25), h->L32,
+        check_kernel<float><<<red_grid(h), RED_THREADS, 0, h->stream>>>((const float *const *)(h->dptr + 25), h->L32,
                                                                            h->partials, h->zlo, h->zhi - h->zlo);
     h->launches += 1;
     CK(h, cudaGetLastError(), "check kernel");
@@ -1576,11 +1593,8 @@ int ns3d_compute_timestep(ns3d_handle *h, double *dt_out) {
     if (h->cfl_valid) {
         // the last RK stage left the per-block minima of this state
         prof_begin(h, "cfl_combine");
-        const int nb = h->red_blocks;  // partials holds at least red_blocks values
-        min_combine_kernel<<<nb, 256, 0, h->stream>>>(h->cfl_part, h->cfl_count, h->partials);
-        min_combine_kernel<<<1, 256, 0, h->stream>>>(h->partials, nb, h->scalars);
+        combine_cfl(h, h->scalars);
         prof_end(h);
-        h->launches += 2;
         CK(h, cudaGetLastError(), "cfl combine");
         double m = 0;
         CK(h, cudaMemcpyAsync(&m, h->scalars, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "copy dt");
@@ -1590,10 +1604,10 @@ int ns3d_compute_timestep(ns3d_handle *h, double *dt_out) {
     }
     prof_begin(h, "cfl_dt");
     if (!h->mixed)
-        dt_kernel64<<<h->red_blocks, RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
+        dt_kernel64<<<red_grid(h), RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
                                                                   h->ph.dx, h->partials, h->zlo, h->zhi - h->zlo);
     else
-        dt_kernel_mixed<<<h->red_blocks, RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
+        dt_kernel_mixed<<<red_grid(h), RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
                                                                       h->ph.dx, h->partials, h->zlo, h->zhi - h->zlo);
     prof_end(h);
     h->launches += 1;
@@ -1620,7 +1634,7 @@ int ns3d_diagnostics(ns3d_handle *h, double out[6]) {
         if ((r = reduce_combine(h, 5, 0, s, h->visc_red, nb))) return r;
         if ((r = check_device_error(h))) return r;
     } else if (!h->mixed) {
-        diag_kernel<double><<<h->red_blocks, RED_THREADS, 0, h->stream>>>(visc_args<double>(h), vol, h->partials,
+        diag_kernel<double><<<red_grid(h), RED_THREADS, 0, h->stream>>>(visc_args<double>(h), vol, h->partials,
                                                                            h->zlo, h->zhi - h->zlo);
     } else {
         // FP64 primitives of the current conserved state for the reductions
@@ -1636,7 +1650,7 @@ int ns3d_diagnostics(ns3d_handle *h, double out[6]) {
         for (int q = 0; q < 5; ++q) a.W[q] = h->S[b][q];
         a.T = h->S[bt][0];
         a.L = h->L64;
-        diag_kernel<double><<<h->red_blocks, RED_THREADS, 0, h->stream>>>(a, vol, h->partials, h->zlo, h->zhi - h->zlo);
+        diag_kernel<double><<<red_grid(h), RED_THREADS, 0, h->stream>>>(a, vol, h->partials, h->zlo, h->zhi - h->zlo);
         h->launches += 1;
     }
     if (h->mixed || h->ph.mu == 0.0 || h->diag_separate) {
@@ -1667,12 +1681,12 @@ int ns3d_residuals(ns3d_handle *h, double out[5]) {
     const int prev = (h->s0 + 2) % 3;
     const double dx3 = h->ph.dx * h->ph.dx * h->ph.dx;  // compute_diagnostics weights by dx^3
     if (!h->mixed)
-        residual_kernel<false><<<h->red_blocks, RED_THREADS, 0, h->stream>>>(
+        residual_kernel<false><<<red_grid(h), RED_THREADS, 0, h->stream>>>(
             state_table(h, h->s0), state_table(h, prev), h->L64, h->ph.gamma, dx3, h->partials, h->zlo, h->zhi - h->zlo);
     else
-        residual_kernel<true><<<h->red_blocks, RED_THREADS, 0, h->stream>>>(
+        residual_kernel<true><<<red_grid(h), RED_THREADS, 0, h->stream>>>(
             state_table(h, h->s0), state_table(h, prev), h->L64, h->ph.gamma, dx3, h->partials, h->zlo, h->zhi - h->zlo);
-    residual_combine_kernel<<<1, 32, 0, h->stream>>>(h->partials, h->red_blocks, h->scalars);
+    combine_kernel<<<1, 320, 0, h->stream>>>(h->partials, red_grid(h), 10, 5, 0, h->scalars);
     h->launches += 2;
     CK(h, cudaGetLastError(), "residuals");
     double v[10];
@@ -1688,10 +1702,11 @@ int ns3d_total_energy(ns3d_handle *h, double *ke_out) {
         // the last RK stage left the per-block kinetic energies of this state
         int r = set_device(h); if (r) return r;
         h->launches = 0;
-        const int nb = h->red_blocks;
-        sum_combine_kernel<<<nb, 256, 0, h->stream>>>(h->ke_part, h->cfl_count, h->partials);
-        sum_combine_kernel<<<1, 256, 0, h->stream>>>(h->partials, nb, h->scalars);
-        h->launches += 2;
+        const int nb = combine_blocks(h, h->cfl_count);
+        if (nb > 1) sum_combine_kernel<<<nb, 256, 0, h->stream>>>(h->ke_part, h->cfl_count, h->partials);
+        sum_combine_kernel<<<1, 256, 0, h->stream>>>(nb > 1 ? h->partials : h->ke_part, nb > 1 ? nb : h->cfl_count,
+                                                     h->scalars);
+        h->launches += nb > 1 ? 2 : 1;
         CK(h, cudaGetLastError(), "kinetic energy combine");
         CK(h, cudaMemcpyAsync(ke_out, h->scalars, sizeof(double), cudaMemcpyDeviceToHost, h->stream), "copy energy");
         CK(h, cudaStreamSynchronize(h->stream), "synchronize");
@@ -1715,16 +1730,17 @@ constexpr int ADV_LENS[3] = {12, 3, 1};
 // stage's per-block minima when they describe it, else the separate reduction.
 int seed_cfl_min(ns3d_handle *h) {
     if (h->cfl_valid) {
-        min_combine_kernel<<<h->red_blocks, 256, 0, h->stream>>>(h->cfl_part, h->cfl_count, h->partials);
-    } else if (!h->mixed) {
-        dt_kernel64<<<h->red_blocks, RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
-                                                                  h->ph.dx, h->partials, h->zlo, h->zhi - h->zlo);
+        combine_cfl(h, &h->clock->cfl_min);
     } else {
-        dt_kernel_mixed<<<h->red_blocks, RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
-                                                                      h->ph.dx, h->partials, h->zlo, h->zhi - h->zlo);
+        if (!h->mixed)
+            dt_kernel64<<<red_grid(h), RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
+                                                                    h->ph.dx, h->partials, h->zlo, h->zhi - h->zlo);
+        else
+            dt_kernel_mixed<<<red_grid(h), RED_THREADS, 0, h->stream>>>(state_table(h, h->s0), h->L64, h->ph.gamma,
+                                                                        h->ph.dx, h->partials, h->zlo, h->zhi - h->zlo);
+        min_combine_kernel<<<1, 256, 0, h->stream>>>(h->partials, red_grid(h), &h->clock->cfl_min);
+        h->launches += 2;
     }
-    min_combine_kernel<<<1, 256, 0, h->stream>>>(h->partials, h->red_blocks, &h->clock->cfl_min);
-    h->launches += 2;
     CK(h, cudaGetLastError(), "cfl seed");
     return NS3D_OK;
 }
@@ -1752,8 +1768,7 @@ int capture_adv_graph(ns3d_handle *h, int li, int s0) {
             schedule_kernel<<<1, 1, 0, h->stream>>>(h->clock, h->P.cfl, h->P.dt_fixed, 1e-12);
             r = rk3_async(h, 0.0);
             if (r == NS3D_OK) {
-                min_combine_kernel<<<h->red_blocks, 256, 0, h->stream>>>(h->cfl_part, h->cfl_count, h->partials);
-                min_combine_kernel<<<1, 256, 0, h->stream>>>(h->partials, h->red_blocks, &h->clock->cfl_min);
+                combine_cfl(h, &h->clock->cfl_min);
             }
         }
         cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
@@ -1791,7 +1806,7 @@ int time_advance_device(ns3d_handle *h, double t_end, int max_steps, double *tim
         const int left = max_steps - total;
         const int li = left >= ADV_LENS[0] ? 0 : (left >= ADV_LENS[1] ? 1 : 2);
         CK(h, cudaGraphLaunch(h->adv_graph[li][s0], h->stream), "graph launch");
-        h->launches += (long)ADV_LENS[li] * (3 + 3 * ((h->ph.mu != 0.0 ? 1 : 0) + 4));
+        h->launches += (long)ADV_LENS[li] * ((combine_blocks(h, h->cfl_count) > 1 ? 3 : 2) + 3 * ((h->ph.mu != 0.0 ? 1 : 0) + 4));
         CK(h, cudaMemcpyAsync(&c, h->clock, sizeof(c), cudaMemcpyDeviceToHost, h->stream), "clock");
         CK(h, cudaStreamSynchronize(h->stream), "synchronize");
         const int ran = c.steps - total;  // steps this launch executed (the rest returned at once)
