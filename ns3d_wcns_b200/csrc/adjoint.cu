@@ -517,10 +517,9 @@ extern "C" int ns3d_debug_face_vjp(int direction, int interpolation, int riemann
         for (int m = 0; m < 6; ++m) sp.lin[m] = li[m];
         for (int m = 0; m < 4; ++m) sp.hd[m] = interpolation == 3 ? hd[m] : 0.0;
         sp.interp = interpolation; sp.riemann = riemann; sp.char_recon = 0;
-        double wi[5] = {0, 0, 0, 0, 0};
-        if (direction == 0) wcns_face<0, double, RUNTIME, RUNTIME, 0>(sp, U, wi, wi, flux5);
-        else if (direction == 1) wcns_face<1, double, RUNTIME, RUNTIME, 0>(sp, U, wi, wi, flux5);
-        else wcns_face<2, double, RUNTIME, RUNTIME, 0>(sp, U, wi, wi, flux5);
+        if (direction == 0) wcns_face<0, double, RUNTIME, RUNTIME>(sp, U, flux5);
+        else if (direction == 1) wcns_face<1, double, RUNTIME, RUNTIME>(sp, U, flux5);
+        else wcns_face<2, double, RUNTIME, RUNTIME>(sp, U, flux5);
     }
     return 0;
 }

@@ -611,91 +611,65 @@ NS3D_HD void riemann(const SchemeParams<R> &sp, const R *UL, const R *UR, R *F) 
 
 // ------------------------------------------------------- characteristic basis
 
-// build_eigen_matrices for the Roe average of a cell state with itself, as
-// WCNS_Riemann_InviscidFlux does for characteristic interpolation
-// (InviscousFlux.cpp:166-231 with :849-987).  w = primitive (rho,u,v,w,p).
-template <int DIR, typename R>
-NS3D_HD void cell_eigen(const R *w, R g, R Lm[5][5], R Rm[5][5]) {
-    const R nx = DIR == 0 ? R(1) : R(0), ny = DIR == 1 ? R(1) : R(0), nz = DIR == 2 ? R(1) : R(0);
-    const R gm1 = g - R(1);
-    R r = w[0], u = w[1], v = w[2], ww = w[3], p = w[4];
-    R E = r * (R(0.5) * (u * u + v * v + ww * ww) + quot_(p, gm1 * r));
-    R sq = sqrt_(r);
-    R rb = sq * sq;
-    R den = rcp_(sq + sq);
-    R ub = (sq * u + sq * u) * den, vb = (sq * v + sq * v) * den, wb = (sq * ww + sq * ww) * den;
-    R H = quot_(E + p, r);
-    R Hb = (sq * H + sq * H) * den;
-    R c = sqrt_(gm1 * (Hb - R(0.5) * (ub * ub + vb * vb + wb * wb)));
-    R V = nx * ub + ny * vb + nz * wb;
-    R phi = R(0.5) * gm1 * (ub * ub + vb * vb + wb * wb);
-    R a1 = gm1;
-    const R ic = rcp_(c), irb = rcp_(rb);
-    R a2 = R(M_SQRT1_2) * irb * ic;
-    R a3 = R(M_SQRT1_2) * rb * ic;
-    const R igm1 = rcp_(gm1);
-    R a4 = (phi + c * c) * igm1;
-    R ic2 = ic * ic;
-    R a5 = R(1) - phi * ic2;
-    R a6 = phi * igm1;
-    Lm[0][0] = a2 * (phi + c * V); Lm[0][1] = -a2 * (a1 * ub + nx * c); Lm[0][2] = -a2 * (a1 * vb + ny * c);
-    Lm[0][3] = -a2 * (a1 * wb + nz * c); Lm[0][4] = a1 * a2;
-    Lm[1][0] = nx * a5 - (nz * vb - ny * wb) * irb; Lm[1][1] = nx * a1 * ub * ic2;
-    Lm[1][2] = nx * a1 * vb * ic2 + nz * irb; Lm[1][3] = nx * a1 * wb * ic2 - ny * irb; Lm[1][4] = -nx * a1 * ic2;
-    Lm[2][0] = nz * a5 - (ny * ub - nx * vb) * irb; Lm[2][1] = nz * a1 * ub * ic2 + ny * irb;
-    Lm[2][2] = nz * a1 * vb * ic2 - nx * irb; Lm[2][3] = nz * a1 * wb * ic2; Lm[2][4] = -nz * a1 * ic2;
-    Lm[3][0] = ny * a5 - (nx * wb - nz * ub) * irb; Lm[3][1] = ny * a1 * ub * ic2 - nz * irb;
-    Lm[3][2] = ny * a1 * vb * ic2; Lm[3][3] = ny * a1 * wb * ic2 + nx * irb; Lm[3][4] = -ny * a1 * ic2;
-    Lm[4][0] = a2 * (phi - c * V); Lm[4][1] = -a2 * (a1 * ub - nx * c); Lm[4][2] = -a2 * (a1 * vb - ny * c);
-    Lm[4][3] = -a2 * (a1 * wb - nz * c); Lm[4][4] = a1 * a2;
-    Rm[0][0] = a3; Rm[1][0] = a3 * (ub - nx * c); Rm[2][0] = a3 * (vb - ny * c); Rm[3][0] = a3 * (wb - nz * c);
-    Rm[4][0] = a3 * (a4 - c * V);
-    Rm[0][1] = nx; Rm[1][1] = nx * ub; Rm[2][1] = nx * vb + nz * rb; Rm[3][1] = nx * wb - ny * rb;
-    Rm[4][1] = nx * a6 + rb * (nz * vb - ny * wb);
-    Rm[0][2] = nz; Rm[1][2] = nz * ub + ny * rb; Rm[2][2] = nz * vb - nx * rb; Rm[3][2] = nz * wb;
-    Rm[4][2] = nz * a6 + rb * (ny * ub - nx * vb);
-    Rm[0][3] = ny; Rm[1][3] = ny * ub - nz * rb; Rm[2][3] = ny * vb; Rm[3][3] = ny * wb + nx * rb;
-    Rm[4][3] = ny * a6 + rb * (nx * wb - nz * ub);
-    Rm[0][4] = a3; Rm[1][4] = a3 * (ub + nx * c); Rm[2][4] = a3 * (vb + ny * c); Rm[3][4] = a3 * (wb + nz * c);
-    Rm[4][4] = a3 * (a4 + c * V);
+// One side's state of characteristic-wise interpolation: the stencil f(q, m)
+// (conserved variable q, m = 0 .. 5 counted towards the face) projected on the
+// left eigenvectors of the flux Jacobian at the cell state w (primitive),
+// interpolated, and taken back (WCNS_Riemann_InviscidFlux with
+// build_eigen_matrices of a cell's Roe average with itself,
+// InviscousFlux.cpp:166-231, 849-987).  The unit normal leaves the five by
+// five matrices (Blazek's form) a handful of scalars: with S = (g-1)(|u|^2/2
+// U0 - u.m + U4) and N = u_n U0 - m_n at a stencil point, the acoustic rows are
+// a2 (S +- c N), the entropy row U0 - S/c^2, the shear rows +-(u_t U0 -
+// m_t)/rho -- 16 operations a point instead of 25, and nothing to keep in
+// arrays.
+template <int DIR, typename R, int INTERP, typename F>
+NS3D_HD void char_state(const SchemeParams<R> &sp, F f, const R *w, R *out) {
+    const R g = sp.gamma, gm1 = g - R(1);
+    const R r = w[0], u = w[1], v = w[2], ww = w[3], p = w[4];
+    const R ir = rcp_(r), q2 = R(0.5) * (u * u + v * v + ww * ww);
+    const R c2 = g * p * ir, c = sqrt_(c2), ic = rcp_(c), ic2 = ic * ic;
+    const R a2 = R(M_SQRT1_2) * ir * ic, a3 = R(M_SQRT1_2) * r * ic;
+    const R H = q2 + c2 * rcp_(gm1), un = DIR == 0 ? u : (DIR == 1 ? v : ww);
+    R am[6], ap[6], en[6], t1[6], t2[6];
+#pragma unroll
+    for (int m = 0; m < (INTERP == I_WENO5 ? 5 : 6); ++m) {
+        const R U0 = f(0, m), m1 = f(1, m), m2 = f(2, m), m3 = f(3, m);
+        const R S = gm1 * (q2 * U0 - (u * m1 + v * m2 + ww * m3) + f(4, m));
+        const R cN = c * (un * U0 - (DIR == 0 ? m1 : (DIR == 1 ? m2 : m3)));
+        am[m] = a2 * (S + cN);
+        ap[m] = a2 * (S - cN);
+        en[m] = U0 - ic2 * S;
+        // the shear rows with the reference's signs and order
+        if (DIR == 0) { t1[m] = ir * (v * U0 - m2); t2[m] = ir * (m3 - ww * U0); }
+        else if (DIR == 1) { t1[m] = ir * (ww * U0 - m3); t2[m] = ir * (m1 - u * U0); }
+        else { t1[m] = ir * (m2 - v * U0); t2[m] = ir * (u * U0 - m1); }
+    }
+    if (INTERP == I_WENO5) am[5] = ap[5] = en[5] = t1[5] = t2[5] = R(0);
+    const R qm = interp_side<R, INTERP>(sp, am, false), qp = interp_side<R, INTERP>(sp, ap, false);
+    const R qe = interp_side<R, INTERP>(sp, en, false);
+    const R q1 = interp_side<R, INTERP>(sp, t1, false), q2t = interp_side<R, INTERP>(sp, t2, false);
+    const R s = a3 * (qm + qp), d = a3 * c * (qp - qm), o0 = s + qe;
+    const R b1 = r * (DIR == 2 ? q1 : -q1), b2 = r * (DIR == 2 ? -q2t : q2t);
+    const int c1 = DIR == 1 ? 3 : 2, c2i = DIR == 0 ? 3 : 1;  // the momenta the shear waves carry
+    const R vel[4] = {R(0), u, v, ww};
+    out[0] = o0;
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+        out[k] = vel[k] * o0;
+        if (k == 1 + DIR) out[k] += d;
+        if (k == c1) out[k] += b1;
+        if (k == c2i) out[k] += b2;
+    }
+    out[4] = s * H + d * un + qe * q2 + b1 * vel[c1] + b2 * vel[c2i];
 }
 
-// WCNS_Riemann_InviscidFlux, InviscousFlux.cpp:146-268.
-// U[n][m]: conserved stencil of cells i-2..i+3; wi / wi1: primitives of the
-// cells i and i+1 (characteristic bases of the left / right states).
-template <int DIR, typename R, int INTERP, int RS, int CHAR>
-NS3D_HD void wcns_face(const SchemeParams<R> &sp, const R U[5][6], const R *wi,
-                                          const R *wi1, R *F) {
+// WCNS_Riemann_InviscidFlux, InviscousFlux.cpp:146-268, component-wise.
+// U[n][m]: conserved stencil of cells i-2..i+3.
+template <int DIR, typename R, int INTERP, int RS>
+NS3D_HD void wcns_face(const SchemeParams<R> &sp, const R U[5][6], R *F) {
     R UL[5], UR[5];
-    const bool ch = CHAR == RUNTIME ? (sp.char_recon != 0) : (CHAR != 0);
-    if (!ch) {
 #pragma unroll
-        for (int n = 0; n < 5; ++n) face_pair<R, INTERP>(sp, U[n], UL[n], UR[n]);
-    } else if (CHAR != 0) {
-        R Lm[5][5], Rm[5][5], Q[5], Wc[6];
-#pragma unroll 1
-        for (int side = 0; side < 2; ++side) {
-            cell_eigen<DIR, R>(side == 0 ? wi : wi1, sp.gamma, Lm, Rm);
-#pragma unroll
-            for (int n = 0; n < 5; ++n) {
-#pragma unroll
-                for (int m = 0; m < 6; ++m) {
-                    R s = R(0);
-#pragma unroll
-                    for (int r = 0; r < 5; ++r) s += Lm[n][r] * U[r][m];
-                    Wc[m] = s;
-                }
-                Q[n] = interp_side<R, INTERP>(sp, Wc, side == 1);
-            }
-#pragma unroll
-            for (int n = 0; n < 5; ++n) {
-                R s = R(0);
-#pragma unroll
-                for (int r = 0; r < 5; ++r) s += Rm[n][r] * Q[r];
-                if (side == 0) UL[n] = s; else UR[n] = s;
-            }
-        }
-    }
+    for (int n = 0; n < 5; ++n) face_pair<R, INTERP>(sp, U[n], UL[n], UR[n]);
     riemann<DIR, R, RS>(sp, UL, UR, F);
 }
 

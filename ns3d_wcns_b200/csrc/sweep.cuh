@@ -286,7 +286,6 @@ sweep_kernel(SweepArgs<R> a) {
     const int cell_end = min(c1 + 5, per ? n + 8 : n + 6);     // one past the last cell needed
     const int chunk_end = c1 + 2;                              // chunks run while fc - 2 < c1
     const bool whole = gridDim.z == 1;
-    const bool char_rt = CHAR == RUNTIME ? (a.sp.char_recon != 0) : (CHAR != 0);
     const int ti = G::tidx(line, slot);
 
     auto wrap = [&](int c) { return per ? (c < NG ? c + n : (c >= n + NG ? c - n : c)) : c; };
@@ -304,7 +303,7 @@ sweep_kernel(SweepArgs<R> a) {
         const int s = G::template idx<NU>(line, pu);
 #pragma unroll
         for (int q = 0; q < 5; ++q) sU[q * NL * NU + s] = U[q];
-        if (USE_W && char_rt) {
+        if (USE_W) {
             R *w5 = sW + s;
             w5[0] = r <= R(0) ? R(1e-12) : r; w5[NL * NU] = u; w5[2 * NL * NU] = v;
             w5[3 * NL * NU] = w; w5[4 * NL * NU] = p;
@@ -556,20 +555,27 @@ sweep_kernel(SweepArgs<R> a) {
             const int s = G::template idx<NF>(line, slot + 5);
 #pragma unroll
             for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
-        } else if (line_ok && f < fe) {
-            R st[5][6];
+        } else if (CHAR != 0 && line_ok && f < fe) {
+            // one copy of the side's code: the stencil read from the near or
+            // the far end, on the basis of cell f or f + 1
+            R UL[5], UR[5];
+#pragma unroll 1
+            for (int side = 0; side < 2; ++side) {
+                const int sw = G::template idx<NU>(line, slot + 2 + side);
+                R w[5], o[5];
 #pragma unroll
-            for (int q = 0; q < 5; ++q)
+                for (int q = 0; q < 5; ++q) w[q] = sW[q * NL * NU + sw];
+                char_state<DIR, R, INTERP>(
+                    a.sp,
+                    [&](int q, int m) { return sU[q * NL * NU + G::template idx<NU>(line, slot + (side ? 5 - m : m))]; }, w, o);
 #pragma unroll
-                for (int m = 0; m < 6; ++m) st[q][m] = sU[q * NL * NU + G::template idx<NU>(line, slot + m)];
-            R wi[5], wi1[5];
-            if (USE_W && char_rt) {
-                const int s0 = G::template idx<NU>(line, slot + 2), s1 = G::template idx<NU>(line, slot + 3);
-#pragma unroll
-                for (int q = 0; q < 5; ++q) { wi[q] = sW[q * NL * NU + s0]; wi1[q] = sW[q * NL * NU + s1]; }
+                for (int q = 0; q < 5; ++q) {
+                    if (side == 0) UL[q] = o[q];
+                    else UR[q] = o[q];
+                }
             }
             R F[5];
-            wcns_face<DIR, R, INTERP, RS, CHAR>(a.sp, st, wi, wi1, F);
+            riemann<DIR, R, RS>(a.sp, UL, UR, F);
             const int s = G::template idx<NF>(line, slot + 5);
 #pragma unroll
             for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
@@ -719,7 +725,7 @@ sweep_kernel(SweepArgs<R> a) {
                         sU[q * NL * NU + G::template idx<NU>(line, slot + 5)];
                     sF[q * NL * NF + G::template idx<NF>(line, slot - C + 5)] =
                         sF[q * NL * NF + G::template idx<NF>(line, slot + 5)];
-                    if (USE_W && char_rt)
+                    if (USE_W)
                         sW[q * NL * NU + G::template idx<NU>(line, slot - C + 5)] =
                             sW[q * NL * NU + G::template idx<NU>(line, slot + 5)];
                 }
@@ -805,19 +811,25 @@ cudaError_t sweep_x(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_y(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<float> &, cudaStream_t);
 
-// Specialised instantiations for the benchmark schemes, generic otherwise.
+// Characteristic reconstruction: the interpolation compiled in.
+template <int DIR, typename R>
+inline cudaError_t sweep_char(const SweepArgs<R> &a, cudaStream_t st) {
+    if (a.sp.interp == I_WENO5) return launch_sweep<DIR, R, I_WENO5, RUNTIME, 1>(a, st);
+    if (a.sp.interp == I_MDCD_LINEAR) return launch_sweep<DIR, R, I_MDCD_LINEAR, RUNTIME, 1>(a, st);
+    return launch_sweep<DIR, R, I_MDCD_HYBRID, RUNTIME, 1>(a, st);
+}
+
+// Every scheme: specialised instantiations for the usual pairs, generic otherwise.
 template <int DIR, typename R>
 inline cudaError_t sweep_select(const SweepArgs<R> &a, cudaStream_t st) {
     const auto &sp = a.sp;
-    if (!sp.char_recon) {
-        if (sp.interp == I_WENO5 && sp.riemann == R_ROE) return launch_sweep<DIR, R, I_WENO5, R_ROE, 0>(a, st);
-        if (sp.interp == I_MDCD_HYBRID && sp.riemann == R_HLLC)
-            return launch_sweep<DIR, R, I_MDCD_HYBRID, R_HLLC, 0>(a, st);
-        if (sp.interp == I_MDCD_LINEAR && sp.riemann == R_HLLC)
-            return launch_sweep<DIR, R, I_MDCD_LINEAR, R_HLLC, 0>(a, st);
-        return launch_sweep<DIR, R, RUNTIME, RUNTIME, 0>(a, st);
-    }
-    return launch_sweep<DIR, R, RUNTIME, RUNTIME, 1>(a, st);
+    if (sp.char_recon) return sweep_char<DIR, R>(a, st);
+    if (sp.interp == I_WENO5 && sp.riemann == R_ROE) return launch_sweep<DIR, R, I_WENO5, R_ROE, 0>(a, st);
+    if (sp.interp == I_MDCD_HYBRID && sp.riemann == R_HLLC)
+        return launch_sweep<DIR, R, I_MDCD_HYBRID, R_HLLC, 0>(a, st);
+    if (sp.interp == I_MDCD_LINEAR && sp.riemann == R_HLLC)
+        return launch_sweep<DIR, R, I_MDCD_LINEAR, R_HLLC, 0>(a, st);
+    return launch_sweep<DIR, R, RUNTIME, RUNTIME, 0>(a, st);
 }
 
 }  // namespace ns3d

@@ -4,7 +4,7 @@
 
 namespace ns3d {
 cudaError_t sweep_y(const SweepArgs<double> &a, cudaStream_t st) {
-    return march_takes(a) ? march_select<1, double>(a, st) : sweep_select<1, double>(a, st);
+    return march_takes(a) ? march_select<1, double>(a, st) : sweep_char<1, double>(a, st);
 }
 cudaError_t sweep_y(const SweepArgs<float> &a, cudaStream_t st) {
     if (!march_takes(a)) return sweep_select<1, float>(a, st);
