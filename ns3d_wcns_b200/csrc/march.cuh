@@ -95,32 +95,35 @@ __device__ __forceinline__ T march_ld(const R *p) { return *reinterpret_cast<con
 
 // ------------------------------------------------------------------ one face
 
-// Variables whose detector does not clearly accept the linear scheme at one
-// cell, from its five points u[m][q]: bit q (and q + 5 for a float2's second
+// Whether the detector of one cell does not clearly accept the linear scheme
+// for one variable, from its five points (bit 0; bit 5 for a float2's second
 // line).  FP64: the two sides of the cross-multiplied test (mdcd_smooth, both
 // scaled by 5/2) compared by their high words; anything rejected or closer
 // than two units in them is left to march_weno, which takes mdcd_smooth's
 // decision.
+__device__ __forceinline__ unsigned march_doubt1(double f0, double f1, double f2, double f3, double f4) {
+    const double eps = 0.9 * 0.4 / (1.0 - 0.9 * 0.4) * 1e-4;
+    const double a = fabs(f2 - f1) + fabs(f2 - 2.0 * f1 + f0);
+    const double b = fabs(f2 - f3) + fabs(f2 - 2.0 * f3 + f4);
+    const double lhs = __fma_rn(5.0 * a, b, 2.5 * eps), rhs = __fma_rn(a, a, __fma_rn(b, b, eps));
+    return f64_hi_word(lhs) - f64_hi_word(rhs) <= 1 ? 1u : 0u;
+}
+__device__ __forceinline__ unsigned march_doubt1(float f0, float f1, float f2, float f3, float f4) {
+    return mdcd_smooth(f0, f1, f2, f3, f4) ? 0u : 1u;
+}
+__device__ __forceinline__ unsigned march_doubt1(float2 f0, float2 f1, float2 f2, float2 f3, float2 f4) {
+    bool sa, sb;
+    mdcd_smooth2(f0, f1, f2, f3, f4, sa, sb);
+    return (sa ? 0u : 1u) | (sb ? 0u : 32u);
+}
+template <typename T>
+__device__ __forceinline__ unsigned march_doubt1(const T *f) { return march_doubt1(f[0], f[1], f[2], f[3], f[4]); }
+// every variable: bit q (and q + 5); u[m][q]
 template <typename T>
 __device__ __forceinline__ unsigned march_doubt(const T (*u)[5]) {
     unsigned r = 0;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
-        if constexpr (LaneOf<T>::N == 2) {
-            bool sa, sb;
-            mdcd_smooth2(u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], sa, sb);
-            if (!sa) r |= 1u << q;
-            if (!sb) r |= 32u << q;
-        } else if constexpr (sizeof(T) == 8) {
-            const double eps = 0.9 * 0.4 / (1.0 - 0.9 * 0.4) * 1e-4;
-            const double a = fabs(u[2][q] - u[1][q]) + fabs(u[2][q] - 2.0 * u[1][q] + u[0][q]);
-            const double b = fabs(u[2][q] - u[3][q]) + fabs(u[2][q] - 2.0 * u[3][q] + u[4][q]);
-            const double lhs = __fma_rn(5.0 * a, b, 2.5 * eps), rhs = __fma_rn(a, a, __fma_rn(b, b, eps));
-            if (f64_hi_word(lhs) - f64_hi_word(rhs) <= 1) r |= 1u << q;
-        } else {
-            if (!mdcd_smooth(u[0][q], u[1][q], u[2][q], u[3][q], u[4][q])) r |= 1u << q;
-        }
-    }
+    for (int q = 0; q < 5; ++q) r |= march_doubt1(u[0][q], u[1][q], u[2][q], u[3][q], u[4][q]) << q;
     return r;
 }
 
@@ -202,32 +205,33 @@ __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5
     }
 }
 
-// Left and right states of the face between u[2] and u[3]; doubt: march_doubt
-// of the two cells (MDCD_HYBRID).
+// Left and right states of one variable at the face between f[2] and f[3]
+// (MDCD_HYBRID: the linear ones).
+template <typename T, int INTERP>
+__device__ __forceinline__ void march_pair(const MarchArgs<T> &m, const T *f, T &l, T &r) {
+    if constexpr (INTERP == I_WENO5) {
+        if constexpr (LaneOf<T>::N == 2) weno5_pair<T>(PairOps(), f[0], f[1], f[2], f[3], f[4], f[5], l, r);
+        else weno5_pair<T>(ScalarOps<T>(), f[0], f[1], f[2], f[3], f[4], f[5], l, r);
+    } else if constexpr (LaneOf<T>::N == 2) {
+        l = mdcd_linear2(m.lin, f[0], f[1], f[2], f[3], f[4], f[5]);
+        r = mdcd_linear2(m.lin, f[5], f[4], f[3], f[2], f[1], f[0]);
+    } else {
+        l = mdcd_linear(m.lin, f[0], f[1], f[2], f[3], f[4], f[5]);
+        r = mdcd_linear(m.lin, f[5], f[4], f[3], f[2], f[1], f[0]);
+    }
+}
+
+// Every variable of the face between u[2] and u[3]; doubt: march_doubt of the
+// two cells (MDCD_HYBRID).
 template <typename T, int INTERP>
 __device__ __forceinline__ void march_states(const MarchArgs<T> &m, const T (*u)[5], unsigned doubt, T *UL, T *UR) {
-    if constexpr (INTERP == I_WENO5) {
 #pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            if constexpr (LaneOf<T>::N == 2)
-                weno5_pair<T>(PairOps(), u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q], UL[q], UR[q]);
-            else
-                weno5_pair<T>(ScalarOps<T>(), u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q], UL[q], UR[q]);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            if constexpr (LaneOf<T>::N == 2) {
-                UL[q] = mdcd_linear2(m.lin, u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q]);
-                UR[q] = mdcd_linear2(m.lin, u[5][q], u[4][q], u[3][q], u[2][q], u[1][q], u[0][q]);
-            } else {
-                UL[q] = mdcd_linear(m.lin, u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q]);
-                UR[q] = mdcd_linear(m.lin, u[5][q], u[4][q], u[3][q], u[2][q], u[1][q], u[0][q]);
-            }
-        }
-        if constexpr (INTERP == I_MDCD_HYBRID) {
-            if (__any_sync(0xffffffffu, doubt != 0)) march_weno<T>(m, u, doubt, UL, UR);
-        }
+    for (int q = 0; q < 5; ++q) {
+        const T f[6] = {u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q]};
+        march_pair<T, INTERP>(m, f, UL[q], UR[q]);
+    }
+    if constexpr (INTERP == I_MDCD_HYBRID) {
+        if (__any_sync(0xffffffffu, doubt != 0)) march_weno<T>(m, u, doubt, UL, UR);
     }
 }
 
@@ -626,8 +630,8 @@ inline dim3 march_grid(const SweepArgs<typename LaneOf<T>::R> &a, MarchArgs<T> &
     return dim3(nb, (n + m.seg_len - 1) / m.seg_len);
 }
 
-template <int DIR, typename T, int INTERP, int RS>
-inline cudaError_t launch_march(const SweepArgs<typename LaneOf<T>::R> &a, cudaStream_t st) {
+template <typename T>
+inline MarchArgs<T> march_args(const SweepArgs<typename LaneOf<T>::R> &a) {
     MarchArgs<T> m;
     m.a = a;
     using R = typename LaneOf<T>::R;
@@ -637,6 +641,13 @@ inline cudaError_t launch_march(const SweepArgs<typename LaneOf<T>::R> &a, cudaS
     };
     for (int k = 0; k < 6; ++k) m.lin[k] = both(a.sp.lin[k]);
     for (int k = 0; k < 3; ++k) { m.dc[k] = both(a.dc[k]); m.vc[k] = both(a.vc[k]); }
+    m.nlines = m.seg_len = 0;
+    return m;
+}
+
+template <int DIR, typename T, int INTERP, int RS>
+inline cudaError_t launch_march(const SweepArgs<typename LaneOf<T>::R> &a, cudaStream_t st) {
+    MarchArgs<T> m = march_args<T>(a);
     const dim3 grid = march_grid<DIR, T>(a, m);
     const int smem = (int)MarchSmem<DIR, T>::bytes;
     static unsigned configured = 0;  // one bit per device ordinal

@@ -294,7 +294,7 @@ sweep_kernel(SweepArgs<R> a) {
     auto vis_pos = [&](int c) -> int {
         if (c < 0) return -1;
         int ci = c - NG;
-        if (per) { if (ci < 0) ci += n; else if (ci >= n) ci -= n; return ci; }
+        if (per) { if (ci < 0) ci += n; else if (ci >= n) ci -= n; return ci < n ? ci : -1; }
         return (ci >= 0 && ci < n) ? ci : -1;
     };
     auto put_cell = [&](int pu, int pv, R r, R u, R v, R w, R p, const R *vf) {
@@ -755,18 +755,18 @@ sweep_kernel(SweepArgs<R> a) {
 }
 
 // Cells per block of a chunked sweep: chunks of C faces on `blocks` bundles of
-// lines, two blocks resident per SM.  A bundle marches its chunks one after
+// lines, `resident` blocks per SM.  A bundle marches its chunks one after
 // another, so few bundles leave most of the chip idle; a segment of k chunks
 // updates k C - 5 cells.  Picks the k with the least rounds x (chunks + the
 // fixed cost of a block, about half a chunk).
-inline int sweep_segment(long blocks, int n, int C) {
+inline int sweep_segment(long blocks, int n, int C, int resident = 2) {
     int best = n;
     double least = 1e300;
     const int all = (n + 5 + C - 1) / C;
     for (int k = all; k >= 1; --k) {
         const int len = k == all ? n : k * C - 5;
         if (len < 1) break;
-        const long rounds = (blocks * ((n + len - 1) / len) + 2 * 148 - 1) / (2 * 148);
+        const long slots = (long)resident * 148, rounds = (blocks * ((n + len - 1) / len) + slots - 1) / slots;
         const double t = rounds * (k + 0.5);
         if (t < least * 0.98) { least = t; best = len; }
     }

@@ -1,0 +1,52 @@
+"""The x-sweep (a line per warp, two faces per lane, chunks of 64 faces) where
+it can go wrong: lines that end just before, at and after a chunk, the
+shortest ones, line counts that leave warps idle, odd and even line pairs, and
+every boundary type, against the CPU oracle.  Tolerance: the FP64 path's own
+bounds, 1e-12 of the largest right-hand side and 1e-10 of the state after two
+steps.  Mixed path (continuous schemes): two steps change the state by less
+than a tenth, in FP32 to some 1e-6 of that, so 1e-6 of the state."""
+import pytest
+
+from helpers import interior, rel_linf
+from ns3d_wcns_b200.config import make_params
+from ns3d_wcns_b200.initial import random_state
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+NX = [3, 4, 58, 59, 60, 61, 63, 64, 65, 66, 124, 128, 131]
+BCS = [(0,) * 6, (3, 3, 0, 0, 1, 2), (1, 2, 3, 3, 0, 0)]
+
+
+@pytest.mark.parametrize("nx", NX)
+@pytest.mark.parametrize("ny", [4, 5])
+@pytest.mark.parametrize("bcs", BCS, ids=["periodic", "outflow", "wall"])
+@pytest.mark.parametrize("interp,rs", [(0, 0), (3, 2), (2, 2)])
+def test_sweep_line_against_oracle(gpu_lib, nx, ny, bcs, interp, rs):
+    from ns3d_wcns_b200.solver import Solver
+    n = (nx, ny, 3)
+    P, G = make_params(n=n, L=(1.0, 0.8, 0.9), interpolation=interp, riemann=rs, bcs=bcs, Re=300.0, dt_fixed=1e-4)
+    st = random_state(n, seed=7, amp=0.2)
+    o = oracle.PortSolver(P, G)
+    o.set_interior_prims(*st)
+    o.compute_rhs()
+    with Solver(P, G) as s:
+        s.set_interior_primitives(*st)
+        s.compute_rhs()
+        for a, b in zip(interior(s.rhs()), interior(o.rhs())):
+            assert rel_linf(a, b) <= 1e-12
+        for _ in range(2):
+            s.rk3_step(1e-4)
+            o.rk3_step(1e-4)
+        for a, b in zip(interior(s.conserved()), interior(o.conserved())):
+            assert rel_linf(a, b) <= 1e-10
+    if interp == 3:  # its detector may flip at a threshold in FP32
+        return
+    Pm, _ = make_params(n=n, L=(1.0, 0.8, 0.9), interpolation=interp, riemann=rs, bcs=bcs, Re=300.0, dt_fixed=1e-4,
+                        precision=1)
+    with Solver(Pm, G) as s:
+        s.set_interior_primitives(*st)
+        for _ in range(2):
+            s.rk3_step(1e-4)
+        for a, b in zip(interior(s.conserved()), interior(o.conserved())):
+            assert rel_linf(a, b) <= 1e-6
