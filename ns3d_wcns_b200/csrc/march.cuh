@@ -62,8 +62,9 @@ __device__ __forceinline__ void march_cons(float gamma, const float2 *w, float2 
     for (int q = 0; q < 5; ++q) U[q] = make_float2(a[q], b[q]);
 }
 
-__device__ __forceinline__ double march_add(double a, double b) { return a + b; }
-__device__ __forceinline__ float march_add(float a, float b) { return a + b; }
+// rounded on its own: the same bits from every copy of the boundary code
+__device__ __forceinline__ double march_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float march_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float2 march_add(float2 a, float2 b) { return add2(a, b); }
 template <typename R, typename F>
 __device__ __forceinline__ R march_visc_edge(R, F v, int order, const R *dinv) {

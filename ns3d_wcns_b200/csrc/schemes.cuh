@@ -119,14 +119,28 @@ NS3D_HD void weno5_pair(const A &o, V f0, V f1, V f2, V f3, V f4, V f5, V &left,
     left = side(f2, d1, d2, d3, d4, s1, s2, s3);
     right = side(f3, o.neg(d5), o.neg(d4), o.neg(d3), o.neg(d2), s4, s3, s2);
 }
+// Rounded as written (nothing is contracted), so that every copy of the code,
+// in whichever kernel and for whichever of a thread's faces, returns the same
+// bits: a z-slab equals the single domain although its faces pair differently.
 template <typename R>
 struct ScalarOps {
     NS3D_HD R c(double x) const { return R(x); }
     NS3D_HD R neg(R a) const { return -a; }
+#ifdef __CUDA_ARCH__
+    NS3D_HD double add(double a, double b) const { return __dadd_rn(a, b); }
+    NS3D_HD double sub(double a, double b) const { return __dsub_rn(a, b); }
+    NS3D_HD double mul(double a, double b) const { return __dmul_rn(a, b); }
+    NS3D_HD double fma(double a, double b, double d) const { return __fma_rn(a, b, d); }
+    NS3D_HD float add(float a, float b) const { return __fadd_rn(a, b); }
+    NS3D_HD float sub(float a, float b) const { return __fsub_rn(a, b); }
+    NS3D_HD float mul(float a, float b) const { return __fmul_rn(a, b); }
+    NS3D_HD float fma(float a, float b, float d) const { return __fmaf_rn(a, b, d); }
+#else
     NS3D_HD R add(R a, R b) const { return a + b; }
     NS3D_HD R sub(R a, R b) const { return a - b; }
     NS3D_HD R mul(R a, R b) const { return a * b; }
     NS3D_HD R fma(R a, R b, R d) const { return a * b + d; }
+#endif
     // g + a / b
     NS3D_HD R add_quot(R g, R a, R b) const {
 #ifdef __CUDA_ARCH__

@@ -158,9 +158,9 @@ __device__ __forceinline__ void to_conserved(const SweepArgs<R> &a, R r, R u, R 
 // it is
 template <typename R>
 __device__ __forceinline__ R diff3(const R *c, R p1, R m1, R p2, R m2, R p3, R m3, R r) {
-    r += c[2] * (p3 - m3);
-    r += c[1] * (p2 - m2);
-    return r + c[0] * (p1 - m1);
+    r = fma(c[2], p3 - m3, r);
+    r = fma(c[1], p2 - m2, r);
+    return fma(c[0], p1 - m1, r);
 }
 
 // first derivative along the line, ViscousFlux.cpp:15-29 with the order of

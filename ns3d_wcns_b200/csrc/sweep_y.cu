@@ -1,13 +1,13 @@
 // sweep_y.cu -- instantiations of the inviscid sweep along y (one translation
 // unit per direction so the builds run in parallel).
-#include "march.cuh"
+#include "sweep_line.cuh"
 
 namespace ns3d {
 cudaError_t sweep_y(const SweepArgs<double> &a, cudaStream_t st) {
-    return march_takes(a) ? march_select<1, double>(a, st) : sweep_char<1, double>(a, st);
+    return march_takes(a) ? line_or_march<1, double>(a, st) : sweep_char<1, double>(a, st);
 }
 cudaError_t sweep_y(const SweepArgs<float> &a, cudaStream_t st) {
     if (!march_takes(a)) return sweep_select<1, float>(a, st);
-    return a.L.nx & 1 ? march_select<1, float>(a, st) : march_select<1, float2>(a, st);
+    return a.L.nx & 1 ? line_or_march<1, float>(a, st) : line_or_march<1, float2>(a, st);
 }
 }  // namespace ns3d

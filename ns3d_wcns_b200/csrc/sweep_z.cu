@@ -1,22 +1,22 @@
 // sweep_z.cu -- instantiations of the fused inviscid sweep along z
 // (one translation unit per direction so the builds run in parallel).
-#include "march.cuh"
+#include "sweep_line.cuh"
 
 namespace ns3d {
 cudaError_t sweep_z(const SweepArgs<double> &a, cudaStream_t st) {
-    return march_takes(a) ? march_select<2, double>(a, st) : sweep_char<2, double>(a, st);
+    return march_takes(a) ? line_or_march<2, double>(a, st) : sweep_char<2, double>(a, st);
 }
 cudaError_t sweep_z(const SweepArgs<float> &a, cudaStream_t st) {
     if (!march_takes(a)) return sweep_select<2, float>(a, st);
-    return a.L.nx & 1 ? march_select<2, float>(a, st) : march_select<2, float2>(a, st);
+    return a.L.nx & 1 ? line_or_march<2, float>(a, st) : line_or_march<2, float2>(a, st);
 }
 
 // blocks of the z-sweep: the partials its fused stage 3 writes
 long sweep_z_blocks(const SweepArgs<double> &a) {
-    return march_takes(a) ? march_blocks<2, double>(a) : sweep_blocks<2, double>(a);
+    return march_takes(a) ? line_or_march_blocks<2, double>(a) : sweep_blocks<2, double>(a);
 }
 long sweep_z_blocks(const SweepArgs<float> &a) {
     if (!march_takes(a)) return sweep_blocks<2, float>(a);
-    return a.L.nx & 1 ? march_blocks<2, float>(a) : march_blocks<2, float2>(a);
+    return a.L.nx & 1 ? line_or_march_blocks<2, float>(a) : line_or_march_blocks<2, float2>(a);
 }
 }  // namespace ns3d

@@ -14,6 +14,16 @@ from oracle import oracle
 
 pytestmark = pytest.mark.gpu
 
+
+@pytest.mark.parametrize("n", [(61, 5, 60), (61, 60, 3), (55, 67, 7), (66, 62, 64)], ids=str)
+@pytest.mark.parametrize("bcs", [(0,) * 6, (3, 3, 1, 2, 4, 4), (1, 2, 3, 3, 0, 0)],
+                         ids=["periodic", "mixed", "z-periodic"])
+@pytest.mark.parametrize("interp,rs", [(0, 0), (3, 2), (2, 2)])
+def test_many_lines_against_oracle(gpu_lib, n, bcs, interp, rs):
+    """More lines than the kernel with a line per warp takes along y and z:
+    the marching kernel, whole lines and segments."""
+    _check(n, bcs, interp, rs)
+
 NX = [3, 4, 58, 59, 60, 61, 63, 64, 65, 66, 124, 128, 131]
 BCS = [(0,) * 6, (3, 3, 0, 0, 1, 2), (1, 2, 3, 3, 0, 0)]
 
@@ -23,8 +33,11 @@ BCS = [(0,) * 6, (3, 3, 0, 0, 1, 2), (1, 2, 3, 3, 0, 0)]
 @pytest.mark.parametrize("bcs", BCS, ids=["periodic", "outflow", "wall"])
 @pytest.mark.parametrize("interp,rs", [(0, 0), (3, 2), (2, 2)])
 def test_sweep_line_against_oracle(gpu_lib, nx, ny, bcs, interp, rs):
+    _check((nx, ny, 3), bcs, interp, rs)
+
+
+def _check(n, bcs, interp, rs):
     from ns3d_wcns_b200.solver import Solver
-    n = (nx, ny, 3)
     P, G = make_params(n=n, L=(1.0, 0.8, 0.9), interpolation=interp, riemann=rs, bcs=bcs, Re=300.0, dt_fixed=1e-4)
     st = random_state(n, seed=7, amp=0.2)
     o = oracle.PortSolver(P, G)
