@@ -274,11 +274,13 @@ __global__ void __launch_bounds__(256) stage_ghost_kernel64(StageArgs64 a) {
 
 // Ghost cells after the mixed path's fused z-sweep (increment form, see
 // FusedStage): a ghost whose source is an interior cell gets that cell's new
-// state -- U0 + D after stages 1 and 2 (the conversion the sweep applies, so
-// the same FP32 primitives), the FP64 state after stage 3 -- with sign flips;
-// a ghost whose source is a ghost keeps its step-start state (its right-hand
-// side is zero in every stage); special states are constants.  Only stage 3
-// writes the FP64 state's ghosts.
+// state -- after stages 1 and 2 the FP32 primitives and temperature that the
+// sweep stored, after stage 3 the FP64 state and its conversion -- with sign
+// flips; a ghost whose source is a ghost keeps its step-start state (its
+// right-hand side is zero in every stage); special states are constants.  Only
+// stage 3 writes the FP64 state's ghosts.  Bound by its scattered reads and
+// writes: 256^3, mean of the three stages, 72 us when stages 1 and 2 read U0
+// and D and converted, 60 us.
 __global__ void __launch_bounds__(256) stage_ghost_kernel_mixed(StageArgsMixed a) {
     if (a.done && *a.done) return;
     const Layout &L = a.L;
@@ -297,15 +299,18 @@ __global__ void __launch_bounds__(256) stage_ghost_kernel_mixed(StageArgsMixed a
     } else {
         const long s = L.at(c[0], c[1], c[2]);
         if (is_interior(L, c)) {
-            if (a.stage == 3) {
+            if (a.stage != 3) {  // the sweep's FP32 primitives themselves: 24 bytes instead of 60, no conversion
+                const long s32 = a.L32.at(c[0], c[1], c[2]), o32 = a.L32.at(i, j, k);
 #pragma unroll
-                for (int q = 0; q < 5; ++q) U[q] = a.Uout[q][s];  // new value, already clamped
-            } else {
-                const long s32 = a.L32.at(c[0], c[1], c[2]);
-#pragma unroll
-                for (int q = 0; q < 5; ++q) U[q] = a.U0[q][s] + (double)a.D[q][s32];
-                if (U[0] <= 0.0) U[0] = 1e-12;
+                for (int q = 0; q < 5; ++q) {
+                    const float w = a.Wout[q][s32];
+                    a.Wout[q][o32] = q >= 1 && q <= 3 && (flip >> (q - 1) & 1) ? -w : w;
+                }
+                a.Tout[o32] = a.Tout[s32];
+                return;
             }
+#pragma unroll
+            for (int q = 0; q < 5; ++q) U[q] = a.Uout[q][s];  // new value, already clamped
         } else {
 #pragma unroll
             for (int q = 0; q < 5; ++q) U[q] = a.U0[q][s];
