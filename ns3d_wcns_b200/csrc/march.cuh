@@ -18,8 +18,7 @@
 // segment recomputes the five faces it shares with its neighbours.
 #pragma once
 
-#include "sweep.cuh"
-#include "sweep_pair.cuh"
+#include "pair.cuh"
 
 namespace ns3d {
 
@@ -676,11 +675,6 @@ inline long sweep_blocks(const SweepArgs<R> &a) {
     const dim3 g = sweep_grid<DIR, R>(a, len);
     return (long)g.x * g.y * g.z;
 }
-
-// Component-wise schemes march; characteristic reconstruction, whose bases
-// and projections want the registers, keeps the chunked kernel.
-inline bool march_takes(const SweepArgs<double> &a) { return !a.sp.char_recon; }
-inline bool march_takes(const SweepArgs<float> &a) { return !a.sp.char_recon && !sweep32_scalar_forced(); }
 
 // The scheme's instantiation: the interpolation always compiled in, the
 // Riemann solver for the schemes' usual partners.

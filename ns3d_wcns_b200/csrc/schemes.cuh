@@ -237,28 +237,6 @@ NS3D_HD bool mdcd_smooth(R fm2, R fm1, R f0, R fp1, R fp2) {
     return lhs > rhs;
 }
 
-// The cross-multiplied decision alone, without a branch: near is set (FP64)
-// where the two sides are too close for it, and the caller then takes
-// mdcd_smooth's decision instead (once for all the detectors of a cell, so
-// the common path has no branch per detector).  Wherever near stays clear the
-// value equals mdcd_smooth's.
-template <typename R>
-NS3D_HD bool mdcd_smooth_fast(R fm2, R fm1, R f0, R fp1, R fp2, bool &near) {
-    const R eps = R(0.9 * 0.4 / (1.0 - 0.9 * 0.4) * 1e-4);
-    R a = fabs(f0 - fm1) + fabs(f0 - R(2) * fm1 + fm2);
-    R b = fabs(f0 - fp1) + fabs(f0 - R(2) * fp1 + fp2);
-    // (FP64: both sides times 5/2, two instructions fewer)
-    const R lhs = sizeof(R) == 8 ? R(5) * a * b + R(2.5) * eps : R(2) * a * b + eps;
-    const R rhs = sizeof(R) == 8 ? a * a + (b * b + eps) : R(0.4) * (a * a + b * b + eps);
-    if constexpr (sizeof(R) == 8) {
-        // where near stays clear the high words decide (both sides are positive)
-        const int d = f64_hi_word(lhs) - f64_hi_word(rhs);
-        near |= (unsigned)(d + 1) <= 2u;
-        return d > 0;
-    }
-    return lhs > rhs;
-}
-
 // The non-linear branch: 4-stencil WENO with weights d_k (20 + tau6/(beta_k +
 // 1e-40))^2 (interpolation.cpp:170-208).
 template <typename R>

@@ -1,4 +1,5 @@
-// sweep.cuh -- fused inviscid + viscous sweep along one direction.
+// sweep.cuh -- what the sweeps share, and the sweep with characteristic
+// reconstruction.
 //
 // One kernel per direction performs, for every interior line of the domain:
 //   primitive -> conserved conversion (field_structures.h:468-488),
@@ -9,7 +10,10 @@
 //   and this direction's term of the viscous divergence: the derivative of the
 //   node viscous fluxes along the line with the reference's boundary orders
 //   (compute_vis_flux, ViscousFlux.cpp:210-255),
-// accumulated into the RHS.
+// accumulated into the RHS.  Component-wise schemes run in sweep_line.cuh (a
+// line per warp) and march.cuh (a line per thread); sweep_kernel is left with
+// characteristic reconstruction, whose bases and projections want a face per
+// thread and its registers.
 //
 // A thread block owns a bundle of lines and marches along them in chunks of C
 // faces.  Conserved cells, viscous node fluxes and face fluxes live in
@@ -47,9 +51,8 @@ namespace ns3d {
 //     stage increment D (both staged with cp.async) give U_s = U0 + D_s;
 //     stages 1 and 2 store the next increment (D_1 = dt L0, D_2 = (D_1 +
 //     dt L1) / 4) in D, stage 3 the FP64 state U0 + 2/3 (D_2 + dt L2) in
-//     Uout.  The FP32 primitives / temperature of U_s are rewritten in place
-//     (W32out, T32out): the first five cells of a periodic line are re-read
-//     by its wrapped end, so their new primitives are written after the line.
+//     Uout.  The FP32 primitives of U_s go to another buffer than the one the
+//     sweep reads (W32out), the temperature is rewritten in place (T32out).
 struct FusedStage {
     int stage;
     const double *W0[5];
@@ -98,18 +101,10 @@ struct SweepArgs {
 // At the end of a chunk the tails are moved to the front and the staged next
 // cells appended, so every stencil read is a fixed offset from the thread's
 // own position.
-// FP64 y/z chunk geometry (faces per chunk, lines per block; C * NLINE = 256)
-#ifndef NS3D_SWEEP64_YZ_C
-#define NS3D_SWEEP64_YZ_C 8
-#endif
-#ifndef NS3D_SWEEP64_YZ_NL
-#define NS3D_SWEEP64_YZ_NL 32
-#endif
 template <int DIR, typename R>
 struct SweepGeom {
-    static constexpr bool F64 = sizeof(R) == 8;
-    static constexpr int C = DIR == 0 ? 32 : (F64 ? NS3D_SWEEP64_YZ_C : 8);        // faces per chunk
-    static constexpr int NLINE = DIR == 0 ? 8 : (F64 ? NS3D_SWEEP64_YZ_NL : 32);  // lines per block
+    static constexpr int C = DIR == 0 ? 32 : 8;      // faces per chunk
+    static constexpr int NLINE = DIR == 0 ? 8 : 32;  // lines per block
     static constexpr int CH = C * NLINE;               // threads
     static constexpr int NU = C + 5, NF = C + 7, NV = C + 8;
     // along x a warp owns one line ([line][pos]); along y/z the lanes span
@@ -123,24 +118,13 @@ struct SweepGeom {
     }
 };
 
-// The old RHS of the updated cell is staged in shared memory with the next
-// chunk's cells (true) or loaded into registers (false).
-constexpr bool kRoldSmem = true;
-// minimum resident blocks per SM requested from the register allocator
-#ifndef NS3D_SWEEP64_MINB
-#define NS3D_SWEEP64_MINB 2
-#endif
+// buffers U(5) F(5) V(4) W(5, the characteristic bases), staging W(5)+V(4),
+// old RHS(5); z-sweep: the fused stage's state
 template <int DIR, typename R>
-constexpr int sweep_min_blocks() { return sizeof(R) == 8 ? NS3D_SWEEP64_MINB : 2; }
-
-// buffers U(5) F(5) V(4) [W(5) for characteristic bases], staging W(5)+V(4)
-// [+ old RHS(5)]
-template <int DIR, typename R, bool CHARW>
 constexpr size_t sweep_smem_bytes() {
     using G = SweepGeom<DIR, R>;
-    return sizeof(R) * ((size_t)G::NLINE * (5 * G::NU + 5 * G::NF + 4 * G::NV + (CHARW ? 5 * G::NU : 0)) +
-                        (size_t)(kRoldSmem ? 14 : 9) * G::CH) +
-           (DIR == 2 ? (size_t)5 * G::CH * (sizeof(double) + (sizeof(R) == 4 ? sizeof(float) : 0)) : 0);  // fused stage
+    return sizeof(R) * ((size_t)G::NLINE * (10 * G::NU + 5 * G::NF + 4 * G::NV) + (size_t)14 * G::CH) +
+           (DIR == 2 ? (size_t)5 * G::CH * (sizeof(double) + (sizeof(R) == 4 ? sizeof(float) : 0)) : 0);
 }
 
 template <typename R>
@@ -210,35 +194,18 @@ __device__ __forceinline__ void fused_stage_cell(const FusedStage &f, double dt,
     }
 }
 
-// The detector bits of a cell (and of the line's first cell) again with
-// mdcd_smooth's exact decisions, for the rare cell where one of the
-// cross-multiplied tests was too close to call.  Stencils re-read from shared
-// memory, so no registers stay alive across the common path.
-template <typename R, int NL, int NU, typename G>
-__device__ __noinline__ uint2 detect_exact(const R *sU, int line, int slot, bool first) {
-    unsigned r3 = 0, r2f = 0;  // as in the sweep: bit q for cell f+1 / f
-    for (int q = 0; q < 5; ++q) {
-        R sq[6];
-        for (int m = 0; m < 6; ++m) sq[m] = sU[q * NL * NU + G::template idx<NU>(line, slot + m)];
-        r3 |= (mdcd_smooth(sq[1], sq[2], sq[3], sq[4], sq[5]) ? 0u : 1u) << q;
-        if (first) r2f |= (mdcd_smooth(sq[0], sq[1], sq[2], sq[3], sq[4]) ? 0u : 1u) << q;
-    }
-    return make_uint2(r3, r2f);
-}
-
-template <int DIR, typename R, int INTERP, int RS, int CHAR>
-__global__ void __launch_bounds__(256, sweep_min_blocks<DIR, R>())
+template <int DIR, typename R, int INTERP>
+__global__ void __launch_bounds__(256, 2)
 sweep_kernel(SweepArgs<R> a) {
     using G = SweepGeom<DIR, R>;
     constexpr int C = G::C, NL = G::NLINE, CH = G::CH, NU = G::NU, NF = G::NF, NV = G::NV;
-    constexpr bool USE_W = (CHAR != 0);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *const sU = reinterpret_cast<R *>(smem_raw);  // [5][NL*NU]
     R *const sF = sU + 5 * NL * NU;                  // [5][NL*NF]
     R *const sV = sF + 5 * NL * NF;                  // [4][NL*NV]
-    R *const sW = sV + 4 * NL * NV;                  // [5][NL*NU] characteristic bases only
-    R *const stg = sW + (USE_W ? 5 * NL * NU : 0);   // [9][CH]
-    R *const srold = stg + 9 * CH;                   // [5][CH] (kRoldSmem)
+    R *const sW = sV + 4 * NL * NV;                  // [5][NL*NU] primitives, the characteristic bases
+    R *const stg = sW + 5 * NL * NU;                 // [9][CH]
+    R *const srold = stg + 9 * CH;                   // [5][CH]
     // fused stage (z-sweep): staged FP64 step-start state, and (mixed) the FP32 increment
     double *const sUf = reinterpret_cast<double *>(srold + 5 * CH);  // z fused stage: [5][CH] FP64
     float *const sDs = reinterpret_cast<float *>(sUf + 5 * CH);       // mixed: [5][CH] stage increment
@@ -249,16 +216,6 @@ sweep_kernel(SweepArgs<R> a) {
     const double fdt = (DIR == 2 && a.fs.stage) ? (a.fs.dt_dev ? *a.fs.dt_dev : a.fs.dt) : 0.0;
     double cfl_acc = 0.0, ke_acc = 0.0, ke_c = 0.0;  // largest wave speed, kinetic energy
     const double irg = (DIR == 2 && sizeof(R) == 4 && a.fs.stage) ? 1.0 / a.fs.Rgas : 0.0;  // mixed: T = p / (rho Rgas)
-    // mixed fused stage: the deferred new primitives of one of a periodic line's first five cells
-    bool has_def = false;
-    long def_id = 0;
-    unsigned det_carry = 0;  // x-sweep detector bits of the previous chunk's last face (cell fc)
-    // y/z-sweep detector bits, position p <-> cell fc + p (MDCD_HYBRID)
-    __shared__ unsigned char sDet[(DIR != 0 && CHAR == 0 && INTERP == I_MDCD_HYBRID) ? (C + 1) * NL : 1];
-    // periodic x-lines: faces 0 .. 4 of each line, kept from the first chunk
-    // for faces n .. n+4 (the same wrapped cells, so the same bits)
-    __shared__ R sWrapF[(DIR == 0 && CHAR == 0 && INTERP == I_MDCD_HYBRID) ? 25 * NL : 1];
-    float def_w[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, def_t = 0.f;
     const int slot = DIR == 0 ? threadIdx.x : threadIdx.y;
     const int line = DIR == 0 ? threadIdx.y : threadIdx.x;
     const int ta0 = blockIdx.x * NL + line, tb0 = blockIdx.y + (DIR == 2 ? 0 : a.zlo);
@@ -285,7 +242,6 @@ sweep_kernel(SweepArgs<R> a) {
     const int fe = min(c1 + 2, per ? n + 5 : n + NG);          // one past the last computed face
     const int cell_end = min(c1 + 5, per ? n + 8 : n + 6);     // one past the last cell needed
     const int chunk_end = c1 + 2;                              // chunks run while fc - 2 < c1
-    const bool whole = gridDim.z == 1;
     const int ti = G::tidx(line, slot);
 
     auto wrap = [&](int c) { return per ? (c < NG ? c + n : (c >= n + NG ? c - n : c)) : c; };
@@ -303,7 +259,7 @@ sweep_kernel(SweepArgs<R> a) {
         const int s = G::template idx<NU>(line, pu);
 #pragma unroll
         for (int q = 0; q < 5; ++q) sU[q * NL * NU + s] = U[q];
-        if (USE_W) {
+        {
             R *w5 = sW + s;
             w5[0] = r <= R(0) ? R(1e-12) : r; w5[NL * NU] = u; w5[2 * NL * NU] = v;
             w5[3 * NL * NU] = w; w5[4 * NL * NU] = p;
@@ -349,13 +305,8 @@ sweep_kernel(SweepArgs<R> a) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) rold[q] = R(0);
         if (rmw && upd) {
-            if constexpr (kRoldSmem) {
 #pragma unroll
-                for (int q = 0; q < 5; ++q) cp_async(&srold[q * CH + ti], a.Rhs[q] + cid);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) rold[q] = a.Rhs[q][cid];
-            }
+            for (int q = 0; q < 5; ++q) cp_async(&srold[q * CH + ti], a.Rhs[q] + cid);
         }
         if constexpr (DIR == 2 && sizeof(R) == 8) {
             if (a.fs.stage > 1 && upd) {  // the step-start primitives of the cell this thread updates
@@ -374,7 +325,7 @@ sweep_kernel(SweepArgs<R> a) {
                 }
             }
         }
-        if constexpr (kRoldSmem) cp_async_commit();
+        cp_async_commit();
         // stage the next chunk's new cell (cell and visc positions 5+slot, 8+slot)
         const int cn = fc + C + 3 + slot;
         const bool stage = fc + C < chunk_end && line_ok && cn < cell_end;
@@ -398,164 +349,7 @@ sweep_kernel(SweepArgs<R> a) {
 
         // ---- face f = fc + slot (between cells f and f+1): cell positions slot .. slot+5
         const int f = fc + slot;
-        if constexpr (DIR == 0 && CHAR == 0 && INTERP == I_MDCD_HYBRID) {
-            // Along x a warp is one line and its lanes are consecutive faces.
-            // The detector at a face's right-hand centre (cell f+1) is the
-            // left-hand centre of the next face, so each lane evaluates one
-            // centre and takes the other from the lane before it (lane 0: from
-            // lane 31 of the previous chunk; in the first chunk it evaluates
-            // both).  Same values as evaluating both centres per face.
-            if (line_ok && per && whole && fc >= n) {
-                // the last chunk of a periodic line holds only faces n .. n+4
-                // (fc >= n: uniform over the block): copies of faces 0 .. 4
-                if (f < fe) {
-#pragma unroll
-                    for (int q = 0; q < 5; ++q)
-                        sF[q * NL * NF + G::template idx<NF>(line, slot + 5)] = sWrapF[(q * NL + line) * 5 + (f - n)];
-                }
-            } else if (line_ok) {  // uniform over the warp
-                // one variable's stencil at a time (its registers die with it);
-                // the rare WENO branch re-reads its stencil from shared memory
-                R UL[5], UR[5];
-                unsigned r3 = 0, r2f = 0;  // bit q: the detector rejects the linear scheme at cell f+1 / f
-                bool near = false;
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    R sq[6];
-#pragma unroll
-                    for (int m = 0; m < 6; ++m) sq[m] = sU[q * NL * NU + G::template idx<NU>(line, slot + m)];
-                    r3 |= (mdcd_smooth_fast(sq[1], sq[2], sq[3], sq[4], sq[5], near) ? 0u : 1u) << q;
-                    if (fc == fb && slot == 0)
-                        r2f |= (mdcd_smooth_fast(sq[0], sq[1], sq[2], sq[3], sq[4], near) ? 0u : 1u) << q;
-                    UL[q] = mdcd_linear(a.sp.lin, sq[0], sq[1], sq[2], sq[3], sq[4], sq[5]);
-                    UR[q] = mdcd_linear(a.sp.lin, sq[5], sq[4], sq[3], sq[2], sq[1], sq[0]);
-                }
-                if (near) {
-                    const uint2 e = detect_exact<R, NL, NU, G>(sU, line, slot, fc == fb && slot == 0);
-                    r3 = e.x;
-                    r2f = e.y;
-                }
-                unsigned r2 = __shfl_up_sync(0xffffffffu, r3, 1);
-                if (slot == 0) r2 = fc == fb ? r2f : det_carry;
-                det_carry = __shfl_sync(0xffffffffu, r3, 31);
-                if (f < fe) {
-                    const unsigned weno = r2 | r3;
-                    if (weno) {
-#pragma unroll
-                        for (int q = 0; q < 5; ++q)
-                            if (weno & (1u << q)) {
-                                const volatile R *vq = sU + q * NL * NU;
-                                R sq[6];
-#pragma unroll
-                                for (int m = 0; m < 6; ++m) sq[m] = vq[G::template idx<NU>(line, slot + m)];
-                                UL[q] = mdcd_weno_branch(a.sp.hd, sq[0], sq[1], sq[2], sq[3], sq[4], sq[5]);
-                                UR[q] = mdcd_weno_branch(a.sp.hd, sq[5], sq[4], sq[3], sq[2], sq[1], sq[0]);
-                            }
-                    }
-                    R F[5];
-                    riemann<DIR, R, RS>(a.sp, UL, UR, F);
-                    const int s = G::template idx<NF>(line, slot + 5);
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
-                    if (per && whole && f < 5) {  // first chunk (fb = 0 on periodic lines)
-#pragma unroll
-                        for (int q = 0; q < 5; ++q) sWrapF[(q * NL + line) * 5 + f] = F[q];
-                    }
-                }
-            }
-        } else if constexpr (DIR != 0 && CHAR == 0 && INTERP == I_MDCD_HYBRID) {
-            // Along y and z the faces of a line are spread over the warps:
-            // each face evaluates the detector at its right-hand centre (cell
-            // f+1) into shared memory and, after a barrier, reads its
-            // left-hand centre (cell f) written by the face before it.  Cell
-            // fc comes from the previous chunk's last face (moved with the
-            // tails); the first chunk's first face evaluates it.
-            const bool act = line_ok && f < fe;
-            // one variable's stencil at a time (its registers die with it);
-            // the rare WENO branch re-reads its stencil from shared memory
-            R UL[5], UR[5];
-            unsigned r3 = 0;
-            if (act) {
-                unsigned r2f = 0;
-                bool near = false;
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    R sq[6];
-#pragma unroll
-                    for (int m = 0; m < 6; ++m) sq[m] = sU[q * NL * NU + G::template idx<NU>(line, slot + m)];
-                    r3 |= (mdcd_smooth_fast(sq[1], sq[2], sq[3], sq[4], sq[5], near) ? 0u : 1u) << q;
-                    if (fc == fb && slot == 0)
-                        r2f |= (mdcd_smooth_fast(sq[0], sq[1], sq[2], sq[3], sq[4], near) ? 0u : 1u) << q;
-                    UL[q] = mdcd_linear(a.sp.lin, sq[0], sq[1], sq[2], sq[3], sq[4], sq[5]);
-                    UR[q] = mdcd_linear(a.sp.lin, sq[5], sq[4], sq[3], sq[2], sq[1], sq[0]);
-                }
-                if (near) {
-                    const uint2 e = detect_exact<R, NL, NU, G>(sU, line, slot, fc == fb && slot == 0);
-                    r3 = e.x;
-                    r2f = e.y;
-                }
-                sDet[(slot + 1) * NL + line] = (unsigned char)r3;
-                if (fc == fb && slot == 0) sDet[line] = (unsigned char)r2f;
-            }
-            __syncthreads();  // detector bits of this chunk's cells complete
-            if (act) {
-                const unsigned weno = r3 | sDet[slot * NL + line];
-                if (weno) {
-#pragma unroll
-                    for (int q = 0; q < 5; ++q)
-                        if (weno & (1u << q)) {
-                            const volatile R *vq = sU + q * NL * NU;
-                            R sq[6];
-#pragma unroll
-                            for (int m = 0; m < 6; ++m) sq[m] = vq[G::template idx<NU>(line, slot + m)];
-                            UL[q] = mdcd_weno_branch(a.sp.hd, sq[0], sq[1], sq[2], sq[3], sq[4], sq[5]);
-                            UR[q] = mdcd_weno_branch(a.sp.hd, sq[5], sq[4], sq[3], sq[2], sq[1], sq[0]);
-                        }
-                }
-                R F[5];
-                riemann<DIR, R, RS>(a.sp, UL, UR, F);
-                const int s = G::template idx<NF>(line, slot + 5);
-#pragma unroll
-                for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
-            }
-        } else if (CHAR == 0 && line_ok && f < fe) {
-            R st[5][6];
-#pragma unroll
-            for (int q = 0; q < 5; ++q)
-#pragma unroll
-                for (int m = 0; m < 6; ++m) st[q][m] = sU[q * NL * NU + G::template idx<NU>(line, slot + m)];
-            R UL[5], UR[5];
-            if constexpr (INTERP == I_MDCD_HYBRID) {
-                // detector of every variable, the linear states of all, then
-                // the WENO branch only where a detector rejected the linear
-                // scheme (rare): the common path has no divergent branch
-                unsigned weno = 0;
-#pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    const bool lin = mdcd_smooth(st[q][0], st[q][1], st[q][2], st[q][3], st[q][4]) &&
-                                     mdcd_smooth(st[q][1], st[q][2], st[q][3], st[q][4], st[q][5]);
-                    weno |= (lin ? 0u : 1u) << q;
-                    UL[q] = mdcd_linear(a.sp.lin, st[q][0], st[q][1], st[q][2], st[q][3], st[q][4], st[q][5]);
-                    UR[q] = mdcd_linear(a.sp.lin, st[q][5], st[q][4], st[q][3], st[q][2], st[q][1], st[q][0]);
-                }
-                if (weno) {
-#pragma unroll
-                    for (int q = 0; q < 5; ++q)
-                        if (weno & (1u << q)) {
-                            UL[q] = mdcd_weno_branch(a.sp.hd, st[q][0], st[q][1], st[q][2], st[q][3], st[q][4], st[q][5]);
-                            UR[q] = mdcd_weno_branch(a.sp.hd, st[q][5], st[q][4], st[q][3], st[q][2], st[q][1], st[q][0]);
-                        }
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) face_pair<R, INTERP>(a.sp, st[q], UL[q], UR[q]);
-            }
-            R F[5];
-            riemann<DIR, R, RS>(a.sp, UL, UR, F);
-            const int s = G::template idx<NF>(line, slot + 5);
-#pragma unroll
-            for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
-        } else if (CHAR != 0 && line_ok && f < fe) {
+        if (line_ok && f < fe) {
             // one copy of the side's code: the stencil read from the near or
             // the far end, on the basis of cell f or f + 1
             R UL[5], UR[5];
@@ -575,22 +369,16 @@ sweep_kernel(SweepArgs<R> a) {
                 }
             }
             R F[5];
-            riemann<DIR, R, RS>(a.sp, UL, UR, F);
+            riemann<DIR, R, RUNTIME>(a.sp, UL, UR, F);
             const int s = G::template idx<NF>(line, slot + 5);
 #pragma unroll
             for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];
         }
-        if constexpr (kRoldSmem) cp_async_wait<1>();  // this thread's old-RHS copies landed
+        cp_async_wait<1>();  // this thread's old-RHS copies landed
         __syncthreads();  // faces of this chunk complete
-        if constexpr (DIR != 0 && CHAR == 0 && INTERP == I_MDCD_HYBRID) {
-            // the last face's bits (cell fc + C) become the next chunk's cell fc
-            if (line_ok && slot == C - 1) sDet[line] = sDet[C * NL + line];
-        }
-        if constexpr (kRoldSmem) {
-            if (rmw && upd) {
+        if (rmw && upd) {
 #pragma unroll
-                for (int q = 0; q < 5; ++q) rold[q] = srold[q * CH + ti];
-            }
+            for (int q = 0; q < 5; ++q) rold[q] = srold[q * CH + ti];
         }
 
         // ---- cell cu: faces cu-3 .. cu+2 at positions slot .. slot+5,
@@ -682,16 +470,9 @@ sweep_kernel(SweepArgs<R> a) {
 #pragma unroll
                         for (int q = 0; q < 5; ++q) f.Uout[q][c64] = U[q];
                     }
-                    if (per && cu < NG + 5) {  // re-read by the line's wrapped end: write after the line
-                        has_def = true; def_id = cid;
 #pragma unroll
-                        for (int q = 0; q < 5; ++q) def_w[q] = (float)W[q];
-                        def_t = (float)(W[4] * ir * irg);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 5; ++q) f.W32out[q][cid] = (float)W[q];
-                        f.T32out[cid] = (float)(W[4] * ir * irg);
-                    }
+                    for (int q = 0; q < 5; ++q) f.W32out[q][cid] = (float)W[q];
+                    f.T32out[cid] = (float)(W[4] * ir * irg);
                     if (f.stage == 3) {
                         cfl_acc = fmax(cfl_acc, cfl_speed(U, f.gamma));
                         const double y = 0.5 * W[0] * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]) * f.vol - ke_c;
@@ -725,9 +506,8 @@ sweep_kernel(SweepArgs<R> a) {
                         sU[q * NL * NU + G::template idx<NU>(line, slot + 5)];
                     sF[q * NL * NF + G::template idx<NF>(line, slot - C + 5)] =
                         sF[q * NL * NF + G::template idx<NF>(line, slot + 5)];
-                    if (USE_W)
-                        sW[q * NL * NU + G::template idx<NU>(line, slot - C + 5)] =
-                            sW[q * NL * NU + G::template idx<NU>(line, slot + 5)];
+                    sW[q * NL * NU + G::template idx<NU>(line, slot - C + 5)] =
+                        sW[q * NL * NU + G::template idx<NU>(line, slot + 5)];
                 }
             }
             if (stage) {
@@ -739,13 +519,6 @@ sweep_kernel(SweepArgs<R> a) {
                 put_cell(5 + slot, 8 + slot, stg[ti], stg[CH + ti], stg[2 * CH + ti], stg[3 * CH + ti],
                          stg[4 * CH + ti], v4);
             }
-        }
-    }
-    if constexpr (DIR == 2 && sizeof(R) == 4) {
-        if (has_def) {  // the line is done: nothing reads these cells any more
-#pragma unroll
-            for (int q = 0; q < 5; ++q) a.fs.W32out[q][def_id] = def_w[q];
-            a.fs.T32out[def_id] = def_t;
         }
     }
     if (DIR == 2 && a.fs.stage == 3)  // uniform: every thread of the block arrives
@@ -783,22 +556,22 @@ inline dim3 sweep_grid(const SweepArgs<R> &a, int &seg_len) {
     return grid;
 }
 
-template <int DIR, typename R, int INTERP, int RS, int CHAR>
+template <int DIR, typename R, int INTERP>
 inline cudaError_t launch_sweep(SweepArgs<R> a, cudaStream_t st) {
     using G = SweepGeom<DIR, R>;
     dim3 block(DIR == 0 ? G::C : G::NLINE, DIR == 0 ? G::NLINE : G::C);
     const dim3 grid = sweep_grid<DIR, R>(a, a.seg_len);
-    const size_t smem = sweep_smem_bytes<DIR, R, CHAR != 0>();
+    const size_t smem = sweep_smem_bytes<DIR, R>();
     static unsigned configured = 0;  // one bit per device ordinal
     int dev = 0;
     cudaGetDevice(&dev);
     if (!(configured & (1u << (dev & 31)))) {
-        cudaError_t e = cudaFuncSetAttribute(sweep_kernel<DIR, R, INTERP, RS, CHAR>,
+        cudaError_t e = cudaFuncSetAttribute(sweep_kernel<DIR, R, INTERP>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         configured |= 1u << (dev & 31);
     }
-    sweep_kernel<DIR, R, INTERP, RS, CHAR><<<grid, block, smem, st>>>(a);
+    sweep_kernel<DIR, R, INTERP><<<grid, block, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -814,22 +587,9 @@ cudaError_t sweep_z(const SweepArgs<float> &, cudaStream_t);
 // Characteristic reconstruction: the interpolation compiled in.
 template <int DIR, typename R>
 inline cudaError_t sweep_char(const SweepArgs<R> &a, cudaStream_t st) {
-    if (a.sp.interp == I_WENO5) return launch_sweep<DIR, R, I_WENO5, RUNTIME, 1>(a, st);
-    if (a.sp.interp == I_MDCD_LINEAR) return launch_sweep<DIR, R, I_MDCD_LINEAR, RUNTIME, 1>(a, st);
-    return launch_sweep<DIR, R, I_MDCD_HYBRID, RUNTIME, 1>(a, st);
-}
-
-// Every scheme: specialised instantiations for the usual pairs, generic otherwise.
-template <int DIR, typename R>
-inline cudaError_t sweep_select(const SweepArgs<R> &a, cudaStream_t st) {
-    const auto &sp = a.sp;
-    if (sp.char_recon) return sweep_char<DIR, R>(a, st);
-    if (sp.interp == I_WENO5 && sp.riemann == R_ROE) return launch_sweep<DIR, R, I_WENO5, R_ROE, 0>(a, st);
-    if (sp.interp == I_MDCD_HYBRID && sp.riemann == R_HLLC)
-        return launch_sweep<DIR, R, I_MDCD_HYBRID, R_HLLC, 0>(a, st);
-    if (sp.interp == I_MDCD_LINEAR && sp.riemann == R_HLLC)
-        return launch_sweep<DIR, R, I_MDCD_LINEAR, R_HLLC, 0>(a, st);
-    return launch_sweep<DIR, R, RUNTIME, RUNTIME, 0>(a, st);
+    if (a.sp.interp == I_WENO5) return launch_sweep<DIR, R, I_WENO5>(a, st);
+    if (a.sp.interp == I_MDCD_LINEAR) return launch_sweep<DIR, R, I_MDCD_LINEAR>(a, st);
+    return launch_sweep<DIR, R, I_MDCD_HYBRID>(a, st);
 }
 
 }  // namespace ns3d

@@ -4,10 +4,10 @@
 
 namespace ns3d {
 cudaError_t sweep_x(const SweepArgs<double> &a, cudaStream_t st) {
-    return march_takes(a) ? sweep_line_select<0, double>(a, st) : sweep_char<0, double>(a, st);
+    return !a.sp.char_recon ? sweep_line_select<0, double>(a, st) : sweep_char<0, double>(a, st);
 }
 cudaError_t sweep_x(const SweepArgs<float> &a, cudaStream_t st) {
-    if (!march_takes(a)) return sweep_select<0, float>(a, st);
-    return a.L.ny & 1 ? sweep_line_select<0, float>(a, st) : sweep_line_select<0, float2>(a, st);
+    if (a.sp.char_recon) return sweep_char<0, float>(a, st);
+    return a.L.ny & 1 || sweep32_scalar_forced() ? sweep_line_select<0, float>(a, st) : sweep_line_select<0, float2>(a, st);
 }
 }  // namespace ns3d

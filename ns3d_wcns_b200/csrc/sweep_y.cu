@@ -4,10 +4,10 @@
 
 namespace ns3d {
 cudaError_t sweep_y(const SweepArgs<double> &a, cudaStream_t st) {
-    return march_takes(a) ? line_or_march<1, double>(a, st) : sweep_char<1, double>(a, st);
+    return !a.sp.char_recon ? line_or_march<1, double>(a, st) : sweep_char<1, double>(a, st);
 }
 cudaError_t sweep_y(const SweepArgs<float> &a, cudaStream_t st) {
-    if (!march_takes(a)) return sweep_select<1, float>(a, st);
-    return a.L.nx & 1 ? line_or_march<1, float>(a, st) : line_or_march<1, float2>(a, st);
+    if (a.sp.char_recon) return sweep_char<1, float>(a, st);
+    return a.L.nx & 1 || sweep32_scalar_forced() ? line_or_march<1, float>(a, st) : line_or_march<1, float2>(a, st);
 }
 }  // namespace ns3d
