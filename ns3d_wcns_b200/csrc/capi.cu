@@ -1126,7 +1126,7 @@ int ns3d_create(const ns3d_params *params, const ns3d_grid *grid, ns3d_handle **
     bytes += 256;                                              // scalars
     {
         const dim3 sg = cell_grid(h->L64, true, STAGE_THREADS);
-        h->cfl_nblocks = (long)sg.x * sg.y * sg.z;
+        h->cfl_nblocks = std::max((long)sg.x * sg.y * sg.z, sweep_z_blocks_max(grid->nx, grid->ny, grid->nz));
     }
     bytes += 2 * (((size_t)h->cfl_nblocks * 8 + 255) / 256 * 256);  // stage CFL minima, kinetic energy
     bytes += 256;                                              // device clock

@@ -580,6 +580,7 @@ cudaError_t sweep_y(const SweepArgs<double> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<double> &, cudaStream_t);
 long sweep_z_blocks(const SweepArgs<double> &);
 long sweep_z_blocks(const SweepArgs<float> &);
+long sweep_z_blocks_max(long nx, long ny, long nz);
 cudaError_t sweep_x(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_y(const SweepArgs<float> &, cudaStream_t);
 cudaError_t sweep_z(const SweepArgs<float> &, cudaStream_t);

@@ -63,3 +63,27 @@ def _check(n, bcs, interp, rs):
             s.rk3_step(1e-4)
         for a, b in zip(interior(s.conserved()), interior(o.conserved())):
             assert rel_linf(a, b) <= 1e-6
+
+
+@pytest.mark.parametrize("n", [(592, 3, 3), (122, 16, 16), (122, 14, 4)], ids=str)
+@pytest.mark.parametrize("char_recon", [0, 1])
+def test_stage_partials(gpu_lib, n, char_recon):
+    """The time step and the kinetic energy come from the partials that the
+    z-sweep's blocks leave: more blocks than the padded grid has rows of 128.
+    Tolerance: the state's 1e-10."""
+    from ns3d_wcns_b200.solver import Solver
+    P, G = make_params(n=n, L=(6.0, 0.8, 0.9), interpolation=2, riemann=2, Re=300.0, cfl=0.4, char_recon=char_recon)
+    st = random_state(n, seed=9, amp=0.2)
+    o = oracle.PortSolver(P, G)
+    o.set_interior_prims(*st)
+    with Solver(P, G) as s:
+        s.set_interior_primitives(*st)
+        for _ in range(3):
+            dt = o.timestep()
+            assert abs(s.compute_timestep() / dt - 1) <= 1e-10
+            s.rk3_step(dt)
+            o.rk3_step(dt)
+        W = [interior(o.get(k)) for k in ("rho", "u", "v", "w")]
+        dv = 6.0 / n[0] * 0.8 / n[1] * 0.9 / n[2]
+        ke = float((0.5 * W[0] * (W[1] ** 2 + W[2] ** 2 + W[3] ** 2)).sum() * dv)
+        assert abs(s.total_energy() / ke - 1) <= 1e-10
