@@ -147,10 +147,17 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
     const int fb = per ? c0 - NG : max(c0 - NG, NG - 1);    // first face computed from cells
     const int fe = min(c1 + 2, per ? n + 5 : n + NG);       // one past the last computed face
     const int cell_end = min(c1 + 5, per ? n + 8 : n + 6);  // one past the last cell needed
-    const bool whole = gridDim.y == 1 && first == 0 && last == n;
+    const bool whole = gridDim.y == 1 && c1 - c0 == n;  // false for a warp without a line
+    // a whole periodic line of up to C cells in one chunk: its faces 0 .. n - 1
+    // are all there are, and the positions of cells -2 .. 2 update the cells
+    // n - 2 .. n + 2 that they repeat (64^3: x 31.1 -> 26.0 us FP64, 28.6 -> 21.1
+    // mixed, y mixed 38.0 -> 29.2; the second chunk held five faces)
+    const bool ring = per && whole && n <= C && n + 5 > C;
+    auto cell = [&](int cu) { return ring && cu < NG ? cu + n : cu; };  // the cell updated at position cu
+    auto update = [&](int cu) { return ring ? cu <= n - 3 : cu >= c0 && cu < c1; };
     auto wrap = [&](int c) { return per ? (c < NG ? c + n : (c >= n + NG ? c - n : c)) : c; };
     auto vis_pos = [&](int c) -> int {  // interior index of a node, -1: never read
-        if (c < 0) return -1;
+        if (c < 0 && !ring) return -1;
         int ci = c - NG;
         if (per) { if (ci < 0) ci += n; else if (ci >= n) ci -= n; return ci < n ? ci : -1; }
         return (ci >= 0 && ci < n) ? ci : -1;
@@ -194,13 +201,13 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
     unsigned carry = 0;  // march_doubt of cell fc
 #pragma unroll 1
     for (int fc = fb; fc - 2 < c1; fc += C) {
-        const bool more = fc + C - 2 < c1;
+        const bool more = !ring && fc + C - 2 < c1;
         if constexpr (DIR != 0) {  // the old right-hand side and step-start state of the cells updated
 #pragma unroll 1
             for (int s = lane; s < C; s += 32) {
                 const int cu = fc - 2 + s;
-                if (cu < c0 || cu >= c1) continue;
-                const uint32_t id = lbase + (uint32_t)cu * ls;
+                if (!update(cu)) continue;
+                const uint32_t id = lbase + (uint32_t)cell(cu) * ls;
                 if (rmw) {
 #pragma unroll
                     for (int q = 0; q < 5; ++q) march_cp(&sRO[q * C + s], a.Rhs[q] + id);
@@ -297,12 +304,22 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
             t.b = fn[1][q];
             *reinterpret_cast<Two *>(sF + q * S::NF + s0 + 6) = t;
         }
+        if (ring) {  // faces -5 .. -1 are faces n - 5 .. n - 1
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = f + h - n;
+                if (k >= -5 && k < 0) {
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) sF[q * S::NF + k + 6] = fn[h][q];
+                }
+            }
+        }
         if constexpr (DIR != 0) cp_async_wait<1>();
         __syncwarp();  // faces of this chunk complete, its old right-hand sides landed
         // ---- cells cu = f - 2 and cu + 1: faces cu - 3 .. cu + 3 at positions
         //      2 lane + 1 .. 2 lane + 7, nodes cu - 3 .. cu + 4 at 2 lane .. 2 lane + 7
         const int cu = f - 2;
-        const bool up0 = cu >= c0 && cu < c1, up1 = cu + 1 >= c0 && cu + 1 < c1;
+        const bool up0 = update(cu), up1 = update(cu + 1);
         if (up0 || up1) {
             T rq[2][5], ro[2][5];
 #pragma unroll
@@ -394,7 +411,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (!(h ? up1 : up0)) continue;
-                    const uint32_t id = lbase + (uint32_t)(cu + h) * ls;
+                    const uint32_t id = lbase + (uint32_t)cell(cu + h) * ls;
 #pragma unroll
                     for (int q = 0; q < 5; ++q) {
                         if constexpr (LN == 2 && DIR == 0) {
@@ -412,8 +429,8 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
 #pragma unroll 1
             for (int s = lane; s < C; s += 32) {
                 const int cl = fc - 2 + s;
-                if (cl < c0 || cl >= c1) continue;
-                const uint32_t cid = lbase + (uint32_t)cl * ls;
+                if (!update(cl)) continue;
+                const uint32_t cid = lbase + (uint32_t)cell(cl) * ls;
                 T r5[5];
 #pragma unroll
                 for (int q = 0; q < 5; ++q) r5[q] = sRO[q * C + s];
@@ -496,6 +513,13 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
     }
 }
 
+// Whole periodic lines of up to C cells take one chunk (see the kernel).
+template <int DIR, typename T>
+inline bool xline_ring(const SweepArgs<typename LaneOf<T>::R> &a) {
+    const int n = DIR == 0 ? a.L.nx : (DIR == 1 ? a.L.ny : a.L.nz);
+    return a.periodic && n <= XLine<DIR, T>::C && (DIR != 2 || (a.zlo == 0 && a.zhi == n));
+}
+
 template <int DIR, typename T>
 inline dim3 xline_grid(const SweepArgs<typename LaneOf<T>::R> &a, int resident, MarchArgs<T> &m) {
     const Layout &L = a.L;
@@ -503,7 +527,7 @@ inline dim3 xline_grid(const SweepArgs<typename LaneOf<T>::R> &a, int resident, 
     m.nlines = DIR == 0 ? L.ny / LaneOf<T>::N * (a.zhi - a.zlo)
                         : L.nx / LaneOf<T>::N * (DIR == 1 ? a.zhi - a.zlo : L.ny);
     const int nb = (m.nlines + XL_WARPS - 1) / XL_WARPS;
-    m.seg_len = sweep_segment(nb, n, XLine<DIR, T>::C, resident);
+    m.seg_len = xline_ring<DIR, T>(a) ? n : sweep_segment(nb, n, XLine<DIR, T>::C, resident);
     return dim3(nb, (n + m.seg_len - 1) / m.seg_len);
 }
 
@@ -554,16 +578,17 @@ inline cudaError_t sweep_line_select(const SweepArgs<typename LaneOf<T>::R> &a, 
 // at most twice along y and once along z, where the fused stage adds more
 // strided traffic.  us, march / line: FP64 y 16x16x16 14.7 / 10.5, 32^3 18.9 /
 // 12.8, 42 x 28 x 42 35.2 / 16.7, 56 x 59 x 56 (3136 chunks) 45.9 / 32.3, 48 x
-// 120 x 48 (4608) 45.0 / 58.1; z 32^3 20.0 / 16.0, 42^3 (1764) 34.2 / 24.6,
-// 48^3 (2304) WENO5 + Roe 28.9 / 28.5, 56^3 (3136) 35.4 / 43.5; FP32 pairs y 48^3
-// 31.4 / 18.7, 56 x 120 x 56 (3136) 39.6 / 35.5; z 48^3 (1152) 31.3 / 23.5, 59 x
-// 48 x 48 (1416) 33.8 / 36.1.
+// 120 x 48 (4608) 45.0 / 58.1, 64^3 (4096) WENO5 + Roe 35.4 / 35.3, MDCD_LINEAR
+// 23.1 / 35.7; z 32^3 20.0 / 16.0, 42^3 (1764) 34.2 / 24.6, 48^3 (2304) WENO5 +
+// Roe 28.9 / 28.5, 56^3 (3136) 35.4 / 43.5; FP32 pairs y 48^3 31.4 / 18.7, 56 x
+// 120 x 56 (3136) 39.6 / 35.5; z 48^3 (1152) 31.3 / 23.5, 59 x 48 x 48 (1416)
+// 33.8 / 36.1.
 template <int DIR, typename T>
 inline bool line_takes(const SweepArgs<typename LaneOf<T>::R> &a) {
     const int n = DIR == 1 ? a.L.ny : a.zhi - a.zlo, C = XLine<DIR, T>::C;
     const long lines = (long)(a.L.nx / LaneOf<T>::N) * (DIR == 1 ? a.zhi - a.zlo : a.L.ny);
     const long warps = 148L * XL_WARPS * xline_resident<DIR, T, I_MDCD_HYBRID, RUNTIME>();
-    return lines * ((n + 5 + C - 1) / C) <= (DIR == 1 ? 2 : 1) * warps;
+    return lines * (xline_ring<DIR, T>(a) ? 1 : (n + 5 + C - 1) / C) <= (DIR == 1 ? 2 : 1) * warps;
 }
 template <int DIR, typename T>
 inline cudaError_t line_or_march(const SweepArgs<typename LaneOf<T>::R> &a, cudaStream_t st) {

@@ -87,3 +87,12 @@ def test_stage_partials(gpu_lib, n, char_recon):
         dv = 6.0 / n[0] * 0.8 / n[1] * 0.9 / n[2]
         ke = float((0.5 * W[0] * (W[1] ** 2 + W[2] ** 2 + W[3] ** 2)).sum() * dv)
         assert abs(s.total_energy() / ke - 1) <= 1e-10
+
+
+@pytest.mark.parametrize("n", [(60, 61, 5), (64, 5, 62), (5, 63, 64), (62, 64, 60)], ids=str)
+@pytest.mark.parametrize("bcs", [(0,) * 6, (0, 0, 0, 0, 1, 3), (3, 2, 0, 0, 0, 0)], ids=["periodic", "xy", "yz"])
+@pytest.mark.parametrize("interp,rs", [(0, 0), (3, 2)])
+def test_one_chunk_lines(gpu_lib, n, bcs, interp, rs):
+    """Periodic lines of 60 to 64 cells take one chunk whose first positions
+    update the line's last cells."""
+    _check(n, bcs, interp, rs)
