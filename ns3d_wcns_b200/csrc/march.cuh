@@ -16,6 +16,13 @@
 // whatever nx is and its accesses stay contiguous.  A line is cut into
 // segments (gridDim.y) when there are too few lines to fill the chip; a
 // segment recomputes the five faces it shares with its neighbours.
+//
+// 256^3, one launch, against the chunked kernel (a face per thread, shared
+// stencils, three barriers a chunk) that it replaced: FP64 MDCD_HYBRID + HLLC y
+// 0.861 -> 0.710 ms, fused z 1.127 -> 0.922; WENO5 + Roe 1.222 -> 0.892 and 1.512
+// -> 1.065; mixed 0.431 -> 0.374 and 0.672 -> 0.618.  Issue and FP64 latency
+// bound it now: 11 warps per SM (168 registers), issue slots 48-54 % and the FP64
+// pipe 39-43 % busy, 3.4 TB/s.
 #pragma once
 
 #include "pair.cuh"
@@ -144,13 +151,39 @@ __device__ __forceinline__ float march_shfl(float2 v, int src, int line) {
     return line ? y : x;
 }
 
+// WENO states from the stencil g of a face: one side (right: from the reversed
+// stencil) into a, or both, the right one into b, through one copy of the code.
+// keep: the linear states stay (the reversed stencil gives the same decision).
+template <typename R, typename H>
+__device__ __forceinline__ void march_sides(const H &hd, bool both, bool right, const R *g, R &a, R &b, bool &keep) {
+    keep = false;
+    if constexpr (sizeof(R) == 8)
+        keep = mdcd_smooth(g[0], g[1], g[2], g[3], g[4]) && mdcd_smooth(g[1], g[2], g[3], g[4], g[5]);
+    a = b = R(0);
+    bool rev = right && !both;
+#pragma unroll 1
+    for (int e = 0; e <= (both ? 1 : 0); ++e) {
+        const R s = mdcd_weno_branch(hd, rev ? g[5] : g[0], rev ? g[4] : g[1], rev ? g[3] : g[2], rev ? g[2] : g[3],
+                                     rev ? g[1] : g[4], rev ? g[0] : g[5]);
+        if (e == 0) a = s;
+        else b = s;
+        rev = true;
+    }
+}
+
 // The states of the variables in doubt, for a warp in which some lane has
 // one: every (lane, variable, line) in doubt is a task, the tasks are dealt
-// out over the 32 lanes, each fetches its stencil by shuffles, takes the
-// exact decision (FP64) and evaluates both sides, and the results go back.
-// An under-resolved flow has a few tasks at most faces; one round then
-// replaces a divergent branch per variable and side, which the whole warp
-// would walk through (64^3 decaying turbulence, y-sweep: 60 -> 41 us).
+// out over pairs of lanes, one for each side, or, where they are more than
+// sixteen, over the lanes; a lane fetches its stencil by shuffles, takes the
+// exact decision (FP64) and evaluates its side or sides, and the results go
+// back.  An under-resolved flow has a
+// few tasks at most faces (64^3 decaying turbulence: 2.6 on average, some at
+// 87 % of the faces); one round then replaces a divergent branch per variable
+// and side, which the whole warp would walk through (y-sweep there: 60 -> 41 us
+// with both sides always in one lane; with the segments of today 50 -> 43 us
+// from that to this, z 55 -> 48, 96^3 x / y / z 76 / 92 / 105 -> 72 / 78 / 91, mixed
+// 128^3 90 / 91 / 137 -> 87 / 82 / 123; a flow with more than sixteen at most
+// faces, 64^3 later on, keeps its time, where sixteen at a time cost 8 % more).
 template <typename T>
 __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5], unsigned doubt, T *UL, T *UR) {
     using R = typename LaneOf<T>::R;
@@ -159,9 +192,12 @@ __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5
     int total = 0;
 #pragma unroll
     for (int v = 0; v < NV; ++v) total += __popc(__ballot_sync(0xffffffffu, (doubt >> v) & 1u));
+    int base = 0;
 #pragma unroll 1
-    for (int base = 0; base < total; base += 32) {
-        int var = -1, nth = 0, off = base + lane;  // this lane's task
+    do {
+        const bool both = total - base > 16;
+        const int sh = both ? 0 : 1, width = 32 >> sh;  // lanes per task, tasks of the round
+        int var = -1, nth = 0, off = base + (lane >> sh);  // this lane's task
         unsigned mask = 0;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -183,26 +219,27 @@ __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5
                 if (q0 == q) g[k] = x;
             }
         }
-        bool keep = false;  // the linear states stay
-        if constexpr (sizeof(R) == 8)
-            keep = mdcd_smooth(g[0], g[1], g[2], g[3], g[4]) && mdcd_smooth(g[1], g[2], g[3], g[4], g[5]);
-        const R l = mdcd_weno_branch(m.a.sp.hd, g[0], g[1], g[2], g[3], g[4], g[5]);
-        const R r = mdcd_weno_branch(m.a.sp.hd, g[5], g[4], g[3], g[2], g[1], g[0]);
-        int from = -base;  // the task of this lane's variable v sits in lane `from` + its rank
+        bool keep;
+        R sa, sb;
+        march_sides(m.a.sp.hd, both, (lane & 1) != 0, g, sa, sb, keep);
+        if (!both) sb = sa;
+        int from = -base;  // the task of this lane's variable v is number `from` + its rank of the round
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             const unsigned b = __ballot_sync(0xffffffffu, (doubt >> v) & 1u);
             if (!b) continue;
             const int t = from + __popc(b & ((1u << lane) - 1u));
-            const R lv = __shfl_sync(0xffffffffu, l, t & 31), rv = __shfl_sync(0xffffffffu, r, t & 31);
-            const bool kv = __shfl_sync(0xffffffffu, (int)keep, t & 31);
-            if (((doubt >> v) & 1u) && t >= 0 && t < 32 && !kv) {
+            const int at = (t << sh) & 31;
+            const R lv = __shfl_sync(0xffffffffu, sa, at), rv = __shfl_sync(0xffffffffu, sb, at + sh);
+            const bool kv = __shfl_sync(0xffffffffu, (int)keep, at);
+            if (((doubt >> v) & 1u) && t >= 0 && t < width && !kv) {
                 march_set(UL[v % 5], v / 5, lv);
                 march_set(UR[v % 5], v / 5, rv);
             }
             from += __popc(b);
         }
-    }
+        base += width;
+    } while (base < total);
 }
 
 // Left and right states of one variable at the face between f[2] and f[3]

@@ -57,7 +57,7 @@ struct XLine {
 };
 
 // Deals the (lane, face, variable, line) whose detector is in doubt out over
-// the warp's lanes, as march_weno; the stencils are in shared memory.
+// pairs of the warp's lanes, as march_weno; the stencils are in shared memory.
 // doubt: bit q + 5 line (+ NV for the lane's second face).
 template <typename T, typename A>
 __device__ __forceinline__ void xline_weno(const A &hd, const T *sU, unsigned doubt, T (*UL)[5], T (*UR)[5]) {
@@ -67,9 +67,12 @@ __device__ __forceinline__ void xline_weno(const A &hd, const T *sU, unsigned do
     int total = 0;
 #pragma unroll 1
     for (int v = 0; v < 2 * NV; ++v) total += __popc(__ballot_sync(0xffffffffu, (doubt >> v) & 1u));
+    int base = 0;
 #pragma unroll 1
-    for (int base = 0; base < total; base += 32) {
-        int var = 0, nth = 0, off = base + lane;  // this lane's task
+    do {
+        const bool both = total - base > 16;
+        const int sh = both ? 0 : 1, width = 32 >> sh;
+        int var = 0, nth = 0, off = base + (lane >> sh);  // this lane's task
         unsigned mask = 0;
 #pragma unroll 1
         for (int v = 0; v < 2 * NV; ++v) {
@@ -84,26 +87,27 @@ __device__ __forceinline__ void xline_weno(const A &hd, const T *sU, unsigned do
         R g[6];
 #pragma unroll
         for (int k = 0; k < 6; ++k) g[k] = st[k * LN];
-        bool keep = false;  // the linear states stay
-        if constexpr (sizeof(R) == 8)
-            keep = mdcd_smooth(g[0], g[1], g[2], g[3], g[4]) && mdcd_smooth(g[1], g[2], g[3], g[4], g[5]);
-        const R l = mdcd_weno_branch(hd, g[0], g[1], g[2], g[3], g[4], g[5]);
-        const R r = mdcd_weno_branch(hd, g[5], g[4], g[3], g[2], g[1], g[0]);
+        bool keep;
+        R sa, sb;
+        march_sides(hd, both, (lane & 1) != 0, g, sa, sb, keep);
+        if (!both) sb = sa;
         int from = -base;
 #pragma unroll
         for (int v = 0; v < 2 * NV; ++v) {
             const unsigned b = __ballot_sync(0xffffffffu, (doubt >> v) & 1u);
             if (!b) continue;
             const int t = from + __popc(b & ((1u << lane) - 1u));
-            const R lv = __shfl_sync(0xffffffffu, l, t & 31), rv = __shfl_sync(0xffffffffu, r, t & 31);
-            const bool kv = __shfl_sync(0xffffffffu, (int)keep, t & 31);
-            if (((doubt >> v) & 1u) && t >= 0 && t < 32 && !kv) {
+            const int at = (t << sh) & 31;
+            const R lv = __shfl_sync(0xffffffffu, sa, at), rv = __shfl_sync(0xffffffffu, sb, at + sh);
+            const bool kv = __shfl_sync(0xffffffffu, (int)keep, at);
+            if (((doubt >> v) & 1u) && t >= 0 && t < width && !kv) {
                 march_set(UL[v / NV][v % NV % 5], v % NV / 5, lv);
                 march_set(UR[v / NV][v % NV % 5], v % NV / 5, rv);
             }
             from += __popc(b);
         }
-    }
+        base += width;
+    } while (base < total);
 }
 
 template <int DIR, typename T, int INTERP, int RS>
