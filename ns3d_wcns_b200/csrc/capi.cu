@@ -437,7 +437,8 @@ SweepArgs<R> sweep_args(ns3d_handle *h, int dir) {
     // right) and the divergence of the node fluxes (right minus left)
     const double inv_h = dir == 0 ? h->ph.inv_dx : dir == 1 ? h->ph.inv_dy : h->ph.inv_dz;
     const double dc[3] = {75.0 / 64.0, -25.0 / 384.0, 3.0 / 640.0}, vc[3] = {45.0, -9.0, 1.0};
-    for (int k = 0; k < 3; ++k) { a.dc[k] = (R)(dc[k] * inv_h); a.vc[k] = (R)(vc[k] * (1.0 / (60.0 * hd))); }
+    a.inv_h = (R)inv_h;
+    for (int k = 0; k < 3; ++k) { a.dc[k] = (R)(m ? dc[k] : dc[k] * inv_h); a.vc[k] = (R)(vc[k] * (1.0 / (60.0 * hd))); }
     a.seg_len = 0;
     if constexpr (sizeof(R) == 8) a.sp = h->sp64; else a.sp = h->sp32;
     a.first = dir == 0;

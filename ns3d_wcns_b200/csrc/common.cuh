@@ -132,7 +132,7 @@ __device__ __forceinline__ double temperature_exact(const double W[5], double Rg
 // FP64.  Density clamp as field_structures.h:444-465.
 __device__ __forceinline__ void c2p_fast(const double U[5], double gamma, double W[5], double &irho) {
     const double rr = U[0] <= 0.0 ? 1e-12 : U[0];
-    irho = rcp_fp64(rr);
+    irho = 1.0 / rr;
     const double u = U[1] * irho, v = U[2] * irho, w = U[3] * irho;
     W[0] = rr; W[1] = u; W[2] = v; W[3] = w;
     W[4] = (gamma - 1.0) * (U[4] - 0.5 * rr * (u * u + v * v + w * w));

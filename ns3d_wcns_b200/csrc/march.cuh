@@ -46,8 +46,8 @@ template <typename T>
 struct MarchArgs {
     SweepArgs<typename LaneOf<T>::R> a;
     T lin[6];        // MDCD linear coefficients (both halves for float2)
-    T dc[3];         // half-node difference: 75/64, -25/384, 3/640 over h (InviscousFlux.cpp:990-992)
-    T vc[3];         // 6th-order derivative: 45, -9, 1 over 60 h (ViscousFlux.cpp:15-29)
+    T dc[3], inv_h;  // half-node difference (SweepArgs)
+    T vc[3], inv_60h;  // 6th-order derivative
     int nlines;      // line units: lines (pairs of lines for float2) of the swept planes
     int seg_len;     // cells per segment
 };
@@ -244,14 +244,16 @@ __device__ __forceinline__ void march_weno(const MarchArgs<T> &m, const T (*u)[5
 
 // Left and right states of one variable at the face between f[2] and f[3]
 // (MDCD_HYBRID: the linear ones).
-template <typename T, int INTERP>
+template <typename T, int INTERP, int RS>
 __device__ __forceinline__ void march_pair(const MarchArgs<T> &m, const T *f, T &l, T &r) {
     if constexpr (INTERP == I_WENO5) {
         if constexpr (LaneOf<T>::N == 2) weno5_pair<T>(PairOps(), f[0], f[1], f[2], f[3], f[4], f[5], l, r);
         else weno5_pair<T>(ScalarOps<T>(), f[0], f[1], f[2], f[3], f[4], f[5], l, r);
     } else if constexpr (LaneOf<T>::N == 2) {
-        l = mdcd_linear2(m.lin, f[0], f[1], f[2], f[3], f[4], f[5]);
-        r = mdcd_linear2(m.lin, f[5], f[4], f[3], f[2], f[1], f[0]);
+        // the order of the one-line form where the Riemann solver runs per line
+        constexpr bool ONE = RS != R_HLLC;
+        l = mdcd_linear2<ONE>(m.lin, f[0], f[1], f[2], f[3], f[4], f[5]);
+        r = mdcd_linear2<ONE>(m.lin, f[5], f[4], f[3], f[2], f[1], f[0]);
     } else {
         l = mdcd_linear(m.lin, f[0], f[1], f[2], f[3], f[4], f[5]);
         r = mdcd_linear(m.lin, f[5], f[4], f[3], f[2], f[1], f[0]);
@@ -260,12 +262,12 @@ __device__ __forceinline__ void march_pair(const MarchArgs<T> &m, const T *f, T 
 
 // Every variable of the face between u[2] and u[3]; doubt: march_doubt of the
 // two cells (MDCD_HYBRID).
-template <typename T, int INTERP>
+template <typename T, int INTERP, int RS>
 __device__ __forceinline__ void march_states(const MarchArgs<T> &m, const T (*u)[5], unsigned doubt, T *UL, T *UR) {
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
         const T f[6] = {u[0][q], u[1][q], u[2][q], u[3][q], u[4][q], u[5][q]};
-        march_pair<T, INTERP>(m, f, UL[q], UR[q]);
+        march_pair<T, INTERP, RS>(m, f, UL[q], UR[q]);
     }
     if constexpr (INTERP == I_MDCD_HYBRID) {
         if (__any_sync(0xffffffffu, doubt != 0)) march_weno<T>(m, u, doubt, UL, UR);
@@ -303,7 +305,7 @@ template <typename T>
 __device__ __forceinline__ void march_stage_mixed(const FusedStage &f, double dt, uint32_t cid, uint32_t c64, const T *rq,
                                                   const double *s0, const T *d, double &smax, double &ke, double &kc) {
     constexpr int LN = LaneOf<T>::N;
-    const double irg = rcp_fp64(f.Rgas);
+    const double irg = 1.0 / f.Rgas;
     T Dn[5], Wn[5], Tn;
 #pragma unroll
     for (int h = 0; h < LN; ++h) {
@@ -313,7 +315,9 @@ __device__ __forceinline__ void march_stage_mixed(const FusedStage &f, double dt
             const double rr = (double)march_half(rq[q], h), u0 = s0[q * LN + h];
             const double dp = f.stage == 1 ? 0.0 : (double)march_half(d[q], h);
             if (f.stage == 3) {
-                U[q] = u0 + (2.0 / 3.0) * (dp + dt * rr);
+                // rounded as written: as the former kernels of two lines and of one
+                const double d3 = __fma_rn(dt, rr, dp);
+                U[q] = LN == 2 ? __fma_rn(2.0 / 3.0, d3, u0) : __dadd_rn(u0, __dmul_rn(2.0 / 3.0, d3));
             } else {
                 const float dn = (float)(f.stage == 1 ? dt * rr : 0.25 * (dp + dt * rr));
                 march_set(Dn[q], h, dn);
@@ -537,7 +541,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
         }
         if (f >= f0 && (per || (f >= NG - 1 && f < n + NG))) {
             T UL[5], UR[5];
-            march_states<T, INTERP>(m, u, doubt, UL, UR);
+            march_states<T, INTERP, RS>(m, u, doubt, UL, UR);
             march_flux<DIR, T, RS>(a.sp, UL, UR, fn);
             if (!per && f == NG - 1 && a.outflow_lo) {  // ghost faces copy the boundary face
 #pragma unroll
@@ -566,7 +570,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
                     auto F = [&](unsigned o) { return *at(S::FL + o + q * S::slot); };
                     const T ro = rmw ? *slot(S::RO, q) : march_const<T>(0.0);
                     // faces cu - 1/2 and cu + 1/2 are f - 3 and f - 2
-                    rq[q] = diff3(m.dc, F(o2), F(o3), F(o1), F(o4), F(fo), fn[q], ro);
+                    rq[q] = face_diff(m.dc, m.inv_h, F(o2), F(o3), F(o1), F(o4), F(fo), fn[q], ro);
                 }
             }
             const bool edge = !per && (cu - NG < 3 || cu - NG >= n - 3);
@@ -576,7 +580,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     auto v = [&](unsigned o) { return *at(S::V + o + q * S::slot); };
-                    rq[q + 1] = diff3(m.vc, v(v4), v(v2), v(v5), v(v1), v(v6), v(vo), rq[q + 1]);
+                    rq[q + 1] = node_diff(m.vc, m.inv_60h, v(v4), v(v2), v(v5), v(v1), v(v6), v(vo), rq[q + 1]);
                 }
             } else if (visc) {
 #pragma unroll 1
@@ -678,6 +682,8 @@ inline MarchArgs<T> march_args(const SweepArgs<typename LaneOf<T>::R> &a) {
     };
     for (int k = 0; k < 6; ++k) m.lin[k] = both(a.sp.lin[k]);
     for (int k = 0; k < 3; ++k) { m.dc[k] = both(a.dc[k]); m.vc[k] = both(a.vc[k]); }
+    m.inv_h = both(a.inv_h);
+    m.inv_60h = both(a.dinv[2]);
     m.nlines = m.seg_len = 0;
     return m;
 }

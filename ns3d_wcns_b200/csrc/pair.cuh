@@ -53,18 +53,30 @@ struct PairOps {
     }
 };
 
-__device__ __forceinline__ float2 diff3(const float2 *c, float2 p1, float2 m1, float2 p2_, float2 m2, float2 p3, float2 m3,
-                                        float2 r) {
-    r = fma2(c[2], sub2(p3, m3), r);
-    r = fma2(c[1], sub2(p2_, m2), r);
-    return fma2(c[0], sub2(p1, m1), r);
+// The scaled sums are taken away from r, not added to it: sub2's multiply-add
+// takes a rounded product, where a product and add2 are contracted.
+__device__ __forceinline__ float2 face_diff(const float2 *dc, float2 inv_h, float2 l1, float2 r1, float2 l2, float2 r2,
+                                            float2 l3, float2 r3, float2 r) {
+    float2 t = mul2(sub2(r1, l1), dc[0]);
+    t = fma2(sub2(r2, l2), dc[1], t);
+    t = fma2(sub2(r3, l3), dc[2], t);
+    return sub2(r, mul2(t, inv_h));
+}
+__device__ __forceinline__ float2 node_diff(const float2 *, float2 inv_60h, float2 p1, float2 m1, float2 q2, float2 m2,
+                                            float2 p3, float2 m3, float2 r) {
+    float2 t = fma2(p2(-9.f), q2, p3);
+    t = fma2(p2(45.f), p1, t);
+    t = fma2(p2(-45.f), m1, t);
+    t = sub2(fma2(p2(9.f), m2, t), m3);
+    return sub2(r, mul2(make_float2(-t.x, -t.y), inv_60h));
 }
 
-// sum_k c_k f_k (mdcd_linear) for both lines
+// sum_k c_k f_k (mdcd_linear) for both lines; ONE: the first product rounded
+// with the sum and not on its own, as in the one-line form
+template <bool ONE>
 __device__ __forceinline__ float2 mdcd_linear2(const float2 *c, float2 f0, float2 f1, float2 f2, float2 f3,
                                                float2 f4, float2 f5) {
-    float2 s = mul2(c[0], f0);
-    s = fma2(c[1], f1, s);
+    float2 s = ONE ? fma2(c[0], f0, mul2(c[1], f1)) : fma2(c[1], f1, mul2(c[0], f0));
     s = fma2(c[2], f2, s);
     s = fma2(c[3], f3, s);
     s = fma2(c[4], f4, s);

@@ -57,6 +57,26 @@ NS3D_HD R quot_(R a, R b) {
     return a / b;
 }
 
+// a / b, rounded as the IEEE quotient (see div_fp64)
+template <typename R>
+NS3D_HD R div_(R a, R b) {
+#ifdef __CUDA_ARCH__
+    if constexpr (sizeof(R) == 8) return div_fp64(a, b, rcp_fp64(b));
+#endif
+    return a / b;
+}
+
+// FP32 operations rounded as written (nothing is contracted)
+#ifdef __CUDA_ARCH__
+NS3D_HD float add_rn(float a, float b) { return __fadd_rn(a, b); }
+NS3D_HD float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+NS3D_HD float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+#else
+NS3D_HD float add_rn(float a, float b) { return a + b; }
+NS3D_HD float mul_rn(float a, float b) { return a * b; }
+NS3D_HD float fma_rn(float a, float b, float c) { return std::fma(a, b, c); }
+#endif
+
 // ------------------------------------------------------------ interpolation
 
 // weno5_interpolate, interpolation.cpp:86-115: WCNS-E5 midpoint value from
@@ -171,12 +191,14 @@ NS3D_HD double mdcd_beta3(double f0, double f1, double f2, double f3, double f4,
             f4 * (3824847.0 * f4 - 1429976.0 * f5) + 139633.0 * (f5 * f5)) / 120960.0;
 }
 NS3D_HD float mdcd_beta3(float f0, float f1, float f2, float f3, float f4, float f5) {
-    const float d1 = f1 - f0, d2 = f2 - f0, d3 = f3 - f0, d4 = f4 - f0, d5 = f5 - f0;
-    float q = d1 * (5653317.f * d1 - 20427884.f * d2 + 17905032.f * d3 - 7727988.f * d4 + 1325006.f * d5) +
-              d2 * (19510972.f * d2 - 35817664.f * d3 + 15929912.f * d4 - 2792660.f * d5) +
-              d3 * (17195652.f * d3 - 15880404.f * d4 + 2863984.f * d5) +
-              d4 * (3824847.f * d4 - 1429976.f * d5) + 139633.f * (d5 * d5);
-    return q * (1.f / 120960.f) + f0 * f0 * (1.f / 6048.f);
+    const float d1 = add_rn(f1, -f0), d2 = add_rn(f2, -f0), d3 = add_rn(f3, -f0), d4 = add_rn(f4, -f0), d5 = add_rn(f5, -f0);
+    const float p1 = fma_rn(1325006.f, d5, fma_rn(-7727988.f, d4, fma_rn(17905032.f, d3, fma_rn(5653317.f, d1, mul_rn(-20427884.f, d2)))));
+    const float p2 = fma_rn(-2792660.f, d5, fma_rn(15929912.f, d4, fma_rn(19510972.f, d2, mul_rn(-35817664.f, d3))));
+    const float p3 = fma_rn(2863984.f, d5, fma_rn(17195652.f, d3, mul_rn(-15880404.f, d4)));
+    const float p4 = fma_rn(3824847.f, d4, mul_rn(-1429976.f, d5));
+    float q = fma_rn(d3, p3, fma_rn(d1, p1, mul_rn(d2, p2)));
+    q = fma_rn(139633.f, mul_rn(d5, d5), fma_rn(d4, p4, q));
+    return fma_rn(mul_rn(f0, f0), 1.f / 6048.f, mul_rn(q, 1.f / 120960.f));
 }
 
 // mdcd_hybrid_interpolate, interpolation.cpp:135-209, split into its
@@ -238,44 +260,60 @@ NS3D_HD bool mdcd_smooth(R fm2, R fm1, R f0, R fp1, R fp2) {
 }
 
 // The non-linear branch: 4-stencil WENO with weights d_k (20 + tau6/(beta_k +
-// 1e-40))^2 (interpolation.cpp:170-208).
+// 1e-40))^2 (interpolation.cpp:170-208), from the smoothness indicators and
+// the candidates (times eight).  The weights span far more than the FP32 range:
+// FP32 inputs quantise a smooth stencil to beta == 0 exactly, and (tau6 *
+// 1e40)^2 overflows to inf (inf/inf = NaN).  So the FP32 build forms the
+// weights and the normalisation in FP64, like the reference; this branch is
+// the rare one (most faces take the linear scheme).
 template <typename R>
-NS3D_HD R mdcd_weno_branch(const R *hd, R f0, R f1, R f2, R f3, R f4, R f5) {
-    const R eps_small = sizeof(R) == 8 ? R(1e-40) : R(1e-40f);
-    const R c13 = R(13.0 / 12.0);
-    R t, u;
-    t = f0 - R(2) * f1 + f2; u = f0 - R(4) * f1 + R(3) * f2;
-    R be0 = c13 * (t * t) + R(0.25) * (u * u);
-    t = f1 - R(2) * f2 + f3; u = f1 - f3;
-    R be1 = c13 * (t * t) + R(0.25) * (u * u);
-    t = f2 - R(2) * f3 + f4; u = R(3) * f2 - R(4) * f3 + f4;
-    R be2 = c13 * (t * t) + R(0.25) * (u * u);
-    R be3 = mdcd_beta3(f0, f1, f2, f3, f4, f5);
-    R q0 = R(3) * f0 - R(10) * f1 + R(15) * f2;
-    R q1 = -f1 + R(6) * f2 + R(3) * f3;
-    R q2 = R(3) * f2 + R(6) * f3 - f4;
-    R q3 = R(15) * f3 - R(10) * f4 + R(3) * f5;
-    // The weights span far more than the FP32 range: FP32 inputs quantise a
-    // smooth stencil to beta == 0 exactly, and (tau6 * 1e40)^2 overflows to
-    // inf (inf/inf = NaN).  So the FP32 build forms the weights and the
-    // normalisation in FP64, like the reference; this branch is the rare one
-    // (most faces take the linear scheme).
+NS3D_HD R mdcd_weno_weigh(const R *hd, R be0, R be1, R be2, R be3, R q0, R q1, R q2, R q3) {
     using Wt = double;
+    const Wt es = 1e-40;
     Wt tau6 = fabs((Wt)be3 - ((Wt)be0 + Wt(4) * (Wt)be1 + (Wt)be2) / Wt(6));
-    const Wt es = sizeof(R) == 8 ? (Wt)eps_small : Wt(1e-40);
-    Wt g0 = Wt(20) + quot_(tau6, (Wt)be0 + es);
-    Wt g1 = Wt(20) + quot_(tau6, (Wt)be1 + es);
-    Wt g2 = Wt(20) + quot_(tau6, (Wt)be2 + es);
-    Wt g3 = Wt(20) + quot_(tau6, (Wt)be3 + es);
+    Wt g0 = Wt(20) + div_(tau6, (Wt)be0 + es);
+    Wt g1 = Wt(20) + div_(tau6, (Wt)be1 + es);
+    Wt g2 = Wt(20) + div_(tau6, (Wt)be2 + es);
+    Wt g3 = Wt(20) + div_(tau6, (Wt)be3 + es);
     Wt al0 = (Wt)hd[0] * (g0 * g0), al1 = (Wt)hd[1] * (g1 * g1), al2 = (Wt)hd[2] * (g2 * g2),
        al3 = (Wt)hd[3] * (g3 * g3);
-    return (R)quot_(al0 * (Wt)q0 + al1 * (Wt)q1 + al2 * (Wt)q2 + al3 * (Wt)q3, Wt(8) * (al0 + al1 + al2 + al3));
+    return (R)div_(al0 * (Wt)q0 + al1 * (Wt)q1 + al2 * (Wt)q2 + al3 * (Wt)q3, Wt(8) * (al0 + al1 + al2 + al3));
+}
+NS3D_HD double mdcd_weno_branch(const double *hd, double f0, double f1, double f2, double f3, double f4, double f5) {
+    const double c13 = 13.0 / 12.0;
+    double t, u;
+    t = f0 - 2.0 * f1 + f2; u = f0 - 4.0 * f1 + 3.0 * f2;
+    const double be0 = c13 * (t * t) + 0.25 * (u * u);
+    t = f1 - 2.0 * f2 + f3; u = f1 - f3;
+    const double be1 = c13 * (t * t) + 0.25 * (u * u);
+    t = f2 - 2.0 * f3 + f4; u = 3.0 * f2 - 4.0 * f3 + f4;
+    const double be2 = c13 * (t * t) + 0.25 * (u * u);
+    return mdcd_weno_weigh(hd, be0, be1, be2, mdcd_beta3(f0, f1, f2, f3, f4, f5), 3.0 * f0 - 10.0 * f1 + 15.0 * f2,
+                           -f1 + 6.0 * f2 + 3.0 * f3, 3.0 * f2 + 6.0 * f3 - f4, 15.0 * f3 - 10.0 * f4 + 3.0 * f5);
+}
+// FP32, rounded as written: the hybrid scheme turns another placement of the
+// fused operations into another trajectory, so it is the same whichever
+// kernel asks.  ch: for characteristic variables, one sum of q1 fused.
+NS3D_HD float mdcd_weno_branch(const float *hd, float f0, float f1, float f2, float f3, float f4, float f5, bool ch = false) {
+    const float c13 = float(13.0 / 12.0);
+    auto ind = [&](float t, float u) { return fma_rn(c13, mul_rn(t, t), mul_rn(0.25f, mul_rn(u, u))); };
+    const float e2 = mul_rn(3.f, f2);
+    const float be0 = ind(add_rn(fma_rn(-2.f, f1, f0), f2), add_rn(fma_rn(-4.f, f1, f0), e2));
+    const float t1 = add_rn(fma_rn(-2.f, f2, f1), f3), u1 = add_rn(f1, -f3);
+    const float be1 = fma_rn(0.25f, mul_rn(u1, u1), mul_rn(c13, mul_rn(t1, t1)));
+    const float be2 = ind(add_rn(fma_rn(-2.f, f3, f2), f4), add_rn(fma_rn(-4.f, f3, e2), f4));
+    const float q0 = fma_rn(15.f, f2, fma_rn(3.f, f0, mul_rn(-10.f, f1)));
+    const float q1 = ch ? fma_rn(3.f, f3, fma_rn(6.f, f2, -f1)) : add_rn(mul_rn(3.f, f3), fma_rn(6.f, f2, -f1));
+    const float q2 = add_rn(fma_rn(6.f, f3, e2), -f4);
+    const float q3 = fma_rn(3.f, f5, fma_rn(15.f, f3, mul_rn(-10.f, f4)));
+    return mdcd_weno_weigh(hd, be0, be1, be2, mdcd_beta3(f0, f1, f2, f3, f4, f5), q0, q1, q2, q3);
 }
 
 template <typename R>
 NS3D_HD R mdcd_hybrid(const R *lin, const R *hd, R f0, R f1, R f2, R f3, R f4, R f5) {
     if (mdcd_smooth(f0, f1, f2, f3, f4) && mdcd_smooth(f1, f2, f3, f4, f5))
         return mdcd_linear(lin, f0, f1, f2, f3, f4, f5);
+    if constexpr (sizeof(R) == 4) return mdcd_weno_branch(hd, f0, f1, f2, f3, f4, f5, true);
     return mdcd_weno_branch(hd, f0, f1, f2, f3, f4, f5);
 }
 
@@ -351,7 +389,15 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     R FL[5], FR[5];
     L.flux(FL); Rt.flux(FR);
     const R gm1 = g - R(1);
-    R HL = (L.E + L.p) * L.ir, HR = (Rt.E + Rt.p) * Rt.ir;
+    R HL, HR;
+    if constexpr (sizeof(R) == 4) {
+        const R kfac = g / gm1;
+        HL = R(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w) + kfac * L.p * L.ir;
+        HR = R(0.5) * (Rt.u * Rt.u + Rt.v * Rt.v + Rt.w * Rt.w) + kfac * Rt.p * Rt.ir;
+    } else {
+        HL = (L.E + L.p) * L.ir;
+        HR = (Rt.E + Rt.p) * Rt.ir;
+    }
     R sL = sqrt_(L.r), sR = sqrt_(Rt.r);
     R den = rcp_(sL + sR);
     R ub = (sL * L.u + sR * Rt.u) * den;
@@ -380,18 +426,33 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     l0 = l0 < delta ? (l0 * l0 + d2) * i2d : l0;
     lv = lv < delta ? (lv * lv + d2) * i2d : lv;
     l4 = l4 < delta ? (l4 * l4 + d2) * i2d : l4;
-    const R k0 = (l0 - lv) * A0, k4 = (l4 - lv) * A4, ks = k0 + k4, kd = (k4 - k0) * c;
+    const R k0 = (l0 - lv) * A0, k4 = (l4 - lv) * A4;
     // R0 = (1, u-nc, v-nc, w-nc, H-cV), R4 = (1, u+nc, v+nc, w+nc, H+cV)
-    R D0 = lv * dU[0] + ks;
-    R D1 = lv * dU[1] + ks * ub + (DIR == 0 ? kd : R(0));
-    R D2 = lv * dU[2] + ks * vb + (DIR == 1 ? kd : R(0));
-    R D3 = lv * dU[3] + ks * wb + (DIR == 2 ? kd : R(0));
-    R D4 = lv * dU[4] + ks * Hb + kd * V;
-    F[0] = R(0.5) * (FL[0] + FR[0] - D0);
-    F[1] = R(0.5) * (FL[1] + FR[1] - D1);
-    F[2] = R(0.5) * (FL[2] + FR[2] - D2);
-    F[3] = R(0.5) * (FL[3] + FR[3] - D3);
-    F[4] = R(0.5) * (FL[4] + FR[4] - D4);
+    if constexpr (sizeof(R) == 4) {
+        R cx = DIR == 0 ? c : R(0), cy = DIR == 1 ? c : R(0), cz = DIR == 2 ? c : R(0);
+        R D0 = lv * dU[0] + k0 + k4;
+        R D1 = lv * dU[1] + k0 * (ub - cx) + k4 * (ub + cx);
+        R D2 = lv * dU[2] + k0 * (vb - cy) + k4 * (vb + cy);
+        R D3 = lv * dU[3] + k0 * (wb - cz) + k4 * (wb + cz);
+        R D4 = lv * dU[4] + k0 * (Hb - c * V) + k4 * (Hb + c * V);
+        F[0] = R(0.5) * (FL[0] + FR[0]) - R(0.5) * D0;
+        F[1] = R(0.5) * (FL[1] + FR[1]) - R(0.5) * D1;
+        F[2] = R(0.5) * (FL[2] + FR[2]) - R(0.5) * D2;
+        F[3] = R(0.5) * (FL[3] + FR[3]) - R(0.5) * D3;
+        F[4] = R(0.5) * (FL[4] + FR[4]) - R(0.5) * D4;
+    } else {
+        const R ks = k0 + k4, kd = (k4 - k0) * c;
+        R D0 = lv * dU[0] + ks;
+        R D1 = lv * dU[1] + ks * ub + (DIR == 0 ? kd : R(0));
+        R D2 = lv * dU[2] + ks * vb + (DIR == 1 ? kd : R(0));
+        R D3 = lv * dU[3] + ks * wb + (DIR == 2 ? kd : R(0));
+        R D4 = lv * dU[4] + ks * Hb + kd * V;
+        F[0] = R(0.5) * (FL[0] + FR[0] - D0);
+        F[1] = R(0.5) * (FL[1] + FR[1] - D1);
+        F[2] = R(0.5) * (FL[2] + FR[2] - D2);
+        F[3] = R(0.5) * (FL[3] + FR[3] - D3);
+        F[4] = R(0.5) * (FL[4] + FR[4] - D4);
+    }
 }
 
 // Rusanov_Riemann_solver, InviscousFlux.cpp:270-311.
@@ -453,7 +514,9 @@ NS3D_HD void hllc_star(const Side<DIR, R> &S, const R *U, const R *Fs, R Sk, R S
 //   rho* = m / (S_k - S_M), p* = p + m (S_M - u_n), m = rho (S_k - u_n),
 //   E* = ((S_k - u_n) E - p u_n + p* S_M) / (S_k - S_M),
 //   F = (rho* S_M, rho* S_M V + p* n, (E* + p*) S_M)
-// -- the same flux with half of the operations and one quotient less.
+// -- the same flux with half of the operations and one quotient less.  FP32
+// keeps hllc_star, as it keeps its form of the Roe dissipation: the hybrid
+// scheme turns another rounding into another trajectory.
 template <int DIR, typename R>
 NS3D_HD void hllc_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
@@ -463,6 +526,29 @@ NS3D_HD void hllc_flux(const R *UL, const R *UR, R g, R *F) {
     R SR = fmax(L.un + aL, Rt.un + aR);
     if (SL >= R(0)) { L.flux(F); return; }
     if (SR <= R(0)) { Rt.flux(F); return; }
+    if constexpr (sizeof(R) == 4) {
+        R num = Rt.r * Rt.un * (SR - Rt.un) - L.r * L.un * (SL - L.un) + L.p - Rt.p;
+        R den = Rt.r * (SR - Rt.un) - L.r * (SL - L.un);
+        R SM;
+        if (fabs(den) > R(1e-12)) {
+            SM = num / den;
+        } else {
+            R sL = sqrt(L.r), sR = sqrt(Rt.r);
+            SM = (sL * L.un + sR * Rt.un) / (sL + sR);
+        }
+        const bool left = SM >= R(0);
+        Side<DIR, R> S;
+        S.r = left ? L.r : Rt.r; S.ir = left ? L.ir : Rt.ir;
+        S.u = left ? L.u : Rt.u; S.v = left ? L.v : Rt.v; S.w = left ? L.w : Rt.w;
+        S.E = left ? L.E : Rt.E; S.p = left ? L.p : Rt.p; S.un = left ? L.un : Rt.un;
+        R Us[5];
+#pragma unroll
+        for (int n = 0; n < 5; ++n) Us[n] = left ? UL[n] : UR[n];
+        R Fs[5];
+        S.flux(Fs);
+        hllc_star<DIR, R>(S, Us, Fs, left ? SL : SR, SM, F);
+        return;
+    }
     const R dL = SL - L.un, dR = SR - Rt.un;
     const R mL = L.r * dL, mR = Rt.r * dR;
     const R num = mR * Rt.un - mL * L.un + L.p - Rt.p;
@@ -602,6 +688,83 @@ NS3D_HD void riemann(const SchemeParams<R> &sp, const R *UL, const R *UR, R *F) 
 }
 
 // ------------------------------------------------------- characteristic basis
+
+// build_eigen_matrices for the Roe average of a cell state with itself, as
+// WCNS_Riemann_InviscidFlux does for characteristic interpolation
+// (InviscousFlux.cpp:166-231 with :849-987).  w = primitive (rho,u,v,w,p).
+template <int DIR, typename R>
+NS3D_HD void cell_eigen(const R *w, R g, R Lm[5][5], R Rm[5][5]) {
+    const R nx = DIR == 0 ? R(1) : R(0), ny = DIR == 1 ? R(1) : R(0), nz = DIR == 2 ? R(1) : R(0);
+    const R gm1 = g - R(1);
+    R r = w[0], u = w[1], v = w[2], ww = w[3], p = w[4];
+    R E = r * (R(0.5) * (u * u + v * v + ww * ww) + p / (gm1 * r));
+    R sq = sqrt(r);
+    R rb = sq * sq;
+    R den = R(1) / (sq + sq);
+    R ub = (sq * u + sq * u) * den, vb = (sq * v + sq * v) * den, wb = (sq * ww + sq * ww) * den;
+    R H = (E + p) / r;
+    R Hb = (sq * H + sq * H) * den;
+    R c = sqrt(gm1 * (Hb - R(0.5) * (ub * ub + vb * vb + wb * wb)));
+    R V = nx * ub + ny * vb + nz * wb;
+    R phi = R(0.5) * gm1 * (ub * ub + vb * vb + wb * wb);
+    R a1 = gm1;
+    R a2 = R(1) / (sqrt(R(2)) * rb * c);
+    R a3 = rb / (sqrt(R(2)) * c);
+    R a4 = (phi + c * c) / gm1;
+    R ic2 = R(1) / (c * c), irb = R(1) / rb;
+    R a5 = R(1) - phi * ic2;
+    R a6 = phi / gm1;
+    Lm[0][0] = a2 * (phi + c * V); Lm[0][1] = -a2 * (a1 * ub + nx * c); Lm[0][2] = -a2 * (a1 * vb + ny * c);
+    Lm[0][3] = -a2 * (a1 * wb + nz * c); Lm[0][4] = a1 * a2;
+    Lm[1][0] = nx * a5 - (nz * vb - ny * wb) * irb; Lm[1][1] = nx * a1 * ub * ic2;
+    Lm[1][2] = nx * a1 * vb * ic2 + nz * irb; Lm[1][3] = nx * a1 * wb * ic2 - ny * irb; Lm[1][4] = -nx * a1 * ic2;
+    Lm[2][0] = nz * a5 - (ny * ub - nx * vb) * irb; Lm[2][1] = nz * a1 * ub * ic2 + ny * irb;
+    Lm[2][2] = nz * a1 * vb * ic2 - nx * irb; Lm[2][3] = nz * a1 * wb * ic2; Lm[2][4] = -nz * a1 * ic2;
+    Lm[3][0] = ny * a5 - (nx * wb - nz * ub) * irb; Lm[3][1] = ny * a1 * ub * ic2 - nz * irb;
+    Lm[3][2] = ny * a1 * vb * ic2; Lm[3][3] = ny * a1 * wb * ic2 + nx * irb; Lm[3][4] = -ny * a1 * ic2;
+    Lm[4][0] = a2 * (phi - c * V); Lm[4][1] = -a2 * (a1 * ub - nx * c); Lm[4][2] = -a2 * (a1 * vb - ny * c);
+    Lm[4][3] = -a2 * (a1 * wb - nz * c); Lm[4][4] = a1 * a2;
+    Rm[0][0] = a3; Rm[1][0] = a3 * (ub - nx * c); Rm[2][0] = a3 * (vb - ny * c); Rm[3][0] = a3 * (wb - nz * c);
+    Rm[4][0] = a3 * (a4 - c * V);
+    Rm[0][1] = nx; Rm[1][1] = nx * ub; Rm[2][1] = nx * vb + nz * rb; Rm[3][1] = nx * wb - ny * rb;
+    Rm[4][1] = nx * a6 + rb * (nz * vb - ny * wb);
+    Rm[0][2] = nz; Rm[1][2] = nz * ub + ny * rb; Rm[2][2] = nz * vb - nx * rb; Rm[3][2] = nz * wb;
+    Rm[4][2] = nz * a6 + rb * (ny * ub - nx * vb);
+    Rm[0][3] = ny; Rm[1][3] = ny * ub - nz * rb; Rm[2][3] = ny * vb; Rm[3][3] = ny * wb + nx * rb;
+    Rm[4][3] = ny * a6 + rb * (nx * wb - nz * ub);
+    Rm[0][4] = a3; Rm[1][4] = a3 * (ub + nx * c); Rm[2][4] = a3 * (vb + ny * c); Rm[3][4] = a3 * (wb + nz * c);
+    Rm[4][4] = a3 * (a4 + c * V);
+}
+
+// Both states of a face in that form, from the stencil of cells i-2 .. i+3 and
+// the primitives of the cells i and i+1 (FP32, whose rounding the hybrid
+// scheme turns into another trajectory; FP64 takes char_state).
+template <int DIR, typename R, int INTERP>
+NS3D_HD void char_pair(const SchemeParams<R> &sp, const R U[5][6], const R *wi, const R *wi1, R *UL, R *UR) {
+    R Lm[5][5], Rm[5][5], Q[5], Wc[6];
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+        cell_eigen<DIR, R>(side == 0 ? wi : wi1, sp.gamma, Lm, Rm);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+#pragma unroll
+            for (int m = 0; m < 6; ++m) {
+                R s = R(0);
+#pragma unroll
+                for (int r = 0; r < 5; ++r) s += Lm[n][r] * U[r][m];
+                Wc[m] = s;
+            }
+            Q[n] = interp_side<R, INTERP>(sp, Wc, side == 1);
+        }
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+            R s = R(0);
+#pragma unroll
+            for (int r = 0; r < 5; ++r) s += Rm[n][r] * Q[r];
+            if (side == 0) UL[n] = s; else UR[n] = s;
+        }
+    }
+}
 
 // One side's state of characteristic-wise interpolation: the stencil f(q, m)
 // (conserved variable q, m = 0 .. 5 counted towards the face) projected on the

@@ -81,8 +81,9 @@ struct SweepArgs {
     int periodic;       // this direction
     int outflow_lo, outflow_hi;  // ghost faces copy the boundary face (else zero)
     R dinv[3];          // 1/(2h), 1/(12h), 1/(60h): the viscous stencils' divisors
-    R dc[3];            // half-node difference: 75/64, -25/384, 3/640 over h
-    R vc[3];            // 6th-order derivative: 45, -9, 1 over 60 h
+    R inv_h;            // 1/h of this direction
+    R dc[3];            // half-node difference: 75/64, -25/384, 3/640 (FP64: over h)
+    R vc[3];            // 6th-order derivative: 45, -9, 1 over 60 h (FP64)
     SchemeParams<R> sp;
     int first;          // 1: write (first direction), 0: accumulate
     int visc;           // 1: add the viscous divergence term
@@ -136,15 +137,43 @@ __device__ __forceinline__ void to_conserved(const SweepArgs<R> &a, R r, R u, R 
     }
 }
 
-// r + c0 (p1 - m1) + c1 (p2 - m2) + c2 (p3 - m3): the half-node difference
-// (InviscousFlux.cpp:990-992) and the 6th-order derivative added to a
-// right-hand side, the differences first so that a uniform field leaves r as
-// it is
-template <typename R>
-__device__ __forceinline__ R diff3(const R *c, R p1, R m1, R p2, R m2, R p3, R m3, R r) {
-    r = fma(c[2], p3 - m3, r);
-    r = fma(c[1], p2 - m2, r);
-    return fma(c[0], p1 - m1, r);
+// The old right-hand side r minus the half-node difference of the faces l3 l2
+// l1 | r1 r2 r3 (InviscousFlux.cpp:990-992), and r plus the 6th-order
+// derivative of the nodes m3 .. p3 (ViscousFlux.cpp:15-29).  A uniform field
+// leaves r as it is.
+//
+// FP64: the differences first, one after another onto r, the spacing in the
+// coefficients (a third less error than the sum scaled and added once, and an
+// operation less).  FP32: that sum, which the mixed path has had from the
+// start; MDCD_HYBRID's detector turns any other rounding into another
+// trajectory.  Rounded as written, so that every kernel returns the same bits.
+__device__ __forceinline__ double add3(const double *c, double p1, double m1, double p2, double m2, double p3, double m3,
+                                       double r) {
+    r = __fma_rn(c[2], p3 - m3, r);
+    r = __fma_rn(c[1], p2 - m2, r);
+    return __fma_rn(c[0], p1 - m1, r);
+}
+__device__ __forceinline__ double face_diff(const double *dc, double, double l1, double r1, double l2, double r2, double l3,
+                                            double r3, double r) {
+    return add3(dc, l1, r1, l2, r2, l3, r3, r);
+}
+__device__ __forceinline__ double node_diff(const double *vc, double, double p1, double m1, double p2, double m2, double p3,
+                                            double m3, double r) {
+    return add3(vc, p1, m1, p2, m2, p3, m3, r);
+}
+__device__ __forceinline__ float face_diff(const float *dc, float inv_h, float l1, float r1, float l2, float r2, float l3,
+                                           float r3, float r) {
+    float t = __fmaf_rn(__fsub_rn(r1, l1), dc[0], __fmul_rn(__fsub_rn(r2, l2), dc[1]));
+    t = __fmaf_rn(__fsub_rn(r3, l3), dc[2], t);
+    return __fsub_rn(r, __fmul_rn(t, inv_h));
+}
+__device__ __forceinline__ float node_diff(const float *, float inv_60h, float p1, float m1, float p2, float m2, float p3,
+                                           float m3, float r) {
+    float t = __fmaf_rn(-9.f, p2, p3);
+    t = __fmaf_rn(45.f, p1, t);
+    t = __fmaf_rn(-45.f, m1, t);
+    t = __fmaf_rn(9.f, m2, t);
+    return __fadd_rn(r, __fmul_rn(__fsub_rn(t, m3), inv_60h));
 }
 
 // first derivative along the line, ViscousFlux.cpp:15-29 with the order of
@@ -350,22 +379,35 @@ sweep_kernel(SweepArgs<R> a) {
         // ---- face f = fc + slot (between cells f and f+1): cell positions slot .. slot+5
         const int f = fc + slot;
         if (line_ok && f < fe) {
-            // one copy of the side's code: the stencil read from the near or
-            // the far end, on the basis of cell f or f + 1
             R UL[5], UR[5];
-#pragma unroll 1
-            for (int side = 0; side < 2; ++side) {
-                const int sw = G::template idx<NU>(line, slot + 2 + side);
-                R w[5], o[5];
-#pragma unroll
-                for (int q = 0; q < 5; ++q) w[q] = sW[q * NL * NU + sw];
-                char_state<DIR, R, INTERP>(
-                    a.sp,
-                    [&](int q, int m) { return sU[q * NL * NU + G::template idx<NU>(line, slot + (side ? 5 - m : m))]; }, w, o);
+            if constexpr (sizeof(R) == 4) {
+                R st[5][6], wi[5], wi1[5];
+                const int s0 = G::template idx<NU>(line, slot + 2), s1 = G::template idx<NU>(line, slot + 3);
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
-                    if (side == 0) UL[q] = o[q];
-                    else UR[q] = o[q];
+#pragma unroll
+                    for (int m = 0; m < 6; ++m) st[q][m] = sU[q * NL * NU + G::template idx<NU>(line, slot + m)];
+                    wi[q] = sW[q * NL * NU + s0];
+                    wi1[q] = sW[q * NL * NU + s1];
+                }
+                char_pair<DIR, R, INTERP>(a.sp, st, wi, wi1, UL, UR);
+            } else {
+                // one copy of the side's code: the stencil read from the near or
+                // the far end, on the basis of cell f or f + 1
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side) {
+                    const int sw = G::template idx<NU>(line, slot + 2 + side);
+                    R w[5], o[5];
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) w[q] = sW[q * NL * NU + sw];
+                    char_state<DIR, R, INTERP>(
+                        a.sp,
+                        [&](int q, int m) { return sU[q * NL * NU + G::template idx<NU>(line, slot + (side ? 5 - m : m))]; }, w, o);
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) {
+                        if (side == 0) UL[q] = o[q];
+                        else UR[q] = o[q];
+                    }
                 }
             }
             R F[5];
@@ -394,14 +436,14 @@ sweep_kernel(SweepArgs<R> a) {
                 for (int q = 0; q < 5; ++q) {
                     const R *fq = sF + q * NL * NF;
                     auto F_ = [&](int m) { return fq[G::template idx<NF>(line, slot + m)]; };
-                    rq[q] = diff3(a.dc, F_(2), F_(3), F_(1), F_(4), F_(0), F_(5), rold[q]);
+                    rq[q] = face_diff(a.dc, a.inv_h, F_(2), F_(3), F_(1), F_(4), F_(0), F_(5), rold[q]);
                 }
                 if (visc) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const R *vq = sV + q * NL * NV;
                         auto V_ = [&](int off) { return vq[G::template idx<NV>(line, slot + 3 + off)]; };
-                        rq[q + 1] = diff3(a.vc, V_(1), V_(-1), V_(2), V_(-2), V_(3), V_(-3), rq[q + 1]);
+                        rq[q + 1] = node_diff(a.vc, a.dinv[2], V_(1), V_(-1), V_(2), V_(-2), V_(3), V_(-3), rq[q + 1]);
                     }
                 }
             } else {
@@ -418,7 +460,7 @@ sweep_kernel(SweepArgs<R> a) {
                         else if (ff > n + NG - 1) { if (a.outflow_hi) pm = pf_hi; else zero = true; }
                         fv[m] = zero ? R(0) : sF[q * NL * NF + G::template idx<NF>(line, pm)];
                     }
-                    rq[q] = diff3(a.dc, fv[2], fv[3], fv[1], fv[4], fv[0], fv[5], rold[q]);
+                    rq[q] = face_diff(a.dc, a.inv_h, fv[2], fv[3], fv[1], fv[4], fv[0], fv[5], rold[q]);
                 }
                 if (visc) {
                     const int o = visc_order(cu - NG, n, false);
@@ -588,6 +630,7 @@ cudaError_t sweep_z(const SweepArgs<float> &, cudaStream_t);
 // Characteristic reconstruction: the interpolation compiled in.
 template <int DIR, typename R>
 inline cudaError_t sweep_char(const SweepArgs<R> &a, cudaStream_t st) {
+    if constexpr (sizeof(R) == 4) return launch_sweep<DIR, R, RUNTIME>(a, st);
     if (a.sp.interp == I_WENO5) return launch_sweep<DIR, R, I_WENO5>(a, st);
     if (a.sp.interp == I_MDCD_LINEAR) return launch_sweep<DIR, R, I_MDCD_LINEAR>(a, st);
     return launch_sweep<DIR, R, I_MDCD_HYBRID>(a, st);

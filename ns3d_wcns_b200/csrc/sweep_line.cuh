@@ -282,7 +282,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
                     if (fc == fb && lane == 0) first |= march_doubt1(v) << q;
                 }
 #pragma unroll
-                for (int h = 0; h < 2; ++h) march_pair<T, INTERP>(m, v + h, UL[h][q], UR[h][q]);
+                for (int h = 0; h < 2; ++h) march_pair<T, INTERP, RS>(m, v + h, UL[h][q], UR[h][q]);
             }
             if constexpr (INTERP == I_MDCD_HYBRID) {
                 unsigned d0 = __shfl_up_sync(0xffffffffu, d2, 1);
@@ -352,7 +352,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
                     v[7] = fn[1][q];
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
-                        rq[h][q] = diff3(m.dc, v[3 + h], v[4 + h], v[2 + h], v[5 + h], v[1 + h], v[6 + h], ro[h][q]);
+                        rq[h][q] = face_diff(m.dc, m.inv_h, v[3 + h], v[4 + h], v[2 + h], v[5 + h], v[1 + h], v[6 + h], ro[h][q]);
                 }
                 if (visc) {
 #pragma unroll
@@ -366,7 +366,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
                         }
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
-                            rq[h][q + 1] = diff3(m.vc, v[4 + h], v[2 + h], v[5 + h], v[1 + h], v[6 + h], v[h], rq[h][q + 1]);
+                            rq[h][q + 1] = node_diff(m.vc, m.inv_60h, v[4 + h], v[2 + h], v[5 + h], v[1 + h], v[6 + h], v[h], rq[h][q + 1]);
                     }
                 }
             } else {
@@ -387,7 +387,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
                             else if (ff > n + NG - 1) { if (a.outflow_hi) p = p_hi; else zero = true; }
                             v[k] = zero ? march_const<T>(0.0) : sF[q * S::NF + p];
                         }
-                        rq[h][q] = diff3(m.dc, v[2], v[3], v[1], v[4], v[0], v[5], ro[h][q]);
+                        rq[h][q] = face_diff(m.dc, m.inv_h, v[2], v[3], v[1], v[4], v[0], v[5], ro[h][q]);
                     }
                     const int idx = cu + h - NG;
                     if (visc && idx >= 0 && idx < n) {
@@ -396,7 +396,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
                         for (int q = 0; q < 4; ++q) {
                             auto v = [&](int k) { return sV[q * S::NV + s0 + h + 3 + k]; };
                             if (o == 6)  // the lane's other cell is the one near the boundary
-                                rq[h][q + 1] = diff3(m.vc, v(1), v(-1), v(2), v(-2), v(3), v(-3), rq[h][q + 1]);
+                                rq[h][q + 1] = node_diff(m.vc, m.inv_60h, v(1), v(-1), v(2), v(-2), v(3), v(-3), rq[h][q + 1]);
                             else
                                 rq[h][q + 1] = march_add(rq[h][q + 1], march_visc_edge(T{}, v, o, a.dinv));
                         }
