@@ -21,6 +21,7 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PORT_LIB = os.path.join(HERE, "_build", "libns3d_oracle.so")
+PORT_LD_LIB = os.path.join(HERE, "_build", "libns3d_oracle_ld.so")
 REF_LIB = os.path.join(HERE, "_ref", "libns3d_ref.so")
 DROPIN_LIB = os.path.join(HERE, "_ref", "libns3d_dropin.so")
 DROPIN_LOOP_LIB = os.path.join(HERE, "_ref", "libns3d_dropin_loop.so")
@@ -157,6 +158,47 @@ class PortSolver(_Base):
     def residuals(self) -> np.ndarray:
         out = np.zeros(5)
         self.lib.orc_residuals(_ptr(out))
+        return out
+
+
+class ExtendedSolver:
+    """The C restatement in 80-bit arithmetic: right-hand sides to measure the rounding of 64-bit code against."""
+
+    class Config(C.Structure):
+        _fields_ = [(n, C.c_longdouble if t is C.c_double else t) for n, t in OrcConfig._fields_]
+
+    def __init__(self, P, G):
+        if not os.path.exists(PORT_LD_LIB):
+            build(ref=False)
+        self.lib = lib = C.CDLL(PORT_LD_LIB)
+        lib.orc_get.restype = C.c_long
+        lib.orc_get.argtypes = [C.c_char_p, C.c_void_p, C.c_long]
+        lib.orc_set_interior_prims.argtypes = [C.c_void_p] * 5
+        cfg = self.Config()
+        for n in ("gamma", "Pr", "Ma", "Re", "cfl", "dt_fixed", "mdcd_diss", "mdcd_disp"):
+            setattr(cfg, n, getattr(P, n))
+        cfg.sutherland_s, cfg.Lx, cfg.Ly, cfg.Lz = P.S_ref, G.Lx, G.Ly, G.Lz
+        cfg.nx, cfg.ny, cfg.nz = G.global_nx, G.global_ny, G.global_nz
+        cfg.interpolation, cfg.riemann, cfg.char_recon = int(P.interpolation), int(P.riemann_solver), int(P.char_recon)
+        for i, b in enumerate(P.bcs):
+            cfg.bc[i] = int(b)
+        if lib.orc_init(C.byref(cfg)) != 0:
+            raise ValueError("oracle rejected the configuration")
+        self.shape = (cfg.nz + 6, cfg.ny + 6, cfg.nx + 6)
+
+    def set_interior_prims(self, rho, u, v, w, p) -> None:
+        arrs = [np.ascontiguousarray(a, dtype=np.longdouble) for a in (rho, u, v, w, p)]
+        if self.lib.orc_set_interior_prims(*[a.ctypes.data for a in arrs]) != 0:
+            raise RuntimeError("set_interior_prims failed")
+
+    def compute_rhs(self) -> None:
+        self.lib.orc_compute_rhs()
+
+    def rhs(self) -> np.ndarray:
+        out = np.empty((5,) + self.shape, dtype=np.longdouble)
+        for a, n in zip(out, ("rhs_rho", "rhs_rhou", "rhs_rhov", "rhs_rhow", "rhs_E")):
+            if self.lib.orc_get(n.encode(), a.ctypes.data, a.size) < 0:
+                raise KeyError(n)
         return out
 
 
