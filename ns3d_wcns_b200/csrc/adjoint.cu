@@ -354,7 +354,7 @@ __global__ void ke_seed_kernel(AdjArgs a, double vol, double *const *Ub) {
     const long ncell = (long)I.nx * I.ny * I.nz;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ncell; t += (long)gridDim.x * blockDim.x) {
         int i, j, k;
-    I.split(t, i, j, k);
+        I.split(t, i, j, k);
         const long c = a.L.at(i + NG, j + NG, k + NG);
         const double u = a.W[1][c], v = a.W[2][c], w = a.W[3][c];
         // J = sum 0.5 |m|^2 / rho * vol (postprocess.cpp:119-122)
@@ -370,7 +370,7 @@ __global__ void velocity_grad_kernel(AdjArgs a, const double *const *Ub, double 
     const long ncell = (long)I.nx * I.ny * I.nz;
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ncell; t += (long)gridDim.x * blockDim.x) {
         int i, j, k;
-    I.split(t, i, j, k);
+        I.split(t, i, j, k);
         const long c = a.L.at(i + NG, j + NG, k + NG);
         const double rho = a.W[0][c];
         for (int q = 0; q < 3; ++q) gvel[q][t] = rho * Ub[1 + q][t] + rho * a.W[1 + q][c] * Ub[4][t];

@@ -44,9 +44,9 @@ NS3D_HD void weno5_vjp(const R *f, R qb, R *fb) {
     R A = a0 + a1 + a2;
     const R iA = rcp_(A);
     R w0 = a0 * iA, w1 = a1 * iA, w2 = a2 * iA;  // normalised weights
-    R p0 = (R(3) * f[0] - R(10) * f[1] + R(15) * f[2]) * R(0.125);
-    R p1 = (-f[1] + R(6) * f[2] + R(3) * f[3]) * R(0.125);
-    R p2 = (R(3) * f[2] + R(6) * f[3] - f[4]) * R(0.125);
+    // the candidates less f[2] (only p_k - q is needed)
+    R d1 = f[1] - f[0], d2 = f[2] - f[1], d3 = f[3] - f[2], d4 = f[4] - f[3];
+    R p0 = (R(7) * d2 - R(3) * d1) * R(0.125), p1 = (d2 + R(3) * d3) * R(0.125), p2 = (R(5) * d3 - d4) * R(0.125);
     R q = w0 * p0 + w1 * p1 + w2 * p2;
     // candidates
     R pb0 = w0 * qb, pb1 = w1 * qb, pb2 = w2 * qb;
@@ -79,8 +79,9 @@ NS3D_HD void mdcd_weno_vjp(const R *f, const R *hd, R qb, R *fb) {
     const R t2 = f[2] - R(2) * f[3] + f[4], u2 = R(3) * f[2] - R(4) * f[3] + f[4];
     const R be[4] = {c13 * (t0 * t0) + R(0.25) * (u0 * u0), c13 * (t1 * t1) + R(0.25) * (u1 * u1),
                      c13 * (t2 * t2) + R(0.25) * (u2 * u2), mdcd_beta3(f[0], f[1], f[2], f[3], f[4], f[5])};
-    const R qk[4] = {R(3) * f[0] - R(10) * f[1] + R(15) * f[2], -f[1] + R(6) * f[2] + R(3) * f[3],
-                     R(3) * f[2] + R(6) * f[3] - f[4], R(15) * f[3] - R(10) * f[4] + R(3) * f[5]};
+    // the candidates times eight, less 8 f[2] (only q_k / 8 - q is needed)
+    const R d1 = f[1] - f[0], d2 = f[2] - f[1], d3 = f[3] - f[2], d4 = f[4] - f[3], d5 = f[5] - f[4];
+    const R qk[4] = {R(7) * d2 - R(3) * d1, d2 + R(3) * d3, R(5) * d3 - d4, R(8) * d3 - R(7) * d4 + R(3) * d5};
     const R D = be[3] - (be[0] + R(4) * be[1] + be[2]) * R(1.0 / 6.0);
     const R tau = fabs(D);
     R g[4], al[4], ib[4], A = R(0), Q = R(0);
@@ -381,7 +382,7 @@ NS3D_HD void rusanov_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *
         ULb[n] += R(0.5) * smax * Fb[n];
     }
     R uLb = 0, vLb = 0, wLb = 0, pLb = 0, ELb = 0, rLb = 0, uRb = 0, vRb = 0, wRb = 0, pRb = 0, ERb = 0, rRb = 0;
-    // smax = |un| + sqrt_(g p / r)
+    // smax = |un| + sqrt(g p / r)
     if (left) {
         R unb = (unL >= R(0) ? R(1) : R(-1)) * smaxb;
         if (DIR == 0) uLb += unb; else if (DIR == 1) vLb += unb; else wLb += unb;
@@ -575,7 +576,7 @@ NS3D_HD void hllc_vjp(const R *UL, const R *UR, R g, const R *Fb, R *ULb, R *URb
     R aLb = 0, aRb = 0;
     if (sl_right) { unRb += SLb; aRb -= SLb; } else { unLb += SLb; aLb -= SLb; }
     if (sr_right) { unRb += SRb; aRb += SRb; } else { unLb += SRb; aLb += SRb; }
-    // a = sqrt_(g p ir)
+    // a = sqrt(g p ir)
     if (aL > R(0)) { const R xb = quot_(aLb, R(2) * aL); pLb += xb * g * L.ir; irLb += xb * g * L.p; }
     if (aR > R(0)) { const R xb = quot_(aRb, R(2) * aR); pRb += xb * g * Rs.ir; irRb += xb * g * Rs.p; }
     if (DIR == 0) { uLb += unLb; uRb += unRb; }
@@ -666,10 +667,9 @@ NS3D_HD void visc_flux_all(R mu0, R S, R cpr, const R *x, const R g[4][3], R V[9
 template <typename R>
 NS3D_HD void visc_flux_vjp(R mu0, R S, R cpr, const R *x, const R g[4][3], const R *Vb, R *xb, R gb[4][3]) {
     const R T = x[3];
-    const R sq = sqrt_(T);
+    const R sq = sqrt(T);
     const R num = mu0 * (T * sq) * (R(1) + S);
-    const R its = rcp_(T + S);
-    const R mu = num * its;
+    const R mu = num / (T + S);
     const R div = g[0][0] + g[1][1] + g[2][2];
     const R txx = R(2) * mu * g[0][0] - R(2.0 / 3.0) * mu * div;
     const R tyy = R(2) * mu * g[1][1] - R(2.0 / 3.0) * mu * div;
@@ -696,7 +696,7 @@ NS3D_HD void visc_flux_vjp(R mu0, R S, R cpr, const R *x, const R g[4][3], const
     gb[0][2] += mu * txzb; gb[2][0] += mu * txzb;
     gb[1][2] += mu * tyzb; gb[2][1] += mu * tyzb;
     // mu = mu0 T^1.5 (1+S)/(T+S)
-    const R dmu = mu0 * (R(1) + S) * (R(1.5) * sq * (T + S) - T * sq) * its * its;
+    const R dmu = mu0 * (R(1) + S) * (R(1.5) * sq * (T + S) - T * sq) / ((T + S) * (T + S));
     xb[3] += mub * dmu;
     (void)num;
 }
