@@ -260,36 +260,35 @@ NS3D_HD bool mdcd_smooth(R fm2, R fm1, R f0, R fp1, R fp2) {
 }
 
 // The non-linear branch: 4-stencil WENO with weights d_k (20 + tau6/(beta_k +
-// 1e-40))^2 (interpolation.cpp:170-208), from the smoothness indicators and
-// the candidates (times eight).  The weights span far more than the FP32 range:
-// FP32 inputs quantise a smooth stencil to beta == 0 exactly, and (tau6 *
-// 1e40)^2 overflows to inf (inf/inf = NaN).  So the FP32 build forms the
-// weights and the normalisation in FP64, like the reference; this branch is
-// the rare one (most faces take the linear scheme).
+// 1e-40))^2 (interpolation.cpp:170-208), here from the smoothness indicators.
+// The weights span far more than the FP32 range: FP32 inputs quantise a
+// smooth stencil to beta == 0 exactly, and (tau6 * 1e40)^2 overflows to inf
+// (inf/inf = NaN).  So the FP32 build forms the weights and the normalisation
+// in FP64, like the reference; this branch is the rare one (most faces take
+// the linear scheme).
 template <typename R>
-NS3D_HD R mdcd_weno_weigh(const R *hd, R be0, R be1, R be2, R be3, R q0, R q1, R q2, R q3) {
-    using Wt = double;
-    const Wt es = 1e-40;
-    Wt tau6 = fabs((Wt)be3 - ((Wt)be0 + Wt(4) * (Wt)be1 + (Wt)be2) / Wt(6));
-    Wt g0 = Wt(20) + div_(tau6, (Wt)be0 + es);
-    Wt g1 = Wt(20) + div_(tau6, (Wt)be1 + es);
-    Wt g2 = Wt(20) + div_(tau6, (Wt)be2 + es);
-    Wt g3 = Wt(20) + div_(tau6, (Wt)be3 + es);
-    Wt al0 = (Wt)hd[0] * (g0 * g0), al1 = (Wt)hd[1] * (g1 * g1), al2 = (Wt)hd[2] * (g2 * g2),
-       al3 = (Wt)hd[3] * (g3 * g3);
-    return (R)div_(al0 * (Wt)q0 + al1 * (Wt)q1 + al2 * (Wt)q2 + al3 * (Wt)q3, Wt(8) * (al0 + al1 + al2 + al3));
+NS3D_HD void mdcd_weno_weights(const R *hd, R be0, R be1, R be2, R be3, double al[4]) {
+    const double tau6 = fabs((double)be3 - ((double)be0 + 4.0 * (double)be1 + (double)be2) / 6.0);
+    const R be[4] = {be0, be1, be2, be3};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        // FP32 keeps the quotients' rounding: a unit of FP64 decides a unit of FP32 now and then
+        const double b = (double)be[k] + 1e-40, g = 20.0 + (sizeof(R) == 4 ? div_(tau6, b) : quot_(tau6, b));
+        al[k] = (double)hd[k] * (g * g);
+    }
 }
+// FP64, through the first differences (weno5_pair): the candidates less the
+// central value, which the quotient is added to, so that it need not be
+// rounded as the quotient of the values must
 NS3D_HD double mdcd_weno_branch(const double *hd, double f0, double f1, double f2, double f3, double f4, double f5) {
-    const double c13 = 13.0 / 12.0;
-    double t, u;
-    t = f0 - 2.0 * f1 + f2; u = f0 - 4.0 * f1 + 3.0 * f2;
-    const double be0 = c13 * (t * t) + 0.25 * (u * u);
-    t = f1 - 2.0 * f2 + f3; u = f1 - f3;
-    const double be1 = c13 * (t * t) + 0.25 * (u * u);
-    t = f2 - 2.0 * f3 + f4; u = 3.0 * f2 - 4.0 * f3 + f4;
-    const double be2 = c13 * (t * t) + 0.25 * (u * u);
-    return mdcd_weno_weigh(hd, be0, be1, be2, mdcd_beta3(f0, f1, f2, f3, f4, f5), 3.0 * f0 - 10.0 * f1 + 15.0 * f2,
-                           -f1 + 6.0 * f2 + 3.0 * f3, 3.0 * f2 + 6.0 * f3 - f4, 15.0 * f3 - 10.0 * f4 + 3.0 * f5);
+    const double d1 = f1 - f0, d2 = f2 - f1, d3 = f3 - f2, d4 = f4 - f3, d5 = f5 - f4;
+    auto ind = [](double t, double u) { return 13.0 / 12.0 * (t * t) + 0.25 * (u * u); };
+    double al[4];
+    mdcd_weno_weights(hd, ind(d2 - d1, 3.0 * d2 - d1), ind(d3 - d2, d2 + d3), ind(d4 - d3, 3.0 * d3 - d4),
+                      mdcd_beta3(f0, f1, f2, f3, f4, f5), al);
+    const double n = al[0] * (7.0 * d2 - 3.0 * d1) + al[1] * (d2 + 3.0 * d3) + al[2] * (5.0 * d3 - d4) +
+                     al[3] * (8.0 * d3 - 7.0 * d4 + 3.0 * d5);
+    return f2 + quot_(n, 8.0 * (al[0] + al[1] + al[2] + al[3]));
 }
 // FP32, rounded as written: the hybrid scheme turns another placement of the
 // fused operations into another trajectory, so it is the same whichever
@@ -306,7 +305,10 @@ NS3D_HD float mdcd_weno_branch(const float *hd, float f0, float f1, float f2, fl
     const float q1 = ch ? fma_rn(3.f, f3, fma_rn(6.f, f2, -f1)) : add_rn(mul_rn(3.f, f3), fma_rn(6.f, f2, -f1));
     const float q2 = add_rn(fma_rn(6.f, f3, e2), -f4);
     const float q3 = fma_rn(3.f, f5, fma_rn(15.f, f3, mul_rn(-10.f, f4)));
-    return mdcd_weno_weigh(hd, be0, be1, be2, mdcd_beta3(f0, f1, f2, f3, f4, f5), q0, q1, q2, q3);
+    double al[4];
+    mdcd_weno_weights(hd, be0, be1, be2, mdcd_beta3(f0, f1, f2, f3, f4, f5), al);
+    return (float)div_(al[0] * (double)q0 + al[1] * (double)q1 + al[2] * (double)q2 + al[3] * (double)q3,
+                       8.0 * (al[0] + al[1] + al[2] + al[3]));
 }
 
 template <typename R>
