@@ -63,8 +63,10 @@ struct Phys {
 // IEEE operations' seven to ten with their range checks and slow paths; the
 // sweeps hold five to thirteen of them per face (256^3, x-sweep: 0.900 -> 0.826 ms
 // with MDCD_HYBRID + HLLC, 1.338 -> 1.207 with WENO5 + Roe).  Range: x normal with a
-// normal reciprocal (an infinite or zero x gives NaN); sqrt_fp64 keeps
-// sqrt(0) = 0 and NaN for negative arguments.
+// normal reciprocal (zero, subnormal and infinite x give NaN, x above 2^1022
+// gives 0); sqrt_fp64 returns 0 for zero and subnormal arguments and NaN for
+// negative and infinite ones.  In a face's flux these stand for states that the
+// scheme has no finite flux for; the conversions below look for them.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double rcp_fp64(double x) {
     double y;
@@ -77,27 +79,45 @@ __device__ __forceinline__ double sqrt_fp64(double t) {
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
     const double a = t * y, r = __fma_rn(-a, y, 1.0);
     const double s = __fma_rn(a * r, __fma_rn(r, 0.375, 0.5), a);
-    return t == 0.0 ? 0.0 : s;
+    return fabs(t) < 2.2250738585072014e-308 ? 0.0 : s;
 }
-// a / b from y = rcp_fp64(b), correctly rounded (P. W. Markstein, IBM J. Res.
-// Dev. 34 (1990) 111: the residual of the first quotient is exact in one FMA,
-// and the corrected one rounds to the IEEE quotient): one reciprocal serves
-// several quotients of the same divisor.
+// a / b from y = rcp_fp64(b): one reciprocal serves several quotients of the
+// same divisor.  The residual of the first quotient is exact in one FMA, and
+// the corrected quotient is off by 2^-103 of itself before it is rounded
+// (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111, whose theorem asks for a
+// correctly rounded y): the IEEE quotient, but for one that close to a tie.
+// Zeros keep their sign for b > 0.  Not for what rcp_fp64 excludes, quotients
+// that overflow (NaN), and numerators below 2^-960 (the residual underflows).
 __device__ __forceinline__ double div_fp64(double a, double b, double y) {
     const double q = a * y;
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(-__fma_rn(q, b, -a), y, q);
 }
+
+// Neither infinite nor NaN.  An integer test: the FP64 pipe is what the sweeps wait for.
+__device__ __forceinline__ bool finite_fp64(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+// The IEEE quotient out of line: for branches that no ordinary state takes, in
+// kernels that fill the instruction cache.
+static __device__ __noinline__ double div_ieee(double a, double b) { return __ddiv_rn(a, b); }
 
 // ---------------------------------------------------------------------------
 // Conversions with the reference's rounding.  The reference compiles without
 // fused multiply-add, so these use the _rn intrinsics (no contraction) and
-// correctly rounded quotients (div_fp64): for identical finite inputs they
-// return identical bits.
+// div_fp64.  Where the result is not finite the IEEE operations decide (a branch
+// that no ordinary state takes), so zero, subnormal and infinite divisors and
+// overflows give what they give there.  ENDS: 1 with that branch, 0 without it
+// (the stencils of the sweeps, which have no finite flux for such a state, and
+// fused_stage_cell, which asks once for all its conversions), 2 the IEEE
+// operations.  A branch in each cost the 192^3 x- and z-sweeps 1.5 and 3 %.
 // ---------------------------------------------------------------------------
+template <int ENDS>
+__device__ __forceinline__ double div_ends(double a, double b, double y) {
+    return ENDS == 2 ? div_ieee(a, b) : div_fp64(a, b, y);
+}
 
 // Field3D::primitiveToConserved, field_structures.h:468-488.
-__device__ __forceinline__ void p2c_exact(double r, double u, double v, double w, double p,
-                                          double gamma, double U[5]) {
+template <int ENDS = 1>
+__device__ __forceinline__ void p2c_exact(double r, double u, double v, double w, double p, double gamma,
+                                          double U[5]) {
     double rr = r <= 0.0 ? 1e-12 : r;
     U[0] = rr;
     U[1] = __dmul_rn(rr, u);
@@ -105,25 +125,33 @@ __device__ __forceinline__ void p2c_exact(double r, double u, double v, double w
     U[3] = __dmul_rn(rr, w);
     double kin = __dmul_rn(0.5, __dadd_rn(__dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v)), __dmul_rn(w, w)));
     const double d = __dmul_rn(gamma - 1.0, rr);
-    double e = div_fp64(p, d, rcp_fp64(d));
+    double e = div_ends<ENDS>(p, d, rcp_fp64(d));
     U[4] = __dmul_rn(rr, __dadd_rn(e, kin));
+    if (ENDS == 1 && __builtin_expect(!finite_fp64(U[4]), 0)) U[4] = __dmul_rn(rr, __dadd_rn(div_ieee(p, d), kin));
 }
 
 // Field3D::conservedToPrimitive, field_structures.h:444-465 (density clamp).
+template <int ENDS = 1>
 __device__ __forceinline__ void c2p_exact(const double U[5], double gamma, double W[5]) {
     double rr = U[0] <= 0.0 ? 1e-12 : U[0];
     const double ir = rcp_fp64(rr);
-    double u = div_fp64(U[1], rr, ir), v = div_fp64(U[2], rr, ir), w = div_fp64(U[3], rr, ir);
+    double u = div_ends<ENDS>(U[1], rr, ir), v = div_ends<ENDS>(U[2], rr, ir), w = div_ends<ENDS>(U[3], rr, ir);
     double kin = __dmul_rn(0.5, __dadd_rn(__dadd_rn(__dmul_rn(u, u), __dmul_rn(v, v)), __dmul_rn(w, w)));
-    double e = __dsub_rn(div_fp64(U[4], rr, ir), kin);
+    double e = __dsub_rn(div_ends<ENDS>(U[4], rr, ir), kin);
     W[0] = rr; W[1] = u; W[2] = v; W[3] = w;
     W[4] = __dmul_rn(__dmul_rn(gamma - 1.0, rr), e);
+    if constexpr (ENDS == 1) {
+        if (__builtin_expect(!finite_fp64(W[4]), 0)) c2p_exact<2>(U, gamma, W);
+    }
 }
 
 // T = p / (rho Rgas), field_structures.h:486
+template <int ENDS = 1>
 __device__ __forceinline__ double temperature_exact(const double W[5], double Rgas) {
     const double d = __dmul_rn(W[0], Rgas);
-    return div_fp64(W[4], d, rcp_fp64(d));
+    double T = div_ends<ENDS>(W[4], d, rcp_fp64(d));
+    if (ENDS == 1 && __builtin_expect(!finite_fp64(T), 0)) T = div_ieee(W[4], d);
+    return T;
 }
 
 // Mixed path: conserved -> primitive in FP64 with one reciprocal (the mixed

@@ -55,7 +55,7 @@ struct MarchArgs {
 // ---------------------------------------------------------------- one value
 
 __device__ __forceinline__ void march_cons(double gamma, const double *w, double *U) {
-    p2c_exact(w[0], w[1], w[2], w[3], w[4], gamma, U);
+    p2c_exact<0>(w[0], w[1], w[2], w[3], w[4], gamma, U);
 }
 __device__ __forceinline__ void march_cons(float gamma, const float *w, float *U) {
     p2c_f(w[0], w[1], w[2], w[3], w[4], gamma - 1.f, U);

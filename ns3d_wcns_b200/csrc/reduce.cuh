@@ -181,12 +181,14 @@ __device__ __forceinline__ double cfl_bound(const double U[5], double gamma, dou
 }
 
 // The wave speed |u| + a of cfl_bound (cfl_bound = dx / cfl_speed, same bits).
+// A quotient that overflows stays infinite, so that the time step is zero.
 __device__ __forceinline__ double cfl_speed(const double U[5], double gamma) {
     double rho = U[0];
     const double ir = rcp_fp64(rho);
-    double u = div_fp64(U[1], rho, ir);
+    auto div = [&](double a) { return fabs(a * ir) <= 1.7976931348623157e308 ? div_fp64(a, rho, ir) : a * ir; };
+    double u = div(U[1]);
     double p = __dmul_rn(gamma - 1., __dsub_rn(U[4], __dmul_rn(__dmul_rn(__dmul_rn(0.5, rho), u), u)));
-    double a = sqrt(div_fp64(__dmul_rn(gamma, p), rho, ir));
+    double a = sqrt(div(__dmul_rn(gamma, p)));
     return __dadd_rn(fabs(u), a);
 }
 

@@ -31,6 +31,8 @@
 // x-lines and the warps march.
 #pragma once
 
+#include <type_traits>
+
 #include "bc.cuh"
 #include "common.cuh"
 #include "reduce.cuh"
@@ -131,7 +133,7 @@ constexpr size_t sweep_smem_bytes() {
 template <typename R>
 __device__ __forceinline__ void to_conserved(const SweepArgs<R> &a, R r, R u, R v, R w, R p, R *U) {
     if constexpr (sizeof(R) == 8) {
-        p2c_exact(r, u, v, w, p, a.sp.gamma, U);
+        p2c_exact<0>(r, u, v, w, p, a.sp.gamma, U);
     } else {
         p2c_f(r, u, v, w, p, a.sp.gamma - 1.f, U);
     }
@@ -197,22 +199,29 @@ __device__ __forceinline__ R dstencil_inv(F f, int order, const R *dinv) {
 __device__ __forceinline__ void fused_stage_cell(const FusedStage &f, double dt, long c, const double *r,
                                                  const double *Ucur, const double *w0, double &smax, double &ke,
                                                  double &kc) {
-    double U0[5], U[5], W[5];
-    if (f.stage == 1) {
+    double W[5], T;
+    auto convert = [&](auto ends) {
+        constexpr int E = decltype(ends)::value;
+        double U0[5], U[5];
+        if (f.stage == 1) {
 #pragma unroll
-        for (int q = 0; q < 5; ++q) U0[q] = Ucur[q];
-    } else {
-        p2c_exact(w0[0], w0[1], w0[2], w0[3], w0[4], f.gamma, U0);
-    }
+            for (int q = 0; q < 5; ++q) U0[q] = Ucur[q];
+        } else {
+            p2c_exact<E>(w0[0], w0[1], w0[2], w0[3], w0[4], f.gamma, U0);
+        }
 #pragma unroll
-    for (int q = 0; q < 5; ++q) U[q] = rk_combine(f.stage, U0[q], f.stage == 1 ? U0[q] : Ucur[q], r[q], dt);
-    c2p_exact(U, f.gamma, W);
+        for (int q = 0; q < 5; ++q) U[q] = rk_combine(f.stage, U0[q], f.stage == 1 ? U0[q] : Ucur[q], r[q], dt);
+        c2p_exact<E>(U, f.gamma, W);
+        T = temperature_exact<E>(W, f.Rgas);
+    };
+    convert(std::integral_constant<int, 0>{});
+    if (__builtin_expect(!finite_fp64(W[4]) || !finite_fp64(T), 0)) convert(std::integral_constant<int, 2>{});
 #pragma unroll
     for (int q = 0; q < 5; ++q) f.Wout[q][c] = W[q];
-    f.Tout[c] = temperature_exact(W, f.Rgas);
+    f.Tout[c] = T;
     if (f.stage == 3) {
         double Un[5];
-        p2c_exact(W[0], W[1], W[2], W[3], W[4], f.gamma, Un);
+        p2c_exact<0>(W[0], W[1], W[2], W[3], W[4], f.gamma, Un);
         smax = fmax(smax, cfl_speed(Un, f.gamma));  // largest wave speed: one division per block
         // a thread adds one cell per chunk along its line: compensated
         // (Kahan) summation keeps its partial exact to rounding
