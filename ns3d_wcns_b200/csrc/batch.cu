@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -829,6 +830,7 @@ struct ns3d_batch {
     SchemeParams<double> sp;
     double *pinned = nullptr;    // host side of ns3d_batch_download, allocated by its first call
     size_t pinned_n = 0;
+    std::mutex download;         // several threads may download problems of one batch
     std::string err;
     std::vector<double> init;    // copy of the uploaded pool (for re-runs after tuning)
 };
@@ -1343,6 +1345,7 @@ int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]) {
     // batch: a pitched copy per field into pageable memory took 1.4 ms for a
     // 750 x 4 x 4 tube, this 1.1 (the rest is the first touch of new host pages)
     const size_t n = (size_t)L.sx * L.sy * L.sz;
+    const std::lock_guard<std::mutex> one(b->download);
     if (!b->pinned) {
         size_t most = 0;
         for (const Inst &J : b->inst) most = std::max(most, (size_t)J.L.sx * J.L.sy * J.L.sz);
