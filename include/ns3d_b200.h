@@ -285,7 +285,10 @@ int ns3d_batch_autotune(ns3d_batch *b, int trial_steps, int config_out[3]);
 int ns3d_batch_set_config(ns3d_batch *b, int cluster, int threads, int ctas_per_sm);
 /* final time, steps taken, status (0 reached t_end, 1 dt <= 1e-12, 2 max_steps) */
 int ns3d_batch_query(ns3d_batch *b, int problem, double *time, int *steps, int *status);
-/* primitive Field3D arrays (rho,u,v,w,p; sx*sy*sz each) of problem i */
+/* primitive Field3D arrays (rho,u,v,w,p; sx*sy*sz each) of problem i.  The
+ * first call allocates a pinned host buffer of the largest problem's size, 64
+ * MB at most, which stays with the batch until ns3d_batch_destroy; where it
+ * cannot be had the copies go without. */
 int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]);
 
 /* ------------------------------------------------- verification helpers
@@ -325,6 +328,9 @@ int ns3d_debug_mdcd_detector(int device, long n, const double *stencils, int *sm
  * entry points do when one of their TMA waits runs out.  No counterpart in
  * the reference; for tests of the failure path. */
 int ns3d_debug_wait_timeout(int device, unsigned polls, int *code_out);
+
+/* The batch as if no pinned host memory could be had (ns3d_batch_download). */
+int ns3d_debug_batch_unpinned(ns3d_batch *b);
 
 /* ------------------------------------------------ z-slab decomposition
  * A handle holding one rank's z-slab of a domain split along z over several

@@ -830,6 +830,7 @@ struct ns3d_batch {
     SchemeParams<double> sp;
     double *pinned = nullptr;    // host side of ns3d_batch_download, allocated by its first call
     size_t pinned_n = 0;
+    bool unpinned = false;       // there was none to be had
     std::mutex download;         // several threads may download problems of one batch
     std::string err;
     std::vector<double> init;    // copy of the uploaded pool (for re-runs after tuning)
@@ -1346,19 +1347,25 @@ int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]) {
     // 750 x 4 x 4 tube, this 1.1 (the rest is the first touch of new host pages)
     const size_t n = (size_t)L.sx * L.sy * L.sz;
     const std::lock_guard<std::mutex> one(b->download);
-    if (!b->pinned) {
+    if (!b->pinned && !b->unpinned) {
         size_t most = 0;
         for (const Inst &J : b->inst) most = std::max(most, (size_t)J.L.sx * J.L.sy * J.L.sz);
         b->pinned_n = std::min(5 * most, (size_t)8 << 20);  // doubles, 64 MB at most
         if (cudaHostAlloc((void **)&b->pinned, b->pinned_n * 8, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
             b->pinned = nullptr;
-            return bfail(b, NS3D_ERR_OOM, "pinned download buffer");
+            b->unpinned = true;
         }
     }
     double *stg = b->pool + I.base + 15L * L.plane;
     batch_pack_kernel<<<dim3((L.sx + 127) / 128, L.sy, L.sz), 128, 0, b->stream>>>(b->pool + I.base, stg, L, b->d_state + s);
     BCK(b, cudaGetLastError(), "pack");
+    if (!b->pinned) {
+        for (int q = 0; q < 5; ++q)
+            BCK(b, cudaMemcpyAsync(out[q], stg + q * n, n * 8, cudaMemcpyDeviceToHost, b->stream), "download");
+        BCK(b, cudaStreamSynchronize(b->stream), "synchronize");
+        return NS3D_OK;
+    }
     for (size_t at = 0; at < 5 * n; at += b->pinned_n) {
         const size_t end = std::min(5 * n, at + b->pinned_n);
         BCK(b, cudaMemcpyAsync(b->pinned, stg + at, (end - at) * 8, cudaMemcpyDeviceToHost, b->stream), "download");
@@ -1369,6 +1376,15 @@ int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]) {
             c = stop;
         }
     }
+    return NS3D_OK;
+}
+
+int ns3d_debug_batch_unpinned(ns3d_batch *b) {
+    if (!b) return NS3D_ERR_INVALID_ARG;
+    const std::lock_guard<std::mutex> one(b->download);
+    cudaFreeHost(b->pinned);
+    b->pinned = nullptr;
+    b->unpinned = true;
     return NS3D_OK;
 }
 

@@ -1,4 +1,4 @@
-"""Several threads downloading from one batch."""
+"""Batch downloads: several threads at once, and without pinned memory."""
 import math
 from concurrent.futures import ThreadPoolExecutor
 
@@ -31,3 +31,11 @@ def test_threads_download(gpu_lib):
         for _ in range(4):
             for a, w in zip(pool.map(b.primitives, range(len(sizes))), want):
                 assert np.array_equal(a, w)
+
+
+def test_unpinned_download(gpu_lib):
+    with batch([48, 200, 31]) as b:
+        want = [b.primitives(i) for i in range(3)]
+        assert b.lib.ns3d_debug_batch_unpinned(b.h) == 0
+        for i in range(3):
+            assert np.array_equal(b.primitives(i), want[i])
