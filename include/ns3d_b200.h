@@ -251,6 +251,15 @@ int ns3d_vjp_rk3_step(ns3d_handle *h, double dt, const double *const ubar_next[5
 int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int checkpoint_every, double *J,
                                 double *const grad[3], double stats[4]);
 
+/* Device memory of the calls above: the first one allocates 69 interior-sized
+ * arrays, which stay with the handle; ns3d_vjp_rk3_step and
+ * ns3d_adjoint_kinetic_energy also keep their stage states and checkpoints
+ * (15 padded arrays; 5 per checkpoint and 15 per step of a segment) between
+ * calls when these take at most 2 GiB, else they are freed before the call
+ * returns.  ns3d_destroy frees all of it, this call at once; the next adjoint
+ * call allocates again. */
+int ns3d_release_scratch(ns3d_handle *h);
+
 /* ------------------------------------------------------------- batched
  * Many independent small problems of uneven size (e.g. quasi-1D shock tubes,
  * Nx x 4 x 4) in one persistent launch: each is a full time_advance run
@@ -287,9 +296,10 @@ int ns3d_batch_set_config(ns3d_batch *b, int cluster, int threads, int ctas_per_
 int ns3d_batch_query(ns3d_batch *b, int problem, double *time, int *steps, int *status);
 /* primitive Field3D arrays (rho,u,v,w,p; sx*sy*sz each) of problem i.  The
  * first call allocates a pinned host buffer of the largest problem's size, 64
- * MB at most, which stays with the batch until ns3d_batch_destroy; where it
- * cannot be had the copies go without. */
+ * MB at most, which stays with the batch until ns3d_batch_destroy or
+ * ns3d_batch_release_scratch; where it cannot be had the copies go without. */
 int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]);
+int ns3d_batch_release_scratch(ns3d_batch *b);
 
 /* ------------------------------------------------- verification helpers
  * Host evaluation (no device needed) of the code the adjoint kernels run,

@@ -31,7 +31,8 @@ EXPORTS = [
     "ns3d_debug_mdcd_detector", "ns3d_vjp_rhs", "ns3d_vjp_rk3_step",
     "ns3d_adjoint_kinetic_energy", "ns3d_batch_create", "ns3d_batch_destroy", "ns3d_batch_last_error",
     "ns3d_batch_set_interior_primitives", "ns3d_batch_run", "ns3d_batch_autotune", "ns3d_batch_set_config",
-    "ns3d_batch_query", "ns3d_batch_download", "ns3d_debug_batch_unpinned",
+    "ns3d_batch_query", "ns3d_batch_download", "ns3d_release_scratch", "ns3d_batch_release_scratch",
+    "ns3d_debug_batch_unpinned",
 ]
 
 
@@ -110,6 +111,8 @@ def load() -> C.CDLL:
     lib.ns3d_batch_set_config.argtypes = [h, C.c_int, C.c_int, C.c_int]
     lib.ns3d_batch_query.argtypes = [h, C.c_int, dp, C.POINTER(C.c_int), C.POINTER(C.c_int)]
     lib.ns3d_batch_download.argtypes = [h, C.c_int, C.POINTER(dp)]
+    lib.ns3d_release_scratch.argtypes = [h]
+    lib.ns3d_batch_release_scratch.argtypes = [h]
     lib.ns3d_debug_batch_unpinned.argtypes = [h]
     lib.ns3d_debug_face_vjp.argtypes = [C.c_int, C.c_int, C.c_int, C.c_double, dp, dp, dp, dp, dp]
     lib.ns3d_debug_visc_vjp.argtypes = [C.c_double, C.c_double, C.c_double, dp, dp, dp, dp, dp, dp]

@@ -80,6 +80,10 @@ class Batch:
         self._check(self.lib.ns3d_batch_query(self.h, i, C.byref(t), C.byref(s), C.byref(st)))
         return t.value, s.value, st.value
 
+    def release_scratch(self) -> None:
+        """Gives back the pinned host memory that ``primitives`` keeps with the batch."""
+        self._check(self.lib.ns3d_batch_release_scratch(self.h))
+
     def primitives(self, i: int) -> np.ndarray:
         g = self.grids[i]
         shp = (g.global_nz + 6, g.global_ny + 6, g.global_nx + 6)

@@ -1379,13 +1379,19 @@ int ns3d_batch_download(ns3d_batch *b, int problem, double *const out[5]) {
     return NS3D_OK;
 }
 
-int ns3d_debug_batch_unpinned(ns3d_batch *b) {
+int ns3d_batch_release_scratch(ns3d_batch *b) {
     if (!b) return NS3D_ERR_INVALID_ARG;
     const std::lock_guard<std::mutex> one(b->download);
     cudaFreeHost(b->pinned);
     b->pinned = nullptr;
-    b->unpinned = true;
+    b->unpinned = false;
     return NS3D_OK;
+}
+
+int ns3d_debug_batch_unpinned(ns3d_batch *b) {
+    const int r = ns3d_batch_release_scratch(b);
+    if (b) b->unpinned = true;
+    return r;
 }
 
 }  // extern "C"

@@ -1988,6 +1988,18 @@ int ns3d_vjp_rk3_step(ns3d_handle *h, double dt, const double *const ubar_next[5
     return r;
 }
 
+int ns3d_release_scratch(ns3d_handle *h) {
+    if (!h) return NS3D_ERR_INVALID_ARG;
+    int r = set_device(h); if (r) return r;
+    CK(h, cudaStreamSynchronize(h->stream), "synchronize");
+    cudaFree(h->adj_pool);
+    cudaFree(h->adj_store);
+    h->adj_pool = nullptr;
+    h->adj_store = nullptr;
+    h->adj_bytes = h->adj_store_bytes = 0;
+    return NS3D_OK;
+}
+
 int ns3d_adjoint_kinetic_energy(ns3d_handle *h, int nsteps, double dt, int checkpoint_every, double *J,
                                 double *const grad[3], double stats[4]) {
     if (!h || !J || !grad || nsteps < 1 || checkpoint_every < 1) return NS3D_ERR_INVALID_ARG;

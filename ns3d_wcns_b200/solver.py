@@ -199,6 +199,10 @@ class Solver:
         return J.value, grad, {"forward_ms": st[0], "adjoint_ms": st[1], "adjoint_bytes": st[2],
                                "recomputed_steps": st[3]}
 
+    def release_scratch(self) -> None:
+        """Gives back the device memory that adjoint and VJP calls keep with the handle."""
+        self._check(self.lib.ns3d_release_scratch(self.h))
+
     def profile(self, enable: bool = True) -> None:
         self._check(self.lib.ns3d_profile(self.h, int(enable)))
 

@@ -1,4 +1,6 @@
-"""Batch downloads: several threads at once, and without pinned memory."""
+"""What adjoint calls and batch downloads keep between calls: several threads
+downloading from one batch, downloads without pinned memory, and the calls
+that give the memory back."""
 import math
 from concurrent.futures import ThreadPoolExecutor
 
@@ -6,7 +8,7 @@ import numpy as np
 import pytest
 
 from ns3d_wcns_b200.config import GridDesc, make_params
-from ns3d_wcns_b200.initial import shock_tube_state
+from ns3d_wcns_b200.initial import isotropic_state, shock_tube_state
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +41,29 @@ def test_unpinned_download(gpu_lib):
         assert b.lib.ns3d_debug_batch_unpinned(b.h) == 0
         for i in range(3):
             assert np.array_equal(b.primitives(i), want[i])
+
+
+def test_release(gpu_lib):
+    import torch
+    from ns3d_wcns_b200.solver import Solver
+    n = (40, 36, 32)
+    P, G = make_params(n=n, Ma=0.3, Re=200.0, interpolation=0, riemann=0)
+    rng = np.random.default_rng(3)
+    with Solver(P, G) as s:
+        s.set_interior_primitives(*isotropic_state(n, P.gamma, P.Ma, seed=11))
+        ubar = rng.standard_normal((5,) + s.shape)
+        s.compute_rhs()
+        before = torch.cuda.mem_get_info()[0]
+        first = s.adjoint_kinetic_energy(4, 1e-3, 2)[:2], s.vjp_rk3_step(1e-3, ubar), s.vjp_rhs(ubar)
+        held = before - torch.cuda.mem_get_info()[0]
+        s.release_scratch()
+        # 69 interior arrays, and 2 checkpoints + 2 steps of 3 stages of 5 padded ones
+        assert held >= 8 * (69 * n[0] * n[1] * n[2] + 40 * s.sx * s.sy * s.sz)
+        assert before - torch.cuda.mem_get_info()[0] <= held // 8
+        again = s.adjoint_kinetic_energy(4, 1e-3, 2)[:2], s.vjp_rk3_step(1e-3, ubar), s.vjp_rhs(ubar)
+    assert first[0][0] == again[0][0] and np.array_equal(first[0][1], again[0][1])
+    assert np.array_equal(first[1], again[1]) and np.array_equal(first[2], again[2])
+    with batch([48, 200]) as b:
+        want = b.primitives(1)
+        b.release_scratch()
+        assert np.array_equal(b.primitives(1), want)
