@@ -200,7 +200,10 @@ int ns3d_time_advance(ns3d_handle *h, double t_end, int max_steps, double *time,
 /* Device pointers of a group (5 pointers, or 1 for TEMPERATURE) plus the
  * padded layout: layout[0..2] = sx, sy, sz, layout[3] = x pitch (elements),
  * layout[4] = x offset of i = 0 (elements), layout[5] = element size (bytes).
- * Pointers stay valid until the next ns3d_rk3_step / ns3d_destroy. */
+ * Mixed path: the primitive, temperature and RHS pointers stay valid until
+ * ns3d_destroy.  The plain path's primitives and the mixed path's conserved
+ * state change places with every step, stage (ns3d_rk3_stage), upload and
+ * ghost fill: ask again after each. */
 int ns3d_device_fields(ns3d_handle *h, int what, void *ptrs[5], long layout[6]);
 
 /* Bind the handle to a caller stream (cudaStream_t as void*).  NULL gives the

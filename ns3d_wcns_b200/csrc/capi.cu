@@ -294,9 +294,10 @@ struct ns3d_handle {
     double *rhs64[5] = {};
     double *T64 = nullptr;
     float *w32[5] = {};
-    // mixed: the FP32 primitives the stencils read.  Between steps w32; during
-    // a step the fused z-sweep writes each stage's result to a buffer of its
-    // own, in FP64 state planes that are free at that time (w32_buffer)
+    // mixed: the FP32 primitives the stencils read.  Between steps and between
+    // the stages of ns3d_rk3_stage w32; within a step the fused z-sweep writes
+    // each stage's result to a buffer of its own, in FP64 state planes that are
+    // free at that time (w32_buffer)
     int w32_cur = 0;
     float *rhs32[5] = {};
     float *T32 = nullptr;
@@ -636,8 +637,9 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
         // rk3_async's buffers: (1: s0, s0 -> b1), (2: s0, b1 -> b2), (3: s0, b2 -> b1)
         const int free_buf = 3 - src0 - (stage == 2 ? srcc : dst);
         if (free_buf < 0 || free_buf > 2 || free_buf == src0 || (stage != 2 && free_buf == dst)) return NS3D_ERR_STATE;
-        // the stage's result: dst == free_buf in stage 2
-        const int next = stage == 1 ? 1 + dst : (stage == 2 ? 4 + dst : 0);
+        // the stage's result, never the buffer it reads: dst == free_buf in
+        // stage 2; stage 3 reads w32 after ns3d_rk3_stage's copies
+        const int next = stage == 1 ? 1 + dst : (stage == 2 ? 4 + dst : (h->w32_cur ? 0 : 4 + srcc));
         FusedStage f{};
         f.stage = stage;
         for (int q = 0; q < 5; ++q) {
@@ -1905,6 +1907,19 @@ int ns3d_rk3_stage(ns3d_handle *h, int stage, double dt) {
         return r;
     }
     h->s0 = dst;
+    if (h->w32_cur) {
+        // between stages the primitives are where ns3d_device_fields has always
+        // had them: the caller writes the halo planes there.  Copied are the
+        // owned planes, and the ghost planes of real boundaries: 40 bytes a cell,
+        // against some 250 that a stage moves.
+        const Layout &L = h->L32;
+        const int k0 = h->zlo == 0 ? 0 : h->zlo + NG, k1 = h->zhi == L.nz ? L.sz : h->zhi + NG;
+        const size_t row = (size_t)L.sy * L.px, at = (size_t)k0 * row;
+        const size_t pitch = (char *)h->S[0][1] - (char *)h->S[0][0], pitch32 = (char *)h->w32[1] - (char *)h->w32[0];
+        CK(h, cudaMemcpy2DAsync(h->w32[0] + at, pitch32, w32_buffer(h, h->w32_cur, 0) + at, pitch, (k1 - k0) * row * 4, 5,
+                                cudaMemcpyDeviceToDevice, h->stream), "stage primitives");
+        h->w32_cur = 0;
+    }
     if (stage == 3) {
         h->step_start = -1;
         h->prev_valid = true;
@@ -1921,7 +1936,7 @@ int ns3d_device_fields(ns3d_handle *h, int what, void *ptrs[5], long layout[6]) 
     if (what == NS3D_PRIMITIVE && !h->mixed) {
         for (int q = 0; q < 5; ++q) ptrs[q] = h->S[h->s0][q];
     } else if (what == NS3D_PRIMITIVE && h->mixed) {
-        for (int q = 0; q < 5; ++q) ptrs[q] = w32_buffer(h, h->w32_cur, q);
+        for (int q = 0; q < 5; ++q) ptrs[q] = h->w32[q];
         L = &h->L32; esz = 4;
     } else if (what == NS3D_CONSERVED && h->mixed) {
         for (int q = 0; q < 5; ++q) ptrs[q] = h->S[h->s0][q];

@@ -33,3 +33,36 @@ def test_slabs_equal_domain(gpu_lib, n, precision, scheme, bcs):
         a = interior(s.primitives())
         b = slabs.owned_primitives()[:, :, 3:-3, 3:-3]
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("bcs", [(0,) * 6, (3, 3, 1, 2, 3, 2)], ids=["periodic", "bounded"])
+def test_mixed_pointers_stay(gpu_lib, bcs):
+    """On the mixed path a caller may take the pointers once: the halos of every stage written through them."""
+    from ns3d_wcns_b200 import _lib
+    from ns3d_wcns_b200.slab import InProcessSlabs
+    from ns3d_wcns_b200.solver import Solver
+    n = (24, 20, 38)
+    P, G = make_params(n=n, L=tuple(0.1 * m for m in n), interpolation=2, riemann=2, Re=300.0, bcs=bcs, precision=1)
+    W = random_state(n, seed=5, amp=0.2)
+    with Solver(P, G) as s, InProcessSlabs(P, G, 2) as slabs:
+        s.set_interior_primitives(*W)
+        slabs.set_interior_primitives(*W)
+        kept = {}
+
+        def planes(x, side, k0, count):
+            from ns3d_wcns_b200.slab import device_planes
+            key = (id(x), k0)
+            if key not in kept:
+                kept[key] = device_planes(x.s, k0, count)
+            return kept[key]
+        for x in slabs.slabs:
+            x.planes = lambda side, k0, count, x=x: planes(x, side, k0, count)
+        first = [x.s.device_fields(_lib.NS3D_PRIMITIVE)[0] for x in slabs.slabs]
+        for _ in range(2):
+            s.rk3_step(1e-3)
+            for stage in (1, 2, 3):
+                for x in slabs.slabs:
+                    assert x.s.lib.ns3d_rk3_stage(x.s.h, stage, 1e-3) == 0
+                assert [x.s.device_fields(_lib.NS3D_PRIMITIVE)[0] for x in slabs.slabs] == first
+                slabs.exchange_halos()
+        assert np.array_equal(interior(s.primitives()), slabs.owned_primitives()[:, :, 3:-3, 3:-3])
