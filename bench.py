@@ -174,6 +174,10 @@ def run_reference(args, rank):
     import multiprocessing as mp
     from oracle import oracle
     oracle.build(ref=os.path.isdir(oracle.REF_SRC_DIR))
+    if not oracle.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not there to be compiled"}),
+              flush=True)
+        return
     cores = len(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else os.cpu_count()
     n = 32
     t0 = time.perf_counter()
