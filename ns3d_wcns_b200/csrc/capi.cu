@@ -604,7 +604,7 @@ int stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, double d
     } else {
         StageArgsMixed a;
         for (int q = 0; q < 5; ++q) {
-            a.U0[q] = h->S[src0][q]; a.Uc[q] = h->S[srcc][q]; a.Rhs[q] = h->rhs32[q]; a.D[q] = nullptr;
+            a.U0[q] = h->S[src0][q]; a.Uc[q] = h->S[srcc][q]; a.Rhs[q] = h->rhs32[q];
             a.Uout[q] = h->S[dst][q]; a.Wout[q] = h->w32[q];
         }
         a.L = h->L64; a.L32 = h->L32; a.b = h->bc; a.dt = dt; a.gamma = h->ph.gamma; a.stage = stage;
@@ -666,7 +666,7 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
         StageArgsMixed a;
         for (int q = 0; q < 5; ++q) {
             a.U0[q] = h->S[src0][q]; a.Uc[q] = nullptr; a.Rhs[q] = h->rhs32[q];
-            a.Uout[q] = h->S[dst][q]; a.Wout[q] = f.W32out[q]; a.D[q] = f.D[q];
+            a.Uout[q] = h->S[dst][q]; a.Wout[q] = f.W32out[q];
         }
         a.L = h->L64; a.L32 = h->L32; a.b = h->bc; a.dt = dt; a.gamma = h->ph.gamma; a.stage = stage;
         a.Tout = h->T32; a.Rgas = h->ph.Rgas;

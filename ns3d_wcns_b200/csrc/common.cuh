@@ -8,6 +8,7 @@
 namespace ns3d {
 
 constexpr int NG = 3;  // ghost layers for WENO5/MDCD (initialization.cpp:175-192)
+constexpr int CHIP_SMS = 148;  // B200: what the rules that split the work by size count on
 
 // Padded device layout of one Field3D array: element (i,j,k), i in [0,sx),
 // lives at ((k*sy + j)*px + i + off).  off puts the first interior cell

@@ -374,12 +374,10 @@ __device__ __forceinline__ unsigned march_ring(unsigned o, unsigned ring) { retu
 // The loop body (some 800 instructions) just fits the instruction cache:
 // unrolling it by two, which would save the moves that slide the stencil,
 // stalls on instruction fetches (0.76 ms), by three 0.91 ms.
-#ifndef NS3D_MARCH_MINB
-#define NS3D_MARCH_MINB 6
-#endif
+constexpr int MARCH_MINB = 6;
 template <int DIR, typename T>
 constexpr int march_resident() {
-    return DIR == 2 && sizeof(typename LaneOf<T>::R) == 4 && LaneOf<T>::N == 2 ? NS3D_MARCH_MINB - 1 : NS3D_MARCH_MINB;
+    return DIR == 2 && sizeof(typename LaneOf<T>::R) == 4 && LaneOf<T>::N == 2 ? MARCH_MINB - 1 : MARCH_MINB;
 }
 
 template <int DIR, typename T, int INTERP, int RS>
@@ -645,7 +643,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
 // resident warp costs `c` per face while the chip is full and a lone warp
 // `latency` (in units of c), and every segment computes five faces more.
 inline int march_segment(long nblocks, int n, int resident) {
-    const int sms = 148;
+    const int sms = CHIP_SMS;
     const double latency = 12.0;
     int best = n;
     double least = 1e300;

@@ -130,7 +130,6 @@ struct StageArgsMixed {
     double dx, vol;
     const double *dt_dev;   // non-null: dt from the device time loop (replaces dt)
     const int *done;        // non-null: skip the launch while *done
-    const float *D[5];      // ghost kernel after the fused z-sweep: stage increments (FP32 layout)
 };
 
 __global__ void __launch_bounds__(STAGE_THREADS) stage_kernel_mixed(StageArgsMixed a) {

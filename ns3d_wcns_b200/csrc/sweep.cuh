@@ -590,7 +590,7 @@ inline int sweep_segment(long blocks, int n, int C, int resident = 2) {
     for (int k = all; k >= 1; --k) {
         const int len = k == all ? n : k * C - 5;
         if (len < 1) break;
-        const long slots = (long)resident * 148, rounds = (blocks * ((n + len - 1) / len) + slots - 1) / slots;
+        const long slots = (long)resident * CHIP_SMS, rounds = (blocks * ((n + len - 1) / len) + slots - 1) / slots;
         const double t = rounds * (k + 0.5);
         if (t < least * 0.98) { least = t; best = len; }
     }

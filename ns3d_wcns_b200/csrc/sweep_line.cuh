@@ -577,7 +577,7 @@ inline cudaError_t sweep_line_select(const SweepArgs<typename LaneOf<T>::R> &a, 
 // x-neighbours, so together they use a 32-byte sector), and the marching kernel
 // with its coalesced lanes is three times as fast on a full chip.  But it has a
 // thread per line and walks it a face at a time: on a small grid it is latency,
-// or cuts the lines into segments that recompute eight faces each.  The line
+// or cuts the lines into segments that recompute five faces each.  The line
 // kernel takes the grids whose chunks of 64 faces fit the chip's resident warps
 // at most twice along y and once along z, where the fused stage adds more
 // strided traffic.  us, march / line: FP64 y 16x16x16 14.7 / 10.5, 32^3 18.9 /
@@ -591,7 +591,7 @@ template <int DIR, typename T>
 inline bool line_takes(const SweepArgs<typename LaneOf<T>::R> &a) {
     const int n = DIR == 1 ? a.L.ny : a.zhi - a.zlo, C = XLine<DIR, T>::C;
     const long lines = (long)(a.L.nx / LaneOf<T>::N) * (DIR == 1 ? a.zhi - a.zlo : a.L.ny);
-    const long warps = 148L * XL_WARPS * xline_resident<DIR, T, I_MDCD_HYBRID, RUNTIME>();
+    const long warps = (long)CHIP_SMS * XL_WARPS * xline_resident<DIR, T, I_MDCD_HYBRID, RUNTIME>();
     return lines * (xline_ring<DIR, T>(a) ? 1 : (n + 5 + C - 1) / C) <= (DIR == 1 ? 2 : 1) * warps;
 }
 template <int DIR, typename T>

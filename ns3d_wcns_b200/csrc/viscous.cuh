@@ -116,7 +116,7 @@ __device__ __forceinline__ R dtile(F f, int order, const R *dinv) {
 inline int visc_planes(const Layout &L, int planes) {
     const long columns = (long)((L.nx + VTX - 1) / VTX) * ((L.ny + VTY - 1) / VTY);
     int zc = VZC;
-    while (zc > VZC_MIN && columns * ((planes + zc - 1) / zc) < 2 * 148) zc /= 2;
+    while (zc > VZC_MIN && columns * ((planes + zc - 1) / zc) < 2 * CHIP_SMS) zc /= 2;
     return zc;
 }
 
