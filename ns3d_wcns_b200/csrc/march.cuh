@@ -681,7 +681,7 @@ inline MarchArgs<T> march_args(const SweepArgs<typename LaneOf<T>::R> &a) {
     for (int k = 0; k < 6; ++k) m.lin[k] = both(a.sp.lin[k]);
     for (int k = 0; k < 3; ++k) { m.dc[k] = both(a.dc[k]); m.vc[k] = both(a.vc[k]); }
     m.inv_h = both(a.inv_h);
-    m.inv_60h = both(a.dinv[2]);
+    m.inv_60h = both(LaneOf<T>::N == 2 ? -a.dinv[2] : a.dinv[2]);
     m.nlines = m.seg_len = 0;
     return m;
 }

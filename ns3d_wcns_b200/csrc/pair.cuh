@@ -54,7 +54,8 @@ struct PairOps {
 };
 
 // The scaled sums are taken away from r, not added to it: sub2's multiply-add
-// takes a rounded product, where a product and add2 are contracted.
+// takes a rounded product, where a product and add2 are contracted.  So
+// node_diff's scale is minus 1/(60 h) (march_args).
 __device__ __forceinline__ float2 face_diff(const float2 *dc, float2 inv_h, float2 l1, float2 r1, float2 l2, float2 r2,
                                             float2 l3, float2 r3, float2 r) {
     float2 t = mul2(sub2(r1, l1), dc[0]);
@@ -62,13 +63,13 @@ __device__ __forceinline__ float2 face_diff(const float2 *dc, float2 inv_h, floa
     t = fma2(sub2(r3, l3), dc[2], t);
     return sub2(r, mul2(t, inv_h));
 }
-__device__ __forceinline__ float2 node_diff(const float2 *, float2 inv_60h, float2 p1, float2 m1, float2 q2, float2 m2,
+__device__ __forceinline__ float2 node_diff(const float2 *, float2 minus_inv_60h, float2 p1, float2 m1, float2 q2, float2 m2,
                                             float2 p3, float2 m3, float2 r) {
     float2 t = fma2(p2(-9.f), q2, p3);
     t = fma2(p2(45.f), p1, t);
     t = fma2(p2(-45.f), m1, t);
     t = sub2(fma2(p2(9.f), m2, t), m3);
-    return sub2(r, mul2(make_float2(-t.x, -t.y), inv_60h));
+    return sub2(r, mul2(t, minus_inv_60h));
 }
 
 // sum_k c_k f_k (mdcd_linear) for both lines; ONE: the first product rounded
