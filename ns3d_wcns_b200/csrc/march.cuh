@@ -19,10 +19,10 @@
 //
 // 256^3, one launch, against the chunked kernel (a face per thread, shared
 // stencils, three barriers a chunk) that it replaced: FP64 MDCD_HYBRID + HLLC y
-// 0.861 -> 0.710 ms, fused z 1.127 -> 0.922; WENO5 + Roe 1.222 -> 0.892 and 1.512
-// -> 1.065; mixed 0.431 -> 0.374 and 0.672 -> 0.618.  Issue and FP64 latency
-// bound it now: 11 warps per SM (168 registers), issue slots 48-54 % and the FP64
-// pipe 39-43 % busy, 3.4 TB/s.
+// 0.861 -> 0.703 ms, fused z 1.127 -> 0.917; WENO5 + Roe 1.222 -> 0.892 and 1.512
+// -> 1.10; mixed 0.431 -> 0.372 and 0.672 -> 0.623.  Issue and FP64 latency
+// bound it now: 11 warps per SM (162-168 registers), issue slots 48-55 % and the
+// FP64 pipe 39-43 % busy, 3.4 TB/s.
 #pragma once
 
 #include "pair.cuh"

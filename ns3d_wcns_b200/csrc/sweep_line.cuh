@@ -14,10 +14,10 @@
 // The one-face kernel (eight lines to a block, a barrier after each phase)
 // waited on shared memory and barriers for 3.3 of every 8.3 stall cycles;
 // 256^3, one launch along x: FP64 MDCD_HYBRID + HLLC 0.842 -> 0.675 ms, WENO5 +
-// Roe 1.083 -> 0.775; FP32 pairs 0.461 -> 0.400 and 0.521 -> 0.476 (0.713,
+// Roe 1.083 -> 0.775; FP32 pairs 0.461 -> 0.402 and 0.521 -> 0.487 (0.713,
 // 0.789, 0.434, 0.508 with the first chunk loaded position by position).  What
 // bounds it now is FP64 issue and latency at twelve warps per SM (192^3, FP64:
-// issue slots 46 % and the FP64 pipe 39 % busy, 2.2 TB/s).
+// issue slots 51 % and the FP64 pipe 41 % busy, 2.3 TB/s).
 #pragma once
 
 #include "march.cuh"
