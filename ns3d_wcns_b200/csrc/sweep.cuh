@@ -215,7 +215,8 @@ __device__ __forceinline__ void fused_stage_cell(const FusedStage &f, double dt,
         T = temperature_exact<E>(W, f.Rgas);
     };
     convert(std::integral_constant<int, 0>{});
-    if (__builtin_expect(!finite_fp64(W[4]) || !finite_fp64(T), 0)) convert(std::integral_constant<int, 2>{});
+    // T is not finite where anything before it is not
+    if (__builtin_expect(!finite_fp64(T), 0)) convert(std::integral_constant<int, 2>{});
 #pragma unroll
     for (int q = 0; q < 5; ++q) f.Wout[q][c] = W[q];
     f.Tout[c] = T;
