@@ -274,8 +274,9 @@ __device__ __forceinline__ void march_states(const MarchArgs<T> &m, const T (*u)
     }
 }
 
-template <int DIR, typename T, int RS>
+template <int DIR, typename T, int INTERP, int RS>
 __device__ __forceinline__ void march_flux(const SchemeParams<typename LaneOf<T>::R> &sp, const T *UL, const T *UR, T *F) {
+    constexpr bool FORMER = sizeof(typename LaneOf<T>::R) == 4 && INTERP != I_WENO5;
     if constexpr (LaneOf<T>::N == 2) {
         if constexpr (RS == R_HLLC) {
             hllc_flux2<DIR>(UL, UR, sp.gamma, F);
@@ -283,15 +284,15 @@ __device__ __forceinline__ void march_flux(const SchemeParams<typename LaneOf<T>
             float l[5], r[5], fa[5], fb[5];
 #pragma unroll
             for (int q = 0; q < 5; ++q) { l[q] = UL[q].x; r[q] = UR[q].x; }
-            riemann<DIR, float, RS>(sp, l, r, fa);
+            riemann<DIR, float, RS, FORMER>(sp, l, r, fa);
 #pragma unroll
             for (int q = 0; q < 5; ++q) { l[q] = UL[q].y; r[q] = UR[q].y; }
-            riemann<DIR, float, RS>(sp, l, r, fb);
+            riemann<DIR, float, RS, FORMER>(sp, l, r, fb);
 #pragma unroll
             for (int q = 0; q < 5; ++q) F[q] = make_float2(fa[q], fb[q]);
         }
     } else {
-        riemann<DIR, T, RS>(sp, UL, UR, F);
+        riemann<DIR, T, RS, FORMER>(sp, UL, UR, F);
     }
 }
 
@@ -540,7 +541,7 @@ __global__ void __launch_bounds__(MARCH_NT, march_resident<DIR, T>()) march_kern
         if (f >= f0 && (per || (f >= NG - 1 && f < n + NG))) {
             T UL[5], UR[5];
             march_states<T, INTERP, RS>(m, u, doubt, UL, UR);
-            march_flux<DIR, T, RS>(a.sp, UL, UR, fn);
+            march_flux<DIR, T, INTERP, RS>(a.sp, UL, UR, fn);
             if (!per && f == NG - 1 && a.outflow_lo) {  // ghost faces copy the boundary face
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {

@@ -384,7 +384,7 @@ struct Side {
 // degenerate waves (eigenvalue V) contribute |V|(dU - a0 R0 - a4 R4): only
 // the two acoustic projections are formed.  Harten entropy fix with
 // delta = 0.1 max|lambda| = 0.1 (|V| + c) as the reference.
-template <int DIR, typename R>
+template <int DIR, typename R, bool FORMER = false>
 NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
     L.load(UL, g); Rt.load(UR, g);
@@ -392,7 +392,7 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     L.flux(FL); Rt.flux(FR);
     const R gm1 = g - R(1);
     R HL, HR;
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (FORMER) {
         const R kfac = g / gm1;
         HL = R(0.5) * (L.u * L.u + L.v * L.v + L.w * L.w) + kfac * L.p * L.ir;
         HR = R(0.5) * (Rt.u * Rt.u + Rt.v * Rt.v + Rt.w * Rt.w) + kfac * Rt.p * Rt.ir;
@@ -430,7 +430,7 @@ NS3D_HD void roe_flux(const R *UL, const R *UR, R g, R *F) {
     l4 = l4 < delta ? (l4 * l4 + d2) * i2d : l4;
     const R k0 = (l0 - lv) * A0, k4 = (l4 - lv) * A4;
     // R0 = (1, u-nc, v-nc, w-nc, H-cV), R4 = (1, u+nc, v+nc, w+nc, H+cV)
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (FORMER) {
         R cx = DIR == 0 ? c : R(0), cy = DIR == 1 ? c : R(0), cz = DIR == 2 ? c : R(0);
         R D0 = lv * dU[0] + k0 + k4;
         R D1 = lv * dU[1] + k0 * (ub - cx) + k4 * (ub + cx);
@@ -514,9 +514,7 @@ NS3D_HD void hllc_star(const Side<DIR, R> &S, const R *U, const R *Fs, R Sk, R S
 //   E* = (dk E - p u_n + p* S_M) / (S_k - S_M),
 //   F = (rho* S_M, rho* S_M V + p* n, (E* + p*) S_M)
 // -- the same flux with half of the operations, one quotient less, and a third
-// less rounding than the sum.  FP32 keeps hllc_star, as it keeps its form of
-// the Roe dissipation: the hybrid scheme turns another rounding into another
-// trajectory.
+// less rounding than the sum of hllc_star (FORMER, see riemann).
 template <int DIR, typename R>
 NS3D_HD void hllc_jump(R u, R v, R w, R E, R p, R un, R Sk, R dk, R m, R SM, R *F) {
     const R is = rcp_(Sk - SM);
@@ -532,7 +530,7 @@ NS3D_HD void hllc_jump(R u, R v, R w, R E, R p, R un, R Sk, R dk, R m, R SM, R *
 
 // HLLC_Riemann_solver, InviscousFlux.cpp:449-592: Davis S_L/S_R, Batten S_M
 // (Roe-averaged normal velocity when the S_M denominator is below 1e-12).
-template <int DIR, typename R>
+template <int DIR, typename R, bool FORMER = false>
 NS3D_HD void hllc_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
     L.load(UL, g); Rt.load(UR, g);
@@ -541,7 +539,7 @@ NS3D_HD void hllc_flux(const R *UL, const R *UR, R g, R *F) {
     R SR = fmax(L.un + aL, Rt.un + aR);
     if (SL >= R(0)) { L.flux(F); return; }
     if (SR <= R(0)) { Rt.flux(F); return; }
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (FORMER) {
         R num = Rt.r * Rt.un * (SR - Rt.un) - L.r * L.un * (SL - L.un) + L.p - Rt.p;
         R den = Rt.r * (SR - Rt.un) - L.r * (SL - L.un);
         R SM;
@@ -585,7 +583,7 @@ NS3D_HD void hllc_flux(const R *UL, const R *UR, R g, R *F) {
 }
 
 // HLLC_p_Riemann_solver, InviscousFlux.cpp:594-717: PVRS p*, Toro speeds.
-template <int DIR, typename R>
+template <int DIR, typename R, bool FORMER = false>
 NS3D_HD void hllc_p_flux(const R *UL, const R *UR, R g, R *F) {
     Side<DIR, R> L, Rt;
     L.load(UL, g); Rt.load(UR, g);
@@ -599,7 +597,7 @@ NS3D_HD void hllc_p_flux(const R *UL, const R *UR, R g, R *F) {
     if (SR <= R(0)) { Rt.flux(F); return; }
     R SM = quot_(Rt.p - L.p + L.r * L.un * (SL - L.un) - Rt.r * Rt.un * (SR - Rt.un),
                  L.r * (SL - L.un) - Rt.r * (SR - Rt.un));
-    if constexpr (sizeof(R) == 4) {
+    if constexpr (FORMER) {
         R Fs[5];
         if (SM >= R(0)) { L.flux(Fs); hllc_star<DIR, R>(L, UL, Fs, SL, SM, F); }
         else { Rt.flux(Fs); hllc_star<DIR, R>(Rt, UR, Fs, SR, SM, F); }
@@ -688,14 +686,18 @@ NS3D_HD void steger_warming_flux(const R *UL, const R *UR, R g, R *F) {
     for (int n = 0; n < 5; ++n) F[n] = Fp[n] + Fm[n];
 }
 
-template <int DIR, typename R, int RS>
+// FORMER: Roe, HLLC and HLLC_P in the form the FP32 sweeps have had from the
+// start.  The hybrid scheme turns another rounding into another trajectory, so
+// FP32 keeps it (component-wise WENO5 has no detector and takes the forms of
+// less error: WENO5 + HLLC 1.4e-6 of a rough box's right-hand side, not 2.3e-6).
+template <int DIR, typename R, int RS, bool FORMER = false>
 NS3D_HD void riemann(const SchemeParams<R> &sp, const R *UL, const R *UR, R *F) {
     const int rs = RS == RUNTIME ? sp.riemann : RS;
     const R g = sp.gamma;
-    if (RS == R_ROE || (RS == RUNTIME && rs == R_ROE)) roe_flux<DIR, R>(UL, UR, g, F);
-    else if (RS == R_HLLC || (RS == RUNTIME && rs == R_HLLC)) hllc_flux<DIR, R>(UL, UR, g, F);
+    if (RS == R_ROE || (RS == RUNTIME && rs == R_ROE)) roe_flux<DIR, R, FORMER>(UL, UR, g, F);
+    else if (RS == R_HLLC || (RS == RUNTIME && rs == R_HLLC)) hllc_flux<DIR, R, FORMER>(UL, UR, g, F);
     else if (RS == R_HLL || (RS == RUNTIME && rs == R_HLL)) hll_flux<DIR, R>(UL, UR, g, F);
-    else if (RS == R_HLLC_P || (RS == RUNTIME && rs == R_HLLC_P)) hllc_p_flux<DIR, R>(UL, UR, g, F);
+    else if (RS == R_HLLC_P || (RS == RUNTIME && rs == R_HLLC_P)) hllc_p_flux<DIR, R, FORMER>(UL, UR, g, F);
     else if (RS == R_RUSANOV || (RS == RUNTIME && rs == R_RUSANOV)) rusanov_flux<DIR, R>(UL, UR, g, F);
     else if (RS == R_STEGER_WARMING || (RS == RUNTIME && rs == R_STEGER_WARMING))
         steger_warming_flux<DIR, R>(UL, UR, g, F);

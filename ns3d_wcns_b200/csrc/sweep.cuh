@@ -421,7 +421,7 @@ sweep_kernel(SweepArgs<R> a) {
                 }
             }
             R F[5];
-            riemann<DIR, R, RUNTIME>(a.sp, UL, UR, F);
+            riemann<DIR, R, RUNTIME, sizeof(R) == 4>(a.sp, UL, UR, F);
             const int s = G::template idx<NF>(line, slot + 5);
 #pragma unroll
             for (int q = 0; q < 5; ++q) sF[q * NL * NF + s] = F[q];

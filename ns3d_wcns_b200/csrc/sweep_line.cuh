@@ -293,7 +293,7 @@ sweep_line_kernel(const __grid_constant__ MarchArgs<T> m) {
                 if (__any_sync(0xffffffffu, doubt != 0)) xline_weno<T>(a.sp.hd, sU, doubt, UL, UR);
             }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) march_flux<DIR, T, RS>(a.sp, UL[h], UR[h], fn[h]);
+            for (int h = 0; h < 2; ++h) march_flux<DIR, T, INTERP, RS>(a.sp, UL[h], UR[h], fn[h]);
             if (per && whole && f < 5) {  // first chunk (fb = 0): faces 0 .. 5
 #pragma unroll
                 for (int h = 0; h < 2; ++h)

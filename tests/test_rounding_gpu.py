@@ -4,7 +4,8 @@ test_rhs_rounding: the right-hand side's error (2-norm) against the oracle in
 80-bit arithmetic is no larger than that of the kernels with IEEE reciprocals,
 quotients and square roots and the eigenvector matrices, measured once on the
 same states; one per cent is left for the compiler's placement of fused
-operations."""
+operations.  test_mixed_rounding: the mixed path's with component-wise WENO5,
+against the first kernels that formed both states from shared differences."""
 import numpy as np
 import pytest
 
@@ -20,13 +21,12 @@ FORMER = {(0, 0, 0): 1.118e-15, (0, 2, 0): 1.487e-15, (0, 3, 0): 1.120e-15, (2, 
           (0, 0, 1): 2.069e-15, (3, 2, 1): 2.495e-15, (0, 3, 1): 2.018e-15}  # interpolation, riemann, characteristic
 
 
-@pytest.mark.parametrize("scheme", list(FORMER), ids=str)
-def test_rhs_rounding(gpu_lib, scheme):
+def rhs_error(n, scheme, precision):
     from ns3d_wcns_b200.solver import Solver
     from oracle import oracle
-    P, G = make_params(n=N, L=tuple(0.1 * m for m in N), interpolation=scheme[0], riemann=scheme[1],
-                       char_recon=scheme[2], Re=300.0)
-    W = random_state(N, seed=5, amp=0.2)
+    P, G = make_params(n=n, L=tuple(0.1 * m for m in n), interpolation=scheme[0], riemann=scheme[1],
+                       char_recon=scheme[2], Re=300.0, precision=precision)
+    W = random_state(n, seed=5, amp=0.2)
     o = oracle.ExtendedSolver(P, G)
     o.set_interior_prims(*W)
     o.compute_rhs()
@@ -35,7 +35,17 @@ def test_rhs_rounding(gpu_lib, scheme):
         s.set_interior_primitives(*W)
         s.compute_rhs()
         off = interior(s.rhs()).astype(np.longdouble) - want
-    assert float(np.sqrt((off ** 2).sum() / (want ** 2).sum())) <= 1.01 * FORMER[scheme]
+    return float(np.sqrt((off ** 2).sum() / (want ** 2).sum()))
+
+
+@pytest.mark.parametrize("scheme", list(FORMER), ids=str)
+def test_rhs_rounding(gpu_lib, scheme):
+    assert rhs_error(N, scheme, 0) <= 1.01 * FORMER[scheme]
+
+
+@pytest.mark.parametrize("riemann,former", [(0, 4.391e-7), (2, 4.896e-7), (3, 4.464e-7), (1, 4.495e-7)])
+def test_mixed_rounding(gpu_lib, riemann, former):
+    assert rhs_error((24, 20, 38), (0, riemann, 0), 1) <= 1.01 * former
 
 
 def line_rhs(U, g, h):
