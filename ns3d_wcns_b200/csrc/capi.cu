@@ -651,7 +651,7 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
         f.L64 = h->L64;
         f.dt = dt;
         f.dt_dev = h->dev_loop ? &h->clock->dt : nullptr;
-        f.gamma = h->ph.gamma; f.Rgas = h->ph.Rgas; f.dx = h->ph.dx;
+        f.gamma = h->ph.gamma; f.Rgas = h->ph.Rgas; f.inv_Rgas = 1.0 / h->ph.Rgas; f.dx = h->ph.dx;
         f.vol = h->ph.dx * h->ph.dy * h->ph.dz;
         f.cfl_part = stage == 3 ? h->cfl_part : nullptr;
         f.ke_part = stage == 3 ? h->ke_part : nullptr;
@@ -692,7 +692,7 @@ int rk_stage_async(ns3d_handle *h, int stage, int src0, int srcc, int dst, doubl
     f.L64 = h->L64;
     f.dt = dt;
     f.dt_dev = h->dev_loop ? &h->clock->dt : nullptr;
-    f.gamma = h->ph.gamma; f.Rgas = h->ph.Rgas; f.dx = h->ph.dx;
+    f.gamma = h->ph.gamma; f.Rgas = h->ph.Rgas; f.inv_Rgas = 1.0 / h->ph.Rgas; f.dx = h->ph.dx;
     f.vol = h->ph.dx * h->ph.dy * h->ph.dz;
     f.cfl_part = stage == 3 ? h->cfl_part : nullptr;
     f.ke_part = stage == 3 ? h->ke_part : nullptr;

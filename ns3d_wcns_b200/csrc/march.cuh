@@ -306,7 +306,7 @@ template <typename T>
 __device__ __forceinline__ void march_stage_mixed(const FusedStage &f, double dt, uint32_t cid, uint32_t c64, const T *rq,
                                                   const double *s0, const T *d, double &smax, double &ke, double &kc) {
     constexpr int LN = LaneOf<T>::N;
-    const double irg = 1.0 / f.Rgas;
+    const double irg = f.inv_Rgas;
     T Dn[5], Wn[5], Tn;
 #pragma unroll
     for (int h = 0; h < LN; ++h) {

@@ -68,7 +68,7 @@ struct FusedStage {
     Layout L64;             // layout of the FP64 arrays
     double dt;
     const double *dt_dev;   // non-null: dt from the device time loop
-    double gamma, Rgas, dx, vol;
+    double gamma, Rgas, inv_Rgas, dx, vol;
     double *cfl_part, *ke_part;  // stage 3: per-block CFL minimum and kinetic energy
     int keep_rhs;                // also write the complete RHS (the handle's keep_rhs, stage 3 only)
 };
@@ -254,7 +254,7 @@ sweep_kernel(SweepArgs<R> a) {
     // fused stage (z-sweep): dt, and the thread's largest wave speed / kinetic energy
     const double fdt = (DIR == 2 && a.fs.stage) ? (a.fs.dt_dev ? *a.fs.dt_dev : a.fs.dt) : 0.0;
     double cfl_acc = 0.0, ke_acc = 0.0, ke_c = 0.0;  // largest wave speed, kinetic energy
-    const double irg = (DIR == 2 && sizeof(R) == 4 && a.fs.stage) ? 1.0 / a.fs.Rgas : 0.0;  // mixed: T = p / (rho Rgas)
+    const double irg = a.fs.inv_Rgas;  // mixed: T = p / (rho Rgas)
     const int slot = DIR == 0 ? threadIdx.x : threadIdx.y;
     const int line = DIR == 0 ? threadIdx.y : threadIdx.x;
     const int ta0 = blockIdx.x * NL + line, tb0 = blockIdx.y + (DIR == 2 ? 0 : a.zlo);
