@@ -276,7 +276,7 @@ __device__ __forceinline__ void march_states(const MarchArgs<T> &m, const T (*u)
 
 template <int DIR, typename T, int INTERP, int RS>
 __device__ __forceinline__ void march_flux(const SchemeParams<typename LaneOf<T>::R> &sp, const T *UL, const T *UR, T *F) {
-    constexpr bool FORMER = sizeof(typename LaneOf<T>::R) == 4 && INTERP != I_WENO5;
+    constexpr bool FORMER = sizeof(typename LaneOf<T>::R) == 4 && INTERP == I_MDCD_HYBRID;
     if constexpr (LaneOf<T>::N == 2) {
         if constexpr (RS == R_HLLC) {
             hllc_flux2<DIR>(UL, UR, sp.gamma, F);

@@ -687,9 +687,10 @@ NS3D_HD void steger_warming_flux(const R *UL, const R *UR, R g, R *F) {
 }
 
 // FORMER: Roe, HLLC and HLLC_P in the form the FP32 sweeps have had from the
-// start.  The hybrid scheme turns another rounding into another trajectory, so
-// FP32 keeps it (component-wise WENO5 has no detector and takes the forms of
-// less error: WENO5 + HLLC 1.4e-6 of a rough box's right-hand side, not 2.3e-6).
+// start, for the hybrid scheme, which turns another rounding into another
+// trajectory, and for characteristic reconstruction.  Component-wise WENO5 and
+// MDCD_LINEAR have no detector and take the forms of less error (WENO5 + HLLC
+// 4.9e-7 of a rough box's right-hand side, not 7.7e-7).
 template <int DIR, typename R, int RS, bool FORMER = false>
 NS3D_HD void riemann(const SchemeParams<R> &sp, const R *UL, const R *UR, R *F) {
     const int rs = RS == RUNTIME ? sp.riemann : RS;

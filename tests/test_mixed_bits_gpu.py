@@ -5,7 +5,8 @@ test_mixed_bits: the right-hand side and the primitives after two steps, bit
 for bit against digests of the kernels that carried a face per thread through
 shared memory (golden/mixed_bits.json), through the line kernel (small grids)
 and the marching kernel, with two lines in a float2 (even line counts) and
-with one.
+with one.  MDCD_LINEAR, which has no detector, with HLLC on pairs, the form
+both have; on single lines its HLLC has less error now.
 
 test_hybrid_against_oracle: the right-hand side against the FP64 oracle on
 under-resolved states whose warps have few and many faces in doubt.  Where no
@@ -48,6 +49,8 @@ def mixed_params(n, scheme, bcs):
 def cases():
     for i, n in enumerate(SIZES):
         for j, sc in enumerate(SCHEMES):
+            if sc == (2, 2, 0) and (n[0] | n[1]) & 1:
+                continue
             b = ("periodic", "bounded")[(i + j) % 2]
             yield n, sc, b, (i + j) % 3
 
